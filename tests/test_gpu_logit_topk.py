@@ -95,3 +95,28 @@ def test_rows_of_the_q8_head(oracle):
     got = run_topk(logits, M, vocab, vocab)
     assert int(err.item()) == 0
     check_rows(oracle, got, logits.cpu().numpy())
+
+
+def test_rows_straight_behind_the_head(oracle):
+    """Head and top-k issued back to back into the caller's buffers, nothing between the two launches, with a vocabulary large enough
+    that the head's CTAs share items (their sums meet in memory at the very end of the launch): the rows have to be those of the
+    finished logits."""
+    vocab, cols, M = 148 * 128 + 1040, 2048, 3
+    bpr = cols // 32
+    w = torch.empty(vocab * bpr * 34, dtype=torch.uint8, device="cuda")
+    capi.call("tsp_synth_weights", formats.Q8_0, 78, 0, vocab * bpr, 0.02, w.data_ptr(), L.stream_ptr())
+    ms = L.matrix_set(w, formats.Q8_0, formats.GGUF, vocab, cols)
+    xs = [torch.from_numpy(synth.activations_f16(32 + i, M, cols).astype(np.float32)).cuda() for i in range(20)]
+    lib, st = capi.lib(), L.stream_ptr()
+    scratch = torch.empty(lib.tsp_logit_topk_scratch_bytes(M, vocab), dtype=torch.uint8, device="cuda")
+    logits = torch.zeros((len(xs), M, vocab), dtype=torch.float32, device="cuda")
+    out = torch.zeros((len(xs), M, 132), dtype=torch.int32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for i, x in enumerate(xs):
+        capi.call("tsp_moe_project", C.byref(ms), x.data_ptr(), cols * 4, 1, M, 1, None, None, None, logits[i].data_ptr(), vocab * 4, 1, err.data_ptr(), st)
+        capi.call("tsp_logit_topk", logits[i].data_ptr(), vocab * 4, M, vocab, scratch.data_ptr(), scratch.numel(), out[i].data_ptr(), M * 528, st)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    for i in range(len(xs)):
+        check_rows(oracle, out[i].cpu().numpy().view(np.uint32), logits[i].cpu().numpy())

@@ -132,6 +132,9 @@ __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, u
 // of this one have started), set-up that touches no global memory, then `pdl_wait()` on every path before the first
 // global access; the wait returns when the previous kernel has completed and its writes are visible, so the chain of
 // kernels stays transitively ordered.
+// Such a kernel takes no `const T* __restrict__` parameter: the compiler may treat loads through one as invariant for the whole
+// kernel and move them above the wait, whatever the "memory" clobber says (the top-64 tile kernel read logits of the
+// vocabulary head before the head's last partial sums had landed: most runs returned a wrong row).
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -732,7 +732,7 @@ int launch_staged_f16(const uint8_t* expert, uint32_t rows, uint32_t cols, void*
 // ---------------------------------------------------------------------------------------------
 // helpers: route offsets, the K-ordered binary16 copy of the input rows
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) route_offsets_kernel(const uint32_t* __restrict__ counts, uint32_t experts, uint32_t* __restrict__ offsets) {
+__global__ void __launch_bounds__(256) route_offsets_kernel(const uint32_t* counts, uint32_t experts, uint32_t* __restrict__ offsets) {
     pdl_launch_dependents();
     pdl_wait();
     __shared__ uint32_t warp_sum[8];
@@ -764,7 +764,7 @@ __global__ void __launch_bounds__(256) route_offsets_kernel(const uint32_t* __re
 // gate-up GEMM, fetched from here by token id. 64 threads per row, four rows per CTA.
 template <bool IN16>
 __global__ void __launch_bounds__(256)
-rows_f16k_kernel(const void* __restrict__ x, uint64_t x_stride, uint32_t rows, uint32_t cols, __half* __restrict__ xk, uint64_t xk_stride, uint32_t* error) {
+rows_f16k_kernel(const void* x, uint64_t x_stride, uint32_t rows, uint32_t cols, __half* __restrict__ xk, uint64_t xk_stride, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t row = blockIdx.x * 4 + (threadIdx.x >> 6);
@@ -797,7 +797,7 @@ rows_f16k_kernel(const void* __restrict__ x, uint64_t x_stride, uint32_t rows, u
 // Routed copy of the K-ordered input rows: position p of the permuted order belongs to the expert e with
 // offsets[e] <= p < offsets[e+1]; its route id is token_map[e*tokens + p - offsets[e]], its input row route / selected.
 __global__ void __launch_bounds__(256)
-gather_rows16_kernel(const uint4* __restrict__ xk, uint64_t xk_stride, const uint32_t* __restrict__ token_map, const uint32_t* __restrict__ offsets,
+gather_rows16_kernel(const uint4* xk, uint64_t xk_stride, const uint32_t* token_map, const uint32_t* offsets,
                      uint32_t experts, uint32_t tokens, uint32_t selected, uint32_t cols, uint4* __restrict__ xp, uint64_t xp_stride) {
     pdl_launch_dependents();
     pdl_wait();

@@ -8,7 +8,7 @@ namespace tsp {
 // out[t][c] = sum_b normalized[t][b][c] * sigmoid(scores[t][b][c]) / branches      (branch order ascending, as the reference adds them)
 // scales[t][b] = 2 * sigmoid(inject_logits[t][b] / branches)
 __global__ void __launch_bounds__(256)
-residual_read_kernel(const float* __restrict__ normalized, const float* __restrict__ scores, const float* __restrict__ inject_logits,
+residual_read_kernel(const float* normalized, const float* scores, const float* inject_logits,
                      uint32_t branches, uint32_t channels, float* __restrict__ output, float* __restrict__ scales, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
@@ -35,7 +35,7 @@ residual_read_kernel(const float* __restrict__ normalized, const float* __restri
 
 // destination[t][b][c] = streams[t][b][c] + scales[t][b] * output[t][c]
 __global__ void __launch_bounds__(256)
-residual_write_kernel(const float* __restrict__ streams, const float* __restrict__ output, const float* __restrict__ scales, uint32_t branches,
+residual_write_kernel(const float* streams, const float* output, const float* scales, uint32_t branches,
                       uint32_t channels, float* __restrict__ destination, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();

@@ -23,7 +23,7 @@ __device__ __forceinline__ double sigmoid_f64(double v) {
 // One warp routes one token row; `row` is the warp's scratch of `experts` floats in shared memory.
 // `margins` (optional): margins[token] = logit of the last selected expert - logit of the best expert left out (+inf when every
 // expert is selected): how far the selection is from changing under a perturbation of the logits.
-__device__ __forceinline__ void route_row(float* row, const float* __restrict__ src, uint32_t token, uint32_t experts, uint32_t selected,
+__device__ __forceinline__ void route_row(float* row, const float* src, uint32_t token, uint32_t experts, uint32_t selected,
                                           uint32_t mode, int normalize, uint32_t* __restrict__ ids, float* __restrict__ weights,
                                           uint32_t* error, uint32_t lane, float* __restrict__ margins = nullptr) {
     bool bad = false;
@@ -104,7 +104,7 @@ __device__ __forceinline__ void route_row(float* row, const float* __restrict__ 
 // routes a whole decode batch: about a fifth of the instructions of the shared-memory form. Same total order (value descending,
 // id ascending), same double-precision weights. Full-softmax weights without renormalisation need the serial ascending-id sum
 // and stay with route_row.
-__device__ __forceinline__ void route_row_regs(const float* __restrict__ src, uint32_t token, uint32_t experts, uint32_t selected,
+__device__ __forceinline__ void route_row_regs(const float* src, uint32_t token, uint32_t experts, uint32_t selected,
                                                uint32_t mode, uint32_t* __restrict__ ids, float* __restrict__ weights, uint32_t* error,
                                                uint32_t lane) {
     float v[16];
@@ -165,7 +165,7 @@ __device__ __forceinline__ void route_row_regs(const float* __restrict__ src, ui
 }
 
 __global__ void __launch_bounds__(kRouteWarps * 32)
-route_kernel(const float* __restrict__ logits, uint64_t stride_bytes, uint32_t tokens, uint32_t experts,
+route_kernel(const float* logits, uint64_t stride_bytes, uint32_t tokens, uint32_t experts,
              uint32_t selected, uint32_t mode, int normalize, uint32_t* __restrict__ ids,
              float* __restrict__ weights, uint32_t* error, float* __restrict__ margins) {
     pdl_launch_dependents();
@@ -187,7 +187,7 @@ constexpr int kPermuteThreads = 512;
 constexpr uint32_t kPermuteExperts = 2;   // experts per block: a token's ids are read once for all of them
 
 __global__ void __launch_bounds__(kPermuteThreads)
-grouped_routes_kernel(const uint32_t* __restrict__ ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t first, int local_only,
+grouped_routes_kernel(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t first, int local_only,
                       uint32_t* __restrict__ token_map, uint32_t* __restrict__ counts, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
@@ -242,7 +242,7 @@ grouped_routes_kernel(const uint32_t* __restrict__ ids, uint32_t tokens, uint32_
 
 // tasks = {live_tiles, routes, (expert, start) pairs in ascending expert order, 0xffffffff padding}
 __global__ void __launch_bounds__(256)
-grouped_tasks_kernel(const uint32_t* __restrict__ counts, uint32_t tokens, uint32_t experts, uint32_t selected,
+grouped_tasks_kernel(const uint32_t* counts, uint32_t tokens, uint32_t experts, uint32_t selected,
                      uint32_t tile, uint32_t bound, int local_only, uint32_t* __restrict__ tasks, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
@@ -305,9 +305,9 @@ constexpr int kPrologueRouteWarps = 4;
 constexpr uint32_t kPrologueTokens = 1024, kPrologueExperts = 1024;
 
 __global__ void __launch_bounds__(kPrologueRouteWarps * 32)
-decode_route_kernel(const float* __restrict__ logits, uint64_t logits_stride, uint32_t tokens, uint32_t experts, uint32_t selected,
+decode_route_kernel(const float* logits, uint64_t logits_stride, uint32_t tokens, uint32_t experts, uint32_t selected,
                     uint32_t mode, int normalize, uint32_t route_blocks, uint32_t* __restrict__ ids, float* __restrict__ weights,
-                    const __half* __restrict__ x16, uint64_t x16_stride, float* __restrict__ x32, uint64_t x32_stride, uint32_t channels,
+                    const __half* x16, uint64_t x16_stride, float* __restrict__ x32, uint64_t x32_stride, uint32_t channels,
                     uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
@@ -335,7 +335,7 @@ decode_route_kernel(const float* __restrict__ logits, uint64_t logits_stride, ui
 // expert in shared memory), positions = number of lower set bits. ids are global; this launch owns experts [first, first + experts);
 // with local_only, routes to other owners are skipped, without it they are an index error.
 __global__ void __launch_bounds__(kPrologueThreads)
-tables_kernel(const uint32_t* __restrict__ ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
+tables_kernel(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
               uint32_t words, uint32_t* __restrict__ token_map, uint32_t* __restrict__ counts, uint32_t* __restrict__ tasks, uint32_t* error) {
     pdl_launch_dependents();
     extern __shared__ uint32_t tables_mask[];   // [experts][words]
@@ -435,9 +435,9 @@ constexpr int kCombineThreads = 256;
 // R16: the route rows are binary16 (the prefill path keeps them so); X16: the input rows of the shared-router dot are binary16.
 template <bool R16, bool X16>
 __global__ void __launch_bounds__(kCombineThreads)
-combine_kernel(const void* __restrict__ routed, uint64_t routed_stride, const float* __restrict__ weights,
-               const float* __restrict__ shared, uint64_t shared_stride, const float* __restrict__ shared_router,
-               const void* __restrict__ x, uint64_t x_stride, float* shared_logit, uint32_t channels,
+combine_kernel(const void* routed, uint64_t routed_stride, const float* weights,
+               const float* shared, uint64_t shared_stride, const float* shared_router,
+               const void* x, uint64_t x_stride, float* shared_logit, uint32_t channels,
                uint32_t selected, float* __restrict__ out, uint64_t out_stride, __half* __restrict__ out16,
                uint64_t out16_stride, int vec4, uint32_t* error) {
     pdl_launch_dependents();
@@ -573,7 +573,7 @@ combine_kernel(const void* __restrict__ routed, uint64_t routed_stride, const fl
 // F32 matrix-vector product for the router projections: one warp per (matrix row, token), FP32 FMA + tree sum.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-gemv_f32_kernel(const float* __restrict__ w, uint32_t rows, uint32_t cols, const float* __restrict__ x, uint64_t x_stride, uint32_t tokens,
+gemv_f32_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, uint64_t x_stride, uint32_t tokens,
                 float* __restrict__ out, uint64_t out_stride, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
@@ -601,7 +601,7 @@ gemv_f32_kernel(const float* __restrict__ w, uint32_t rows, uint32_t cols, const
 constexpr int kRgM = 64, kRgN = 128, kRgK = 16, kRgThreads = 256;
 
 __global__ void __launch_bounds__(kRgThreads)
-router_gemm_kernel(const float* __restrict__ w, uint32_t rows, uint32_t cols, const float* __restrict__ extra, const float* __restrict__ x,
+router_gemm_kernel(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x,
                    uint64_t x_stride, uint32_t tokens, float* __restrict__ out, uint64_t out_stride, float* __restrict__ extra_out, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
@@ -679,7 +679,7 @@ constexpr int kSgT = 128, kSgK = 16, kSgThreads = 256;
 // (ms): this form 0.278; 128 x 128 tiles with 8 x 8 outputs (one block per SM, 128 blocks) 0.402; packed FP32 FMAs 0.280
 // (the kernel is not bound by issue slots); a warp-broadcast mapping with 16 x 4 outputs 0.415.
 __global__ void __launch_bounds__(kSgThreads, 2)
-router_sgemm_kernel(const float* __restrict__ w, uint32_t rows, uint32_t cols, const float* __restrict__ x, uint64_t x_stride, uint32_t tokens,
+router_sgemm_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, uint64_t x_stride, uint32_t tokens,
                     float* __restrict__ out, uint64_t out_stride, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
@@ -770,7 +770,7 @@ int launch_gemv_f32(const float* w, uint32_t rows, uint32_t cols, const float* e
     return TSP_OK;
 }
 
-__global__ void rows_f16_to_f32_kernel(const __half* __restrict__ in, uint64_t in_stride, float* __restrict__ out,
+__global__ void rows_f16_to_f32_kernel(const __half* in, uint64_t in_stride, float* __restrict__ out,
                                        uint64_t out_stride, uint32_t rows, uint32_t cols) {
     pdl_launch_dependents();
     pdl_wait();
@@ -785,7 +785,7 @@ __global__ void rows_f16_to_f32_kernel(const __half* __restrict__ in, uint64_t i
 // dequantise test hook: FP32 fmaf(d*sc, q, -(dmin*mn)) is the exactly rounded reference value
 // because d*sc, (d*sc)*q and dmin*mn are exact in FP32 (at most 21 significant bits).
 // ---------------------------------------------------------------------------------------------
-__global__ void dequant_q4k_kernel(const uint8_t* __restrict__ expert, uint32_t layout, uint64_t total_blocks,
+__global__ void dequant_q4k_kernel(const uint8_t* expert, uint32_t layout, uint64_t total_blocks,
                                    float* __restrict__ out, uint32_t* error) {
     const uint64_t blk = blockIdx.x;
     const uint32_t i = threadIdx.x;  // 0..255
@@ -814,7 +814,7 @@ __global__ void dequant_q4k_kernel(const uint8_t* __restrict__ expert, uint32_t 
     out[blk * 256 + i] = v;
 }
 
-__global__ void dequant_q8_kernel(const uint8_t* __restrict__ expert, uint32_t layout, uint64_t total_blocks,
+__global__ void dequant_q8_kernel(const uint8_t* expert, uint32_t layout, uint64_t total_blocks,
                                   float* __restrict__ out, uint32_t* error) {
     const uint64_t blk = static_cast<uint64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5);
     if (blk >= total_blocks) return;

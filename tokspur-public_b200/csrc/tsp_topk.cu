@@ -103,7 +103,7 @@ __device__ unsigned long long topk_ranked(TopkShared& sh, unsigned long long* ra
 }
 
 __global__ void __launch_bounds__(kTopkThreads)
-logit_topk_tiles_kernel(const float* __restrict__ logits, uint64_t stride, uint32_t vocabulary, uint32_t tiles, uint32_t* __restrict__ partial) {
+logit_topk_tiles_kernel(const float* logits, uint64_t stride, uint32_t vocabulary, uint32_t tiles, uint32_t* __restrict__ partial) {
     pdl_launch_dependents();
     __shared__ TopkShared sh;
     __shared__ unsigned long long ranked[kTopkCap];
@@ -164,7 +164,7 @@ logit_topk_tiles_kernel(const float* __restrict__ logits, uint64_t stride, uint3
 
 template <bool REGS>
 __global__ void __launch_bounds__(kTopkThreads)
-logit_topk_merge_kernel(const uint32_t* __restrict__ partial, uint32_t vocabulary, uint32_t tiles, uint32_t* __restrict__ rows_out) {
+logit_topk_merge_kernel(const uint32_t* partial, uint32_t vocabulary, uint32_t tiles, uint32_t* __restrict__ rows_out) {
     pdl_launch_dependents();
     __shared__ TopkShared sh;
     __shared__ unsigned long long ranked[kTopkCap];
