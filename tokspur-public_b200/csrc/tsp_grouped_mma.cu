@@ -1,22 +1,28 @@
 // Prefill-size grouped expert GEMMs on the 5th-generation tensor cores (tcgen05) for sm_100a.
 //
-// One launch computes, for every task of <= 256 routes of one expert (two sub-tiles of <= 128 token columns), either
+// One launch computes, for every task of <= 256 routes of one expert (worked on as sub-tiles of <= 128 token columns), either
 //   gate-up:  H[pos][h]   = silu(W_gate[h] . x[token]) * (W_up[h] . x[token])
 //   down:     Y[route][c] = W_down[c] . H[pos]
 // with the weights as the M operand (128 weight rows per item fill the MMA's M extent whatever the number of tokens), the
 // tokens as the N operand (32, 64 or 128 columns per sub-tile) and K walked in chunks of 64.
 //
-//   * A dequantised weight chunk is used for BOTH sub-tiles of a task before it is released: an expert with many routes
-//     pays the dequantisation once per 256 routes. Each sub-tile has its own accumulator (128 columns of tensor memory);
-//     two such pairs are double-buffered (512 columns), so the epilogue of an item runs under the MMAs of the next.
-//   * One pipeline stage = one K chunk = {dequantised weight chunk, activation tile of sub-tile 0, of sub-tile 1}, filled by
-//     the dequant warps and the activation producer, emptied by ONE commit. The thread that issues the MMAs does one wait,
-//     four MMAs (N = 256 when both sub-tiles are full: their tiles are adjacent) and one commit per chunk: with separate rings
-//     for weights and activations its waits and commits, not the tensor pipe, set the pace (measured: removing the MMAs
-//     altogether made the launch only 30 % shorter).
+//   * What bounds it: with loads skewed over 512 experts most sub-tiles hold fewer than 32 routes, so the work is dequantising
+//     weights, not multiplying. The dequantised chunk therefore goes to TENSOR memory (`tcgen05.st`, the A operand of the MMA), not to
+//     shared memory: a chunk in shared memory is 16 KB written and 16 KB read back by the MMA at 128 bytes a cycle, as much again as
+//     everything else on its way. It also frees the room for eight stages (three before) and four super-blocks in flight (two before).
+//   * Two accumulators of 128 columns are double-buffered (256 columns; the other 256 hold the weight stages), so the epilogue of a
+//     sub-tile runs under the MMAs of the next. A task of more than 128 routes dequantises once per sub-tile: under its MMAs, for
+//     nothing (N = 128 from tensor memory reads 64 bytes of shared memory a cycle, the tensor pipe's own pace).
+//   * One pipeline stage = one K chunk = {weight chunk in tensor memory, activation tile in shared memory}, filled by the dequant
+//     warps and the activation producer, emptied by ONE commit.
+//   * MMAs and copies are issued by whole warps with uniform arguments and `elect.sync`. Issued from a `lane == 0` branch they cost
+//     about 100 cycles each (operands moved to uniform registers under a loop over the lanes the compiler cannot rule out): with
+//     the rest in place, 470 k of the 731 k cycles of the 4096-row gate-up launch; 485 k in all without it.
+//   * Measured (layer with 512 experts of 512 x 2048, ten per token, Zipf loads, whole layer): 4096 rows 761 -> 646 us, 1003 rows
+//     (dense Q8_0 shared expert) 430 -> 318 us, 160 rows 180 -> 115 us.
 //   * Gate-up items hold 64 hidden units as 128 A rows: inside every group of 32 rows (one tensor-memory lane quarter)
 //     rows 0..15 are gate rows and rows 16..31 the up rows of the same 16 units, so SwiGLU is a lane exchange inside one
-//     warp and one accumulator serves both matrices (a 16 KB A stage per chunk, four stages).
+//     warp and one accumulator serves both matrices.
 //   * Activation tiles are plain tile copies (one `cp.async.bulk.tensor` per tile and K chunk) of rows kept in permuted
 //     position order: the routed copy of the input rows for gate-up (written once per layer by `gather_rows16_kernel`; the
 //     shared expert's tasks read the input rows themselves), the hidden rows for down. Fetching rows by token id inside the
@@ -28,14 +34,15 @@
 // Roles inside a CTA (one persistent CTA per SM):
 //   warp 0      TMA producer of the quantised planes: Pack v3 planar code lines + 6-bit factor bytes of one super-block
 //               (256 columns of K) per quant stage; the (d, dmin) pairs once per item.
-//   warp 1      allocates tensor memory, issues tcgen05.mma (one elected lane), commits to mbarriers.
-//   warps 2..9  dequantise: a thread owns one weight row and every other K chunk (threads 0..127 the even chunks, 128..255
-//               the odd ones): 32 code bytes -> 64 binary16 weights written as one 128-byte row of the K-major,
-//               128-byte-swizzled operand tile. Per group of 32 weights the value staged is
+//   warp 1      allocates tensor memory, issues tcgen05.mma, commits to mbarriers.
+//   warps 2..17 dequantise, four groups of four warps: a thread owns one weight row and every fourth K chunk: 32 code bytes -> 64
+//               binary16 weights in 32 registers -> its lane's 32 columns of the stage. (Two groups: 698 / 354 / 130 us.)
+//               Per group of 32 weights the value staged is
 //               RN16((q - 8) * RN16(d*sc) + RN16(8*d*sc - dmin*mn)): the centred code keeps the products small, so the three
 //               roundings cost about 1.5x the error of rounding the exact value once (measured by the tile hook below).
-//   warp 10     activation producer.
-//   warps 11..18 epilogue (two per tensor-memory lane quarter): tcgen05.ld of their 32 accumulator lanes, SwiGLU / store.
+//   warp 18     activation producer.
+//   warps 19..26 epilogue (two per tensor-memory lane quarter): tcgen05.ld of their 32 accumulator lanes, SwiGLU / store.
+//   warp 27     item hand-out.
 // Accumulation is FP32 in tensor memory. Operands are binary16 (kind::f16, f16 inputs): the activations of this path are
 // binary16-exact, and Q4_K values keep 11 significant bits instead of bf16's 8.
 // Every mbarrier wait is bounded; a timeout sets TSP_ERR_TIMEOUT, and every path still frees the tensor memory.
@@ -62,13 +69,41 @@ __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence:
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem desc] * B[smem desc], kind::f16, one CTA
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// One K chunk of 64: four D[tmem] (+)= A[tmem] * B[smem], kind::f16, one CTA, then a commit on `bar` (it completes when the MMAs have
+// read their operands). Called by a whole warp with uniform arguments; one elected lane issues. (A lane picked by `lane == 0` in
+// front of separate instructions cost about 400 cycles per chunk: the compiler cannot know that one thread is left and serialises
+// every operand's move to a uniform register.) b_lo: low word of the K-major 128-byte-swizzle descriptor of the activation tile.
+constexpr uint32_t kUmmaDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);   // stride 1024 bytes per eight rows, version 1, SWIZZLE_128B
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
+__device__ __forceinline__ void umma_chunk_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t idesc, uint32_t accumulate, uint32_t bar) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q, t;\n\t.reg .b64 b0, b1, b2, b3;\n\t.reg .b32 a1, a2, a3, l1, l2, l3;\n\t"
+        "setp.ne.b32 q, %4, 0;\n\tsetp.eq.b32 t, 0, 0;\n\t"
+        "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+        "add.u32 l1, %2, 2;\n\tadd.u32 l2, %2, 4;\n\tadd.u32 l3, %2, 6;\n\t"
+        "mov.b64 b0, {%2, %6};\n\tmov.b64 b1, {l1, %6};\n\tmov.b64 b2, {l2, %6};\n\tmov.b64 b3, {l3, %6};\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "@p tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b0, %3, q;\n\t"
+        "@p tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, t;\n\t"
+        "@p tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, t;\n\t"
+        "@p tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, t;\n\t"
+        "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(bar), "n"(kUmmaDescHi) : "memory");
 }
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+// 32 registers per thread -> 32 lanes x 32 consecutive columns (the warp's own lane quarter)
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+                   "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+                   "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // arrive on an mbarrier when all MMAs issued so far by this thread have completed
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -99,27 +134,27 @@ __device__ __forceinline__ void tma_load_5d_g(void* smem_dst, const CUtensorMap*
                  : "memory");
 }
 
-// Shared-memory matrix descriptor of a K-major operand tile whose rows are 128 bytes (64 binary16) in the 128-byte swizzle:
-// start address >> 4, leading byte offset (unused for this layout) 1, stride byte offset 1024 (eight rows), descriptor
-// version 1 (sm_100), layout type 2 (SWIZZLE_128B).
-__device__ __forceinline__ uint64_t umma_desc_k128(const void* smem_tile) {
-    const uint64_t addr = smem_u32(smem_tile);
-    return ((addr & 0x3FFFFull) >> 4) | (1ull << 16) | (uint64_t(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
-}
 // Instruction descriptor for kind::f16: D = FP32, A = B = binary16, both K-major, M x N tile.
 __host__ __device__ constexpr uint32_t umma_idesc_f16(uint32_t m, uint32_t n) {
     return (1u << 4) | (0u << 7) | (0u << 10) | (0u << 15) | (0u << 16) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
 
-constexpr uint32_t kDqWarps = 8;           // dequantise warps: 256 threads = 128 weight rows x {even, odd} K chunks
+constexpr uint32_t kDqWarps = 16;          // dequantise warps: four groups of 128 threads (weight rows), each taking every fourth K chunk
+constexpr uint32_t kDqGroups = kDqWarps / 4;
 constexpr uint32_t kEpWarps = 8;           // epilogue warps: two per tensor-memory lane quarter, taking the 32-column batches in turn
-constexpr uint32_t kGWarps = 3 + kDqWarps + kEpWarps;   // weight producer, MMA, dequant warps, activation producer, epilogue warps
+constexpr uint32_t kGWarps = 4 + kDqWarps + kEpWarps;   // weight producer, MMA, dequant warps, activation producer, epilogue warps, item hand-out
 constexpr uint32_t kTaskRoutes = TSP_GROUPED_TILE;      // routes per task (two sub-tiles)
 constexpr uint32_t kSub = 128;             // token columns per sub-tile (N extent at most)
 constexpr uint32_t kRowsM = 128;           // A rows per item (M)
-constexpr uint32_t kStages = 3;            // K chunks in flight: a stage holds the dequantised weight chunk AND the activation tiles it meets
-constexpr uint32_t kStageBytes = 3 * 16384;   // [A: 128 rows x 128 B][B sub-tile 0][B sub-tile 1]
-constexpr uint32_t kEpTileBytes = 32 * 144;   // per epilogue warp: 32 token rows of 32 FP32 values, rows padded by 16 bytes
+constexpr uint32_t kStages = 8;            // K chunks in flight: dequantised weight chunk (tensor memory) and the activation tile it meets (shared memory)
+constexpr uint32_t kStageBytes = 16384;    // activation tile: up to 128 rows x 128 B
+constexpr uint32_t kAccCols = 128;         // tensor-memory columns of one accumulator; two of them, then the weight stages
+constexpr uint32_t kACols = 32;            // columns of one weight stage: 64 binary16 values of K per lane (= weight row)
+constexpr uint32_t kQuant = 4;             // quantised super-blocks in flight
+static_assert(2 * kAccCols + kStages * kACols == 512 && kStages % kDqGroups == 0, "tensor memory holds two accumulators and the weight stages");
+// per epilogue warp: 32 token rows of 16 hidden units (gate-up) or 32 channels (down) in binary16, or 16 rows of 32 FP32 values,
+// rows padded by 16 bytes
+__host__ __device__ constexpr uint32_t ep_tile_bytes(bool gateup) { return gateup ? 32 * 48 : 32 * 80; }
 static_assert(kTaskRoutes == 2 * kSub, "a task is two sub-tiles");
 
 // Tensor maps of one launch: codes / factor bytes / (d, dmin) pairs with index 0 matrix A low ids, 1 A high ids, 2 B low ids,
@@ -133,7 +168,7 @@ struct GroupedParams {
     uint32_t chunks;               // K chunks of 64 per item
     uint32_t row_blocks;           // items per task: hidden / 64 (gate-up) or rows / 128 (down)
     uint32_t merged, sh_merged;    // both matrices of an expert arrive with one copy per plane (routed experts; shared expert)
-    // optional dense shared expert processed by the same launch after the routed tasks: every one of sh_tokens rows, in
+    // optional dense shared expert processed by the same launch before the routed tasks: every one of sh_tokens rows, in
     // row order (position = token = route id)
     uint32_t sh_tasks, sh_tokens;
     void* sh_out; uint64_t sh_out_stride_bytes;
@@ -149,6 +184,7 @@ struct GroupedParams {
     uint32_t* error;
     uint32_t* work_counter;        // next item index; zero when the launch starts (tsp_moe_route_offsets clears it)
     // shared-memory plan
+    uint32_t n_quant;              // quantised super-blocks in flight: kQuant, or one less beside the (d, dmin) pairs of a long K
     uint32_t off_q, q_stage_bytes, off_d, d_stage_bytes, dm_mat_bytes, off_st, off_ep;
 };
 
@@ -160,25 +196,23 @@ struct GTask { uint32_t expert, start, count, row0; };
 // A task of the shared expert carries the expert id p.experts (one past the routed ids).
 __device__ __forceinline__ GTask gtask(const GroupedParams& p, uint32_t task) {
     GTask t;
-    const uint32_t routed = p.tasks ? p.tasks[0] : 0u;
-    if (task >= routed) {
+    if (task < p.sh_tasks) {
         t.expert = p.experts;
-        t.start = (task - routed) * kTaskRoutes;
+        t.start = task * kTaskRoutes;
         t.count = t.start < p.sh_tokens ? min(p.sh_tokens - t.start, kTaskRoutes) : 0u;
         t.row0 = t.start;
         return t;
     }
+    task -= p.sh_tasks;
     t.expert = p.tasks[2 + 2 * task];
     t.start = p.tasks[3 + 2 * task];
     if (t.expert >= p.experts) { t.expert = 0; t.start = 0; t.count = 0; t.row0 = 0; return t; }
-    const uint32_t c = p.counts[t.expert];
+    const uint32_t c = p.counts[t.expert], at = p.offsets[t.expert];
     t.count = c > t.start ? min(c - t.start, kTaskRoutes) : 0u;
-    t.row0 = p.offsets[t.expert] + t.start;
+    t.row0 = at + t.start;
     return t;
 }
-__device__ __forceinline__ uint32_t sub_count(const GTask& t, uint32_t g) { return g == 0 ? min(t.count, kSub) : (t.count > kSub ? t.count - kSub : 0u); }
 __device__ __forceinline__ uint32_t sub_cols(uint32_t count) { return count <= 32 ? 32u : (count <= 64 ? 64u : 128u); }
-__device__ __forceinline__ uint32_t sub_tiles(const GTask& t) { return t.count > kSub ? 2u : 1u; }
 
 // ---------------------------------------------------------------------------------------------
 // dequantisation of one 64-wide K chunk of one weight row (shared by the GEMM kernel and the tile hook)
@@ -223,22 +257,27 @@ __device__ __forceinline__ void dequant8(uint32_t a, uint32_t b, const ChunkScal
     hi = make_uint4(h[0], h[1], h[2], h[3]);
 }
 
-// Item hand-out. One thread (the weight producer) takes the next item index from the global counter, looks its task up and
-// publishes both in a ring of kSched slots; the other 18 warps read it (one arrival per warp frees the slot). An index
-// >= n_items ends every role.
+// Item hand-out. One thread of a warp of its own takes the next item index from the global counter, looks its task up and
+// publishes both in a ring of kSched slots; the other 27 warps read it (one arrival per warp frees the slot). An index
+// >= n_items ends every role. The counter and the three dependent table reads take about 2000 cycles: done by the weight
+// producer between its copies, they stood in front of every item's first byte (a down item is eight chunks of work). The next
+// index is taken when the weight producer is two super-blocks from the end of its item, not earlier: items that wait in a CTA's
+// ring while other CTAs run dry cost more than the latency they hide. The dense tasks, the heaviest ones, come first.
 constexpr uint32_t kSched = 4;
-constexpr uint32_t kSchedReaders = 2 + kDqWarps + kEpWarps;   // MMA issuer, activation producer, dequant warps, epilogue warps
+constexpr uint32_t kSchedReaders = 3 + kDqWarps + kEpWarps;   // weight producer, MMA issuer, activation producer, dequant warps, epilogue warps
 struct SchedItem { uint32_t item; GTask t; };
 struct SchedReader {
     uint64_t* full; uint64_t* empty; const volatile uint32_t* slots;   // 8 words per slot: item, expert, start, count, row0
     uint32_t s = 0, ph = 0;
     // every lane of the warp calls this; item 0xffffffff when a bounded wait expired
     __device__ __forceinline__ SchedItem next(uint32_t lane) {
-        const bool ok = mbar_wait(&full[s], ph, 1u << 21);
+        const bool ok = __all_sync(0xffffffffu, mbar_wait(&full[s], ph, 1u << 21));
         SchedItem it;
         const volatile uint32_t* w = slots + s * 8;
-        it.item = ok ? w[0] : 0xffffffffu;
-        it.t.expert = w[1]; it.t.start = w[2]; it.t.count = w[3]; it.t.row0 = w[4];
+        const uint32_t v = ok && lane < 5 ? w[lane] : 0xffffffffu;   // broadcast: uniform values
+        it.item = __shfl_sync(0xffffffffu, v, 0);
+        it.t.expert = __shfl_sync(0xffffffffu, v, 1); it.t.start = __shfl_sync(0xffffffffu, v, 2);
+        it.t.count = __shfl_sync(0xffffffffu, v, 3); it.t.row0 = __shfl_sync(0xffffffffu, v, 4);
         __syncwarp();
         if (lane == 0 && ok) mbar_arrive(&empty[s]);
         if (++s == kSched) { s = 0; ph ^= 1u; }
@@ -258,34 +297,38 @@ struct SchedReader {
 //               so odd spans are fetched from 8 bytes earlier and read from byte 8 of the line.
 constexpr int kEncPlanar = 0, kEncGguf = 1, kEncQ8 = 2;
 
-// One Q8_0 chunk (two blocks = 68 bytes starting at word WS of the 20 words `L`) -> the chunk's 128-byte A row. Block 0 starts on
-// a word boundary (scale in the low half-word, codes two bytes off: realigned with funnel shifts), block 1 two bytes past one
-// (scale in the high half-word, codes word-aligned). A code byte b becomes binary16 through 0x6400 | (b ^ 0x80) = 1152 + q, the
-// subtraction is exact and d * q is rounded once: the staged value is RN16 of the exact weight.
-template <uint32_t WS>
-__device__ __forceinline__ bool q8_chunk_row(const uint32_t (&L)[20], uint8_t* arow, uint32_t sw) {
+// One Q8_0 chunk (two blocks = 68 bytes starting at word `ws` of the 20 words at `src`, 16-byte aligned) -> its 64 weights in operand
+// order. Block 0 starts on a word boundary (scale in the low half-word, codes two bytes off: realigned with funnel shifts), block 1
+// two bytes past one (scale in the high half-word, codes word-aligned). A code byte b becomes binary16 through
+// 0x6400 | (b ^ 0x80) = 1152 + q, the subtraction is exact and d * q is rounded once: the staged value is RN16 of the exact weight.
+// The word offset is resolved with selects, not with a copy of the code for each.
+__device__ __forceinline__ bool q8_chunk(const uint8_t* src, uint32_t ws, uint32_t (&out)[32]) {
     const __half2 k1152 = __float2half2_rn(1152.f);
-    const uint32_t s0 = L[WS] & 0xffffu, s1 = L[WS + 8] >> 16;
-    const bool finite = (s0 & 0x7c00u) != 0x7c00u && (s1 & 0x7c00u) != 0x7c00u;
+    uint32_t L[20];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) { const uint4 v = reinterpret_cast<const uint4*>(src)[i]; L[4 * i] = v.x; L[4 * i + 1] = v.y; L[4 * i + 2] = v.z; L[4 * i + 3] = v.w; }
+#pragma unroll
+    for (int i = 0; i < 19; ++i) L[i] = ws & 1u ? L[i + 1] : L[i];
+#pragma unroll
+    for (int i = 0; i < 17; ++i) L[i] = ws & 2u ? L[i + 2] : L[i];
+    const uint32_t s0 = L[0] & 0xffffu, s1 = L[8] >> 16;
     const uint32_t dw0 = s0 | (s0 << 16), dw1 = s1 | (s1 << 16);
     const __half2 d0 = *reinterpret_cast<const __half2*>(&dw0), d1 = *reinterpret_cast<const __half2*>(&dw1);
 #pragma unroll
     for (uint32_t u = 0; u < 8; ++u) {          // unit u: K positions 8u .. 8u+7 of the chunk
         uint32_t a, b;
-        if (u < 4) { a = __funnelshift_r(L[WS + 2 * u], L[WS + 2 * u + 1], 16); b = __funnelshift_r(L[WS + 2 * u + 1], L[WS + 2 * u + 2], 16); }
-        else { a = L[WS + 9 + 2 * (u - 4)]; b = L[WS + 10 + 2 * (u - 4)]; }
+        if (u < 4) { a = __funnelshift_r(L[2 * u], L[2 * u + 1], 16); b = __funnelshift_r(L[2 * u + 1], L[2 * u + 2], 16); }
+        else { a = L[9 + 2 * (u - 4)]; b = L[10 + 2 * (u - 4)]; }
         a ^= 0x80808080u; b ^= 0x80808080u;
-        const __half2 d = u < 4 ? d0 : d1;
-        uint32_t w[4] = {__byte_perm(a, 0x64646464u, 0x4240), __byte_perm(a, 0x64646464u, 0x4341),
-                         __byte_perm(b, 0x64646464u, 0x4240), __byte_perm(b, 0x64646464u, 0x4341)};
+        const uint32_t w[4] = {__byte_perm(a, 0x64646464u, 0x4240), __byte_perm(a, 0x64646464u, 0x4341),
+                               __byte_perm(b, 0x64646464u, 0x4240), __byte_perm(b, 0x64646464u, 0x4341)};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&w[i]), k1152), d);
-            w[i] = *reinterpret_cast<const uint32_t*>(&v);
+            const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&w[i]), k1152), u < 4 ? d0 : d1);
+            out[4 * u + i] = *reinterpret_cast<const uint32_t*>(&v);
         }
-        *reinterpret_cast<uint4*>(arow + ((u ^ sw) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    return finite;
+    return (s0 & 0x7c00u) != 0x7c00u && (s1 & 0x7c00u) != 0x7c00u;
 }
 
 template <bool GATEUP, int ENC>
@@ -294,28 +337,29 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
     extern __shared__ uint8_t gsm_raw[];
     uint8_t* gsm = gsm_raw + ((1024u - (smem_u32(gsm_raw) & 1023u)) & 1023u);
     uint64_t* bars = reinterpret_cast<uint64_t*>(gsm);
-    // rings: quantised super-blocks (2 stages, TMA), the (d, dmin) pairs of an item (2 stages, TMA), the K-chunk stages
+    // rings: quantised super-blocks (kQuant stages, TMA), the (d, dmin) pairs of an item (2 stages, TMA), the K-chunk stages
     // (weight chunk from the dequant warps + activation tiles by TMA) and the item hand-out
-    uint64_t *qfull = bars, *qempty = bars + 2, *dfull = bars + 4, *dempty = bars + 6, *full = bars + 8, *empty = full + kStages,
-             *acc_full = empty + kStages, *acc_empty = acc_full + 2, *sfull = acc_empty + 2, *sempty = sfull + kSched;
+    uint64_t *qfull = bars, *qempty = qfull + kQuant, *dfull = qempty + kQuant, *dempty = dfull + 2, *full = dempty + 2, *empty = full + kStages,
+             *acc_full = empty + kStages, *acc_empty = acc_full + 2, *sfull = acc_empty + 2, *sempty = sfull + kSched, *want = sempty + kSched;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gsm + 512);
     volatile uint32_t* sched_slots = reinterpret_cast<volatile uint32_t*>(gsm + 640);   // kSched x 8 words
     constexpr uint32_t NMAT = GATEUP ? 2 : 1;
     constexpr uint32_t RM = GATEUP ? 64 : 128;    // rows of ONE matrix in an item
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // warp-uniform for the compiler too
 
     if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < kQuant; ++s) { mbar_init(&qfull[s], 1); mbar_init(&qempty[s], kDqWarps); }
         for (int s = 0; s < 2; ++s) {
-            mbar_init(&qfull[s], 1); mbar_init(&qempty[s], kDqWarps);
             mbar_init(&dfull[s], 1); mbar_init(&dempty[s], kDqWarps);
             mbar_init(&acc_full[s], 1); mbar_init(&acc_empty[s], kEpWarps);
         }
         // a stage is full when the four dequant warps that own its chunk have written it and the activation bytes have landed
-        for (uint32_t s = 0; s < kStages; ++s) { mbar_init(&full[s], kDqWarps / 2 + 1); mbar_init(&empty[s], 1); }
+        for (uint32_t s = 0; s < kStages; ++s) { mbar_init(&full[s], kDqWarps / kDqGroups + 1); mbar_init(&empty[s], 1); }
         for (uint32_t s = 0; s < kSched; ++s) { mbar_init(&sfull[s], 1); mbar_init(&sempty[s], kSchedReaders); }
+        mbar_init(want, 1);
         mbar_fence_init();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }   // two sets of two 128-column accumulators
+    if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }   // two accumulators and the weight stages
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -326,50 +370,46 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
     const uint32_t routed_tasks = p.tasks ? p.tasks[0] : 0u;   // no table: a dense launch (the shared expert's tasks only)
     const uint32_t n_tasks = routed_tasks + p.sh_tasks;
     const uint32_t n_items = n_tasks * p.row_blocks;
-    const uint32_t chunks_per_item = p.chunks;     // K chunks of 64 (an even number: a dequant thread's chunk parity is the same in every item)
+    const uint32_t chunks_per_item = p.chunks;     // K chunks of 64 (a multiple of four: K is whole super-blocks)
     SchedReader sched{sfull, sempty, sched_slots};
     uint8_t* const stages = gsm + p.off_st;
 
     if (warp == 0) {
-        // =========================== item hand-out + TMA producer of the quantised planes ===========================
-        if (lane == 0) {
-            bool ok = true;
-            uint32_t qs = 0, qph = 0, ds = 0, dph = 0, cur = 0xffffffffu, ss = 0, sph = 0;
-            GTask t{};
-            while (ok) {
-                ok = gwait(&sempty[ss], sph ^ 1u);
+        // =========================== TMA producer of the quantised planes ===========================
+        bool ok = true;
+        uint32_t qs = 0, qph = 0, ds = 0, dph = 0;
+        for (;;) {
+            const SchedItem it = sched.next(lane);
+            if (it.item >= n_items) { ok = it.item != 0xffffffffu; break; }
+            const GTask& t = it.t;
+            const uint32_t rb = it.item % p.row_blocks;
+            const int r0 = static_cast<int>(rb * RM);
+            const bool shared = t.expert >= p.experts;
+            const bool hi = !shared && t.expert >= p.split;
+            const int el = shared ? 0 : static_cast<int>(hi ? t.expert - p.split : t.expert);
+            const uint32_t mi = shared ? 4u : (hi ? 1u : 0u);                 // map of matrix A; matrix B's is `ms` further
+            const uint32_t ms = shared ? 1u : 2u;
+            const uint32_t ncopy = (NMAT == 1 || (shared ? p.sh_merged : p.merged)) ? 1u : NMAT;
+            if (ENC == kEncPlanar) {
+                // the (d, dmin) pairs of the item's rows over the whole K: RM * nblk * 4 bytes per matrix = lines of 256 bytes
+                ok = __all_sync(0xffffffffu, gwait(&dempty[ds], dph ^ 1u));
                 if (!ok) break;
-                uint32_t item = atomicAdd(p.work_counter, 1u);
-                if (item >= n_items) item = 0xfffffffeu;            // the end marker (0xffffffff is reserved for an expired wait)
-                else if (item / p.row_blocks != cur) { cur = item / p.row_blocks; t = gtask(p, cur); }
-                volatile uint32_t* w = sched_slots + ss * 8;
-                w[0] = item; w[1] = t.expert; w[2] = t.start; w[3] = t.count; w[4] = t.row0;
-                mbar_arrive(&sfull[ss]);
-                if (++ss == kSched) { ss = 0; sph ^= 1u; }
-                if (item >= n_items) break;
-                const uint32_t rb = item % p.row_blocks;
-                const int r0 = static_cast<int>(rb * RM);
-                const bool shared = t.expert >= p.experts;
-                const bool hi = !shared && t.expert >= p.split;
-                const int el = shared ? 0 : static_cast<int>(hi ? t.expert - p.split : t.expert);
-                const uint32_t mi = shared ? 4u : (hi ? 1u : 0u);                 // map of matrix A; matrix B's is `ms` further
-                const uint32_t ms = shared ? 1u : 2u;
-                const uint32_t ncopy = (NMAT == 1 || (shared ? p.sh_merged : p.merged)) ? 1u : NMAT;
-                if (ENC == kEncPlanar) {
-                    // the (d, dmin) pairs of the item's rows over the whole K: RM * nblk * 4 bytes per matrix = lines of 256 bytes
-                    ok = gwait(&dempty[ds], dph ^ 1u);
-                    if (!ok) break;
+                if (elect_one()) {
                     mbar_arrive_expect_tx(&dfull[ds], NMAT * p.dm_mat_bytes);
                     for (uint32_t m = 0; m < ncopy; ++m)
                         tma_load_4d_g(gsm + p.off_d + ds * p.d_stage_bytes + m * p.dm_mat_bytes, &maps.d[mi + ms * m], 0,
                                       static_cast<int>(rb * (p.dm_mat_bytes / 256u)), 0, el, &dfull[ds]);
-                    if (++ds == 2) { ds = 0; dph ^= 1u; }
                 }
-                for (uint32_t sb = 0; sb < p.nblk && ok; ++sb) {
-                    // quant stage: code lines [matrix][RM][128 B], then factor bytes [matrix][RM][16 B]
-                    ok = gwait(&qempty[qs], qph ^ 1u);
-                    if (!ok) break;
-                    uint8_t* q = gsm + p.off_q + qs * p.q_stage_bytes;
+                if (++ds == 2) { ds = 0; dph ^= 1u; }
+            }
+            const uint32_t ask = p.nblk > 2 ? p.nblk - 2 : 0u;
+            for (uint32_t sb = 0; sb < p.nblk; ++sb) {
+                // quant stage: code lines [matrix][RM][128 B], then factor bytes [matrix][RM][16 B]
+                ok = __all_sync(0xffffffffu, gwait(&qempty[qs], qph ^ 1u));
+                if (!ok) break;
+                uint8_t* q = gsm + p.off_q + qs * p.q_stage_bytes;
+                if (elect_one()) {
+                    if (sb == ask) mbar_arrive(want);   // time to fetch the next item
                     mbar_arrive_expect_tx(&qfull[qs], kRowsM * 128u + kRowsM * 16u);
                     if (Q8) {
                         // four blocks of every row: [matrix][RM][144 B]; odd spans start 8 bytes early (16-byte aligned x)
@@ -382,11 +422,12 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                         if (GGUF) tma_load_5d_g(q + kRowsM * 128u + m * (RM * 16u), &maps.f[mi + ms * m], 0, r0, static_cast<int>(sb), 0, el, &qfull[qs]);
                         else tma_load_4d_g(q + kRowsM * 128u + m * (RM * 16u), &maps.f[mi + ms * m], static_cast<int>(sb * 16), r0, 0, el, &qfull[qs]);
                     }
-                    if (++qs == 2) { qs = 0; qph ^= 1u; }
                 }
+                if (++qs == p.n_quant) { qs = 0; qph ^= 1u; }
             }
-            if (!ok) raise_error(p.error, TSP_ERR_TIMEOUT);
+            if (!ok) break;
         }
+        if (!ok && lane == 0) raise_error(p.error, TSP_ERR_TIMEOUT);
     } else if (warp == 2 + kDqWarps) {
         // =========================== activation-tile producer ===========================
         bool ok = true;
@@ -394,76 +435,50 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
         for (;;) {
             const SchedItem it = sched.next(lane);
             if (it.item >= n_items) { ok = it.item != 0xffffffffu; break; }
-            if (lane == 0) {
-                const GTask& t = it.t;
-                const bool shared = t.expert >= p.experts;
-                const uint32_t nsub = sub_tiles(t);
-                const uint32_t nc0 = sub_cols(sub_count(t, 0)), nc1 = sub_cols(sub_count(t, 1));
-                const CUtensorMap* map0 = &maps.x[(shared ? 3 : 0) + (nc0 == 32 ? 0 : (nc0 == 64 ? 1 : 2))];
-                const CUtensorMap* map1 = &maps.x[(shared ? 3 : 0) + (nc1 == 32 ? 0 : (nc1 == 64 ? 1 : 2))];
-                const uint32_t bytes = (nc0 + (nsub > 1 ? nc1 : 0u)) * 128u;
-                for (uint32_t c = 0; c < chunks_per_item && ok; ++c) {
-                    ok = gwait(&empty[st], sph ^ 1u);
-                    if (!ok) break;
-                    uint8_t* b0 = stages + st * kStageBytes + 16384u;
-                    mbar_arrive_expect_tx(&full[st], bytes);
+            const uint32_t nc = sub_cols(it.t.count);
+            const CUtensorMap* map = &maps.x[(it.t.expert >= p.experts ? 3 : 0) + (nc == 32 ? 0 : (nc == 64 ? 1 : 2))];
+            for (uint32_t c = 0; c < chunks_per_item; ++c) {
+                ok = __all_sync(0xffffffffu, gwait(&empty[st], sph ^ 1u));
+                if (!ok) break;
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&full[st], nc * 128u);
                     // byte coordinate: the map's element is a byte
-                    tma_load_2d(b0, map0, static_cast<int>(c * 128), static_cast<int>(t.row0), &full[st]);
-                    if (nsub > 1) tma_load_2d(b0 + 16384u, map1, static_cast<int>(c * 128), static_cast<int>(t.row0 + kSub), &full[st]);
-                    if (++st == kStages) { st = 0; sph ^= 1u; }
+                    tma_load_2d(stages + st * kStageBytes, map, static_cast<int>(c * 128), static_cast<int>(it.t.row0), &full[st]);
                 }
+                if (++st == kStages) { st = 0; sph ^= 1u; }
             }
-            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
-            st = __shfl_sync(0xffffffffu, st, 0); sph = __shfl_sync(0xffffffffu, sph, 0);
         }
         if (!ok && lane == 0) raise_error(p.error, TSP_ERR_TIMEOUT);
     } else if (warp == 1) {
         // =========================== MMA issuer ===========================
         bool ok = true;
         uint32_t st = 0, sph = 0, ab = 0, accph = 0;
+        const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0), b_lo0 = umma_desc_lo(smem_u32(stages)), empty0 = smem_u32(empty);
         for (;;) {
             const SchedItem it = sched.next(lane);
             if (it.item >= n_items) { ok = it.item != 0xffffffffu; break; }
-            if (lane == 0) {
-                const GTask& t = it.t;
-                const uint32_t nsub = sub_tiles(t);
-                const uint32_t nc0 = sub_cols(sub_count(t, 0)), nc1 = sub_cols(sub_count(t, 1));
-                const bool wide = nsub > 1 && nc1 == kSub;          // both sub-tiles full: one N = 256 instruction over the adjacent tiles
-                const uint32_t id0 = umma_idesc_f16(kRowsM, wide ? 256u : nc0), id1 = umma_idesc_f16(kRowsM, nc1);
-                const uint32_t dcol = tmem_base + ab * 256u;
-                ok = gwait(&acc_empty[ab], accph ^ 1u);   // the epilogue has drained this accumulator set (used two items ago)
-                if (ok) tc_fence_after();
-                for (uint32_t c = 0; c < chunks_per_item && ok; ++c) {
-                    ok = gwait(&full[st], sph);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint8_t* sbase = stages + st * kStageBytes;
-                    const uint64_t adesc = umma_desc_k128(sbase), bdesc = umma_desc_k128(sbase + 16384u);
-#pragma unroll
-                    for (uint32_t kk = 0; kk < 4; ++kk) umma_f16(dcol, adesc + kk * 2, bdesc + kk * 2, id0, (c | kk) != 0 ? 1u : 0u);
-                    if (nsub > 1 && !wide) {
-                        const uint64_t bdesc1 = umma_desc_k128(sbase + 32768u);
-#pragma unroll
-                        for (uint32_t kk = 0; kk < 4; ++kk) umma_f16(dcol + kSub, adesc + kk * 2, bdesc1 + kk * 2, id1, (c | kk) != 0 ? 1u : 0u);
-                    }
-                    umma_commit(&empty[st]);   // the stage is free once the MMAs above have read it
-                    if (++st == kStages) { st = 0; sph ^= 1u; }
-                }
-                if (ok) umma_commit(&acc_full[ab]);
-                if (++ab == 2) { ab = 0; accph ^= 1u; }
-            }
-            ok = __all_sync(0xffffffffu, ok);
+            const uint32_t id = umma_idesc_f16(kRowsM, sub_cols(it.t.count));
+            const uint32_t dcol = tmem + ab * kAccCols;
+            ok = __all_sync(0xffffffffu, gwait(&acc_empty[ab], accph ^ 1u));   // the epilogue has drained this accumulator (used two items ago)
             if (!ok) break;
-            st = __shfl_sync(0xffffffffu, st, 0); sph = __shfl_sync(0xffffffffu, sph, 0);
-            ab = __shfl_sync(0xffffffffu, ab, 0); accph = __shfl_sync(0xffffffffu, accph, 0);
+            tc_fence_after();
+            for (uint32_t c = 0; c < chunks_per_item; ++c) {
+                ok = __all_sync(0xffffffffu, gwait(&full[st], sph));
+                if (!ok) break;
+                tc_fence_after();
+                umma_chunk_ts(dcol, tmem + 2 * kAccCols + st * kACols, b_lo0 + st * (kStageBytes >> 4), id, c, empty0 + st * 8u);
+                if (++st == kStages) { st = 0; sph ^= 1u; }
+            }
+            if (!ok) break;
+            if (elect_one()) umma_commit(&acc_full[ab]);
+            if (++ab == 2) { ab = 0; accph ^= 1u; }
         }
         if (!ok && lane == 0) raise_error(p.error, TSP_ERR_TIMEOUT);
     } else if (warp < 2 + kDqWarps) {
         // =========================== dequantise (warps 2 .. 2 + kDqWarps - 1) ===========================
-        const uint32_t dt = threadIdx.x - 64;                 // 0..255
-        const uint32_t half = dt >> 7;                        // which K chunks of every super-block: half, half + 2
-        const uint32_t r = dt & 127u;                         // A row of the item
+        const uint32_t group = (warp - 2) >> 2;               // which K chunk of every super-block
+        const uint32_t r = (warp & 3u) * 32u + lane;          // A row of the item = tensor-memory lane (a warp reaches its own lane quarter)
         // the row's line in the quant stage: gate-up interleaves 16 gate + 16 up rows per lane quarter
         const uint32_t mat = GATEUP ? ((r >> 4) & 1u) : 0u;
         const uint32_t mrow = GATEUP ? ((r >> 5) * 16u + (r & 15u)) : r;          // row inside the matrix's RM rows
@@ -471,8 +486,19 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
         const uint32_t sw = r & 7u;                           // == line & 7
         bool ok = true;
         uint32_t qs = 0, qph = 0, ds = 0, dph = 0;
-        // this thread's chunks are every other one of the launch-wide chunk sequence: its stage advances by two (mod kStages)
-        uint32_t st = half % kStages, sph = 0;
+        // this thread's chunks are every fourth one of the launch-wide chunk sequence: its stage advances by four
+        uint32_t st = group, sph = 0;
+        const uint32_t acol0 = tmem_base + (((warp & 3u) * 32u) << 16) + 2 * kAccCols;
+        auto publish = [&](const uint32_t (&w)[32]) {   // the thread's 64 weights -> its lane of the stage's columns
+            tc_fence_after();
+            tmem_st32(acol0 + st * kACols, w);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[st]);
+            st += kDqGroups;
+            if (st >= kStages) { st -= kStages; sph ^= 1u; }
+        };
         for (;;) {
             const SchedItem it = sched.next(lane);
             if (it.item >= n_items) { ok = it.item != 0xffffffffu; break; }
@@ -480,34 +506,23 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
             const uint8_t* dmp = gsm + p.off_d + ds * p.d_stage_bytes + mat * p.dm_mat_bytes + mrow * p.nblk * 4u;
             for (uint32_t sb = 0; sb < p.nblk; ++sb) {
                 if (ok) ok = gwait(&qfull[qs], qph);
+                ok = __all_sync(0xffffffffu, ok);
                 const uint8_t* q = gsm + p.off_q + qs * p.q_stage_bytes;
                 if (Q8) {
-                    // this thread's chunk of the span: blocks 2 * half, 2 * half + 1 of the row's four
-                    if (ok) ok = gwait(&empty[st], sph ^ 1u);
-                    if (ok) {
-                        const uint4* src = reinterpret_cast<const uint4*>(q + line * 144u) + half * 4u;
-                        uint32_t L[20];
-#pragma unroll
-                        for (int i = 0; i < 5; ++i) { const uint4 v = src[i]; L[4 * i] = v.x; L[4 * i + 1] = v.y; L[4 * i + 2] = v.z; L[4 * i + 3] = v.w; }
-                        uint8_t* arow = stages + st * kStageBytes + r * 128u;
-                        bool finite;
-                        // first word of the chunk among the 20: byte (8 if the span is odd) + 68 * half - 64 * half
-                        switch (half + 2u * (sb & 1u)) {
-                            case 0: finite = q8_chunk_row<0>(L, arow, sw); break;
-                            case 1: finite = q8_chunk_row<1>(L, arow, sw); break;
-                            case 2: finite = q8_chunk_row<2>(L, arow, sw); break;
-                            default: finite = q8_chunk_row<3>(L, arow, sw); break;
+                    // a span is two chunks: the four groups share two spans. This thread's chunk: blocks 2 half, 2 half + 1 of the row's four
+                    if ((sb & 1u) == (group >> 1)) {
+                        const uint32_t half = group & 1u;
+                        if (ok) ok = __all_sync(0xffffffffu, gwait(&empty[st], sph ^ 1u));
+                        if (ok) {
+                            uint32_t w[32];
+                            // first word of the chunk among the 20: byte (8 if the span is odd) + 68 * half - 64 * half
+                            if (!q8_chunk(q + line * 144u + half * 64u, half + 2u * (sb & 1u), w)) raise_error(p.error, TSP_ERR_NONFINITE);
+                            publish(w);
                         }
-                        if (!finite) raise_error(p.error, TSP_ERR_NONFINITE);
-                        fence_async_smem();
                     }
                     __syncwarp();
-                    if (lane == 0 && ok) mbar_arrive(&full[st]);
-                    st += 2;
-                    if (st >= kStages) { st -= kStages; sph ^= 1u; }
-                    __syncwarp();
                     if (lane == 0 && ok) mbar_arrive(&qempty[qs]);
-                    if (++qs == 2) { qs = 0; qph ^= 1u; }
+                    if (++qs == p.n_quant) { qs = 0; qph ^= 1u; }
                     continue;
                 }
                 // d, dmin and the sixteen 6-bit factors of this row's super-block
@@ -527,34 +542,25 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                 const float dd = half_bits_to_float(dmw & 0xffffu), dmn = half_bits_to_float(dmw >> 16);
                 if (ok && (!finite_f32(dd) || !finite_f32(dmn))) raise_error(p.error, TSP_ERR_NONFINITE);
                 const uint8_t* codes = q + line * 128u;
+                if (ok) ok = __all_sync(0xffffffffu, gwait(&empty[st], sph ^ 1u));  // the MMAs that read this stage kStages chunks ago are done
+                if (ok) {
+                    const ChunkScale cs = chunk_scale(dd, dmn, group & 2u ? fac.y : fac.x, group & 2u ? fac.w : fac.z, 2u * (group & 1u));
+                    const uint4 w0 = *reinterpret_cast<const uint4*>(codes + (((2 * group) ^ sw) << 4));
+                    const uint4 w1 = *reinterpret_cast<const uint4*>(codes + (((2 * group + 1) ^ sw) << 4));
+                    const uint32_t cw[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+                    uint32_t w[32];
 #pragma unroll
-                for (uint32_t pp = 0; pp < 2; ++pp) {
-                    const uint32_t c = 2 * pp + half;          // chunk of the super-block
-                    if (ok) ok = gwait(&empty[st], sph ^ 1u);  // the MMAs that read this stage kStages chunks ago are done
-                    if (ok) {
-                        const ChunkScale cs = chunk_scale(dd, dmn, pp ? fac.y : fac.x, pp ? fac.w : fac.z, 2u * half);
-                        const uint4 w0 = *reinterpret_cast<const uint4*>(codes + (((2 * c) ^ sw) << 4));
-                        const uint4 w1 = *reinterpret_cast<const uint4*>(codes + (((2 * c + 1) ^ sw) << 4));
-                        uint8_t* arow = stages + st * kStageBytes + r * 128u;
+                    for (uint32_t u = 0; u < 4; ++u) {     // unit u: low nibbles -> K positions 8u.., high nibbles -> 32 + 8u..
                         uint4 lo, hi;
-                        dequant8(w0.x, w0.y, cs, lo, hi);
-                        *reinterpret_cast<uint4*>(arow + ((0u ^ sw) << 4)) = lo; *reinterpret_cast<uint4*>(arow + ((4u ^ sw) << 4)) = hi;
-                        dequant8(w0.z, w0.w, cs, lo, hi);
-                        *reinterpret_cast<uint4*>(arow + ((1u ^ sw) << 4)) = lo; *reinterpret_cast<uint4*>(arow + ((5u ^ sw) << 4)) = hi;
-                        dequant8(w1.x, w1.y, cs, lo, hi);
-                        *reinterpret_cast<uint4*>(arow + ((2u ^ sw) << 4)) = lo; *reinterpret_cast<uint4*>(arow + ((6u ^ sw) << 4)) = hi;
-                        dequant8(w1.z, w1.w, cs, lo, hi);
-                        *reinterpret_cast<uint4*>(arow + ((3u ^ sw) << 4)) = lo; *reinterpret_cast<uint4*>(arow + ((7u ^ sw) << 4)) = hi;
-                        fence_async_smem();   // make the generic-proxy writes visible to the tensor-core (async) proxy
+                        dequant8(cw[2 * u], cw[2 * u + 1], cs, lo, hi);
+                        w[4 * u] = lo.x; w[4 * u + 1] = lo.y; w[4 * u + 2] = lo.z; w[4 * u + 3] = lo.w;
+                        w[16 + 4 * u] = hi.x; w[17 + 4 * u] = hi.y; w[18 + 4 * u] = hi.z; w[19 + 4 * u] = hi.w;
                     }
-                    __syncwarp();
-                    if (lane == 0 && ok) mbar_arrive(&full[st]);
-                    st += 2;
-                    if (st >= kStages) { st -= kStages; sph ^= 1u; }
+                    publish(w);
                 }
                 __syncwarp();
                 if (lane == 0 && ok) mbar_arrive(&qempty[qs]);
-                if (++qs == 2) { qs = 0; qph ^= 1u; }
+                if (++qs == p.n_quant) { qs = 0; qph ^= 1u; }
             }
             if (ENC == kEncPlanar) {
                 __syncwarp();
@@ -565,11 +571,36 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
             if (!ok) break;
         }
         if (!ok && lane == 0) raise_error(p.error, TSP_ERR_TIMEOUT);
+    } else if (warp == kGWarps - 1) {
+        // =========================== item hand-out ===========================
+        if (lane == 0) {
+            bool ok = true;
+            uint32_t ss = 0, sph = 0, n = 0, item = 0;
+            GTask t{};
+            for (;; ++n) {
+                if (n && p.nblk > 2) ok = gwait(want, (n - 1) & 1u);   // short items (K of two super-blocks): the ring is the limit
+                if (ok) ok = gwait(&sempty[ss], sph ^ 1u);
+                if (!ok) break;
+                if (n && t.count > kSub) {                          // the second sub-tile of the same item
+                    t.start += kSub; t.count -= kSub; t.row0 += kSub;
+                } else {
+                    item = atomicAdd(p.work_counter, 1u);
+                    if (item >= n_items) item = 0xfffffffeu;        // the end marker (0xffffffff is reserved for an expired wait)
+                    else t = gtask(p, item / p.row_blocks);
+                }
+                volatile uint32_t* w = sched_slots + ss * 8;
+                w[0] = item; w[1] = t.expert; w[2] = t.start; w[3] = min(t.count, kSub); w[4] = t.row0;
+                mbar_arrive(&sfull[ss]);
+                if (++ss == kSched) { ss = 0; sph ^= 1u; }
+                if (item >= n_items) break;
+            }
+            if (!ok) raise_error(p.error, TSP_ERR_TIMEOUT);
+        }
     } else {
-        // =========================== epilogue (the last kEpWarps warps) ===========================
+        // =========================== epilogue (kEpWarps warps) ===========================
         const uint32_t quarter = warp & 3u;                   // tensor-memory lane quarter this warp may read
         const uint32_t ehalf = (warp - (3 + kDqWarps)) >> 2;  // the two warps of a quarter take the 32-column batches in turn
-        uint8_t* const etile = gsm + p.off_ep + (warp - (3 + kDqWarps)) * kEpTileBytes;   // this warp's transposition tile
+        uint8_t* const etile = gsm + p.off_ep + (warp - (3 + kDqWarps)) * ep_tile_bytes(GATEUP);   // this warp's transposition tile
         bool ok = true;
         uint32_t ab = 0, accph = 0;
         for (;;) {
@@ -578,21 +609,15 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
             const GTask& t = it.t;
             const uint32_t rb = it.item % p.row_blocks;
             const bool shared = t.expert >= p.experts;
-            const uint32_t nsub = sub_tiles(t);
             // down: route ids of this lane's columns (column j0 + lane of each batch), fetched before the wait so their latency
-            // hides behind the MMAs: slot [g][b] = batch j0 = ehalf * 32 + 64 * b of sub-tile g
-            uint32_t rt[2][2] = {{0, 0}, {0, 0}};
+            // hides behind the MMAs: slot b = batch j0 = ehalf * 32 + 64 * b
+            uint32_t rt[2] = {0, 0};
             if (!GATEUP) {
 #pragma unroll
-                for (uint32_t g = 0; g < 2; ++g)
-#pragma unroll
-                    for (uint32_t b = 0; b < 2; ++b) {
-                        const uint32_t j = ehalf * 32 + 64 * b + lane;
-                        if (j < sub_count(t, g)) {
-                            const uint32_t at = t.start + g * kSub + j;
-                            rt[g][b] = shared ? at : p.token_map[static_cast<uint64_t>(t.expert) * p.tokens + at];
-                        }
-                    }
+                for (uint32_t b = 0; b < 2; ++b) {
+                    const uint32_t j = ehalf * 32 + 64 * b + lane;
+                    if (j < t.count) rt[b] = shared ? t.start + j : p.token_map[static_cast<uint64_t>(t.expert) * p.tokens + t.start + j];
+                }
             }
             ok = gwait(&acc_full[ab], accph);
             if (ok) {
@@ -600,15 +625,14 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                 char* const obase = reinterpret_cast<char*>(shared ? p.sh_out : p.out);
                 const uint64_t ostride = shared ? p.sh_out_stride_bytes : p.out_stride_bytes;
                 bool bad = false;
-#pragma unroll
-                for (uint32_t g = 0; g < 2; ++g) {
-                    if (g >= nsub) break;
-                    const uint32_t cnt = sub_count(t, g), nc = sub_cols(cnt);
-                    const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + ab * 256u + g * kSub;
-#pragma unroll
+                const uint32_t cnt = t.count;
+                const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + ab * kAccCols;
+                {
+#pragma unroll 1
                     for (uint32_t b = 0; b < 2; ++b) {
                         const uint32_t j0 = ehalf * 32 + 64 * b;
-                        if (j0 >= nc || j0 >= cnt) break;
+                        const uint32_t route = b ? rt[1] : rt[0];
+                        if (j0 >= cnt) break;
                         uint32_t v[32];
                         tmem_ld32(taddr + j0, v);
                         tmem_ld_wait();
@@ -638,7 +662,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                             __syncwarp();
                             if (j0 + lane < cnt) {   // this lane's token: 16 hidden units = 32 bytes
                                 const uint4 o0 = *reinterpret_cast<const uint4*>(etile + lane * RS), o1 = *reinterpret_cast<const uint4*>(etile + lane * RS + 16);
-                                uint4* dst = reinterpret_cast<uint4*>(obase + static_cast<uint64_t>(t.row0 + g * kSub + j0 + lane) * ostride + (rb * 64u + quarter * 16u) * 2);
+                                uint4* dst = reinterpret_cast<uint4*>(obase + static_cast<uint64_t>(t.row0 + j0 + lane) * ostride + (rb * 64u + quarter * 16u) * 2);
                                 dst[0] = o0; dst[1] = o1;
                             }
                             __syncwarp();
@@ -649,26 +673,30 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
 #pragma unroll
                             for (uint32_t i = 0; i < 32; ++i) nf |= (j0 + i < cnt) && !finite_f32(__uint_as_float(v[i]));
                             bad |= nf;
-                            char* orow = obase + static_cast<uint64_t>(rt[g][b]) * ostride;   // this lane's token = column j0 + lane
                             if (f16) {
                                 constexpr uint32_t RS = 80;   // 32 channels x 2 B + 16
 #pragma unroll
                                 for (uint32_t i = 0; i < 32; ++i) *reinterpret_cast<__half*>(etile + i * RS + lane * 2) = __float2half_rn(__uint_as_float(v[i]));
                                 __syncwarp();
                                 if (j0 + lane < cnt) {
-                                    uint4* dst = reinterpret_cast<uint4*>(orow + wbase * 2);
+                                    uint4* dst = reinterpret_cast<uint4*>(obase + static_cast<uint64_t>(route) * ostride + wbase * 2);   // this lane's token = column j0 + lane
 #pragma unroll
                                     for (uint32_t k = 0; k < 4; ++k) dst[k] = *reinterpret_cast<const uint4*>(etile + lane * RS + k * 16);
                                 }
                             } else {
-                                constexpr uint32_t RS = 144;  // 32 channels x 4 B + 16
+                                constexpr uint32_t RS = 144;  // 32 channels x 4 B + 16; sixteen token rows at a time, two lanes per row
 #pragma unroll
-                                for (uint32_t i = 0; i < 32; ++i) *reinterpret_cast<uint32_t*>(etile + i * RS + lane * 4) = v[i];
-                                __syncwarp();
-                                if (j0 + lane < cnt) {
-                                    uint4* dst = reinterpret_cast<uint4*>(orow + wbase * 4);
+                                for (uint32_t h = 0; h < 2; ++h) {
 #pragma unroll
-                                    for (uint32_t k = 0; k < 8; ++k) dst[k] = *reinterpret_cast<const uint4*>(etile + lane * RS + k * 16);
+                                    for (uint32_t i = 0; i < 16; ++i) *reinterpret_cast<uint32_t*>(etile + i * RS + lane * 4) = v[16 * h + i];
+                                    __syncwarp();
+                                    const uint32_t j = 16 * h + (lane >> 1), rid = __shfl_sync(0xffffffffu, route, j);
+                                    if (j0 + j < cnt) {
+                                        uint4* dst = reinterpret_cast<uint4*>(obase + static_cast<uint64_t>(rid) * ostride + wbase * 4 + (lane & 1u) * 64);
+#pragma unroll
+                                        for (uint32_t k = 0; k < 4; ++k) dst[k] = *reinterpret_cast<const uint4*>(etile + (lane >> 1) * RS + (lane & 1u) * 64 + k * 16);
+                                    }
+                                    __syncwarp();
                                 }
                             }
                             __syncwarp();
@@ -885,12 +913,16 @@ int launch_grouped(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     p.dm_mat_bytes = q8 ? 0u : rm * nblk * 4u;        // a multiple of 256: rm >= 64 (Q8_0: no (d, dmin) ring)
     p.off_q = 1024;
     p.q_stage_bytes = kRowsM * (128u + 16u);
-    p.off_d = p.off_q + 2 * p.q_stage_bytes;
     p.d_stage_bytes = (nmat * p.dm_mat_bytes + 1023u) & ~1023u;
-    p.off_st = p.off_d + 2 * p.d_stage_bytes;
-    p.off_ep = p.off_st + kStages * kStageBytes;
-    const size_t smem = p.off_ep + kEpWarps * kEpTileBytes + 1024;
-    TSP_REQUIRE(smem <= 227 * 1024, "grouped GEMM: K extent needs more shared memory than one SM has");
+    size_t smem = 0;
+    for (p.n_quant = kQuant; p.n_quant >= kQuant - 1; --p.n_quant) {
+        p.off_d = p.off_q + p.n_quant * p.q_stage_bytes;
+        p.off_st = p.off_d + 2 * p.d_stage_bytes;
+        p.off_ep = p.off_st + kStages * kStageBytes;
+        smem = p.off_ep + kEpWarps * ep_tile_bytes(gateup) + 1024;
+        if (smem <= 227 * 1024) break;
+    }
+    TSP_REQUIRE(p.d_stage_bytes <= 4096 && smem <= 227 * 1024, "grouped GEMM: K extent needs more shared memory than one SM has");
 
     // gate and up of an expert at one constant distance: one copy per plane brings both
     auto mergeable = [](const uint8_t* first, const uint8_t* second, uint64_t* delta) {
