@@ -10,7 +10,7 @@ from tokspur_public_b200 import capi  # noqa: E402
 from tokspur_public_b200 import layer as L  # noqa: E402
 
 
-@pytest.mark.parametrize("tokens,branches,channels,rank", [(1, 4, 2560, 16), (5, 4, 2048, 8), (3, 2, 100, 4), (2, 64, 33, 3)])
+@pytest.mark.parametrize("tokens,branches,channels,rank", [(1, 4, 2560, 16), (5, 4, 2048, 8), (3, 2, 100, 4), (2, 64, 33, 3), (2, 5, 516, 3)])
 def test_residual_read_write_rows(oracle, tokens, branches, channels, rank):
     rng = np.random.default_rng(tokens * 7 + branches)
     width = branches * channels
