@@ -45,6 +45,20 @@ def test_router_projection_against_double(T, rows, cols):
     assert np.max(np.abs(gex - wex) / np.maximum(1.0, np.abs(wex))) <= 5e-5
 
 
+# Edges of the tensor-core product's tiles (128 token rows x 64 matrix rows x 64 columns, sums emptied every 256 columns), rows that are
+# not whole 16-byte units, and the last batch of the one-warp-per-output form. Each value is the sum of three bfloat16 parts (8 + 8 + 8
+# bits), the products left out are below 2^-23 of their term and a sum of n terms in FP32 keeps n * 2^-24 of its magnitude sum.
+@pytest.mark.parametrize("T,rows,cols,pad", [(95, 65, 64, 0), (96, 1, 7, 0), (96, 64, 256, 4), (128, 63, 260, 0), (129, 130, 257, 3), (257, 65, 2048, 0)])
+def test_router_projection_tile_edges(T, rows, cols, pad):
+    w, x = synth.normal(3 + rows, (rows, cols), 0.05), synth.normal(5 + T, (T, cols))
+    x[0] *= 1e30   # far outside binary16: the parts have FP32's range
+    w[0] *= 1e-20
+    got, _ = project(w, x, x_pad=pad)
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    magnitude = np.abs(x.astype(np.float64)) @ np.abs(w.astype(np.float64)).T
+    assert np.max(np.abs(got - want) / magnitude) <= (cols + 4) * 2.0 ** -24
+
+
 def test_forced_route_fixture_ids_and_margins(oracle):
     E, Cn, K = 512, 64, 10
     w = np.zeros((E, Cn), np.float32)

@@ -90,11 +90,6 @@ __device__ __forceinline__ void umma_chunk_ts(uint32_t d_tmem, uint32_t a_tmem, 
         "@p tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t}"
         ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(bar), "n"(kUmmaDescHi) : "memory");
 }
-__device__ __forceinline__ bool elect_one() {
-    uint32_t r;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
-    return r != 0;
-}
 // 32 registers per thread -> 32 lanes x 32 consecutive columns (the warp's own lane quarter)
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"

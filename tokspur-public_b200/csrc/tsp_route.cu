@@ -592,176 +592,17 @@ gemv_f32_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, ui
     }
 }
 
-// ---------------------------------------------------------------------------------------------
-// F32 router projection for batches: logits[t][e] = sum_c W[e][c] * x[t][c] as a register-tiled FP32 GEMM (FP32 FMA only: the
-// ids chosen from these logits must follow the reference's double-precision logits, so no reduced-precision tensor path).
-// W is read once per tile of 64 token rows. Every output is one FMA chain in ascending c, i.e. the plain sequential FP32 dot
-// product. An optional extra row `extra` (the shared-router vector) is projected in the same pass into `extra_out[t]`.
-// ---------------------------------------------------------------------------------------------
-constexpr int kRgM = 64, kRgN = 128, kRgK = 16, kRgThreads = 256;
-
-__global__ void __launch_bounds__(kRgThreads)
-router_gemm_kernel(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x,
-                   uint64_t x_stride, uint32_t tokens, float* __restrict__ out, uint64_t out_stride, float* __restrict__ extra_out, uint32_t* error) {
-    pdl_launch_dependents();
-    pdl_wait();
-    __shared__ float xs[kRgK][kRgM + 4];
-    __shared__ float ws[kRgK][kRgN + 4];
-    const uint32_t tid = threadIdx.x;
-    const uint32_t t0 = blockIdx.y * kRgM, r0 = blockIdx.x * kRgN;
-    const uint32_t all_rows = rows + (extra ? 1u : 0u);
-    // thread -> 4 token rows x 8 matrix rows of the tile
-    const uint32_t tm = (tid >> 4) * 4, tn = (tid & 15u) * 8;
-    float acc[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    // loaders: x tile = 64 rows x 16 columns = 256 float4 (one per thread); w tile = 128 x 16 = 512 float4 (two per thread)
-    const uint32_t lx_row = tid >> 2, lx_c4 = (tid & 3u) * 4;
-    for (uint32_t k0 = 0; k0 < cols; k0 += kRgK) {
-        {
-            const uint32_t t = t0 + lx_row, c = k0 + lx_c4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (t < tokens) {
-                const float* src = reinterpret_cast<const float*>(reinterpret_cast<const char*>(x) + t * x_stride) + c;
-                if (c + 4 <= cols && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) v = *reinterpret_cast<const float4*>(src);
-                else { if (c < cols) v.x = src[0]; if (c + 1 < cols) v.y = src[1]; if (c + 2 < cols) v.z = src[2]; if (c + 3 < cols) v.w = src[3]; }
-            }
-            xs[lx_c4][lx_row] = v.x; xs[lx_c4 + 1][lx_row] = v.y; xs[lx_c4 + 2][lx_row] = v.z; xs[lx_c4 + 3][lx_row] = v.w;
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t lr = (tid >> 2) + h * 64, r = r0 + lr, c = k0 + lx_c4;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < all_rows) {
-                const float* src = (r < rows ? w + static_cast<uint64_t>(r) * cols : extra) + c;
-                if (c + 4 <= cols && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) v = *reinterpret_cast<const float4*>(src);
-                else { if (c < cols) v.x = src[0]; if (c + 1 < cols) v.y = src[1]; if (c + 2 < cols) v.z = src[2]; if (c + 3 < cols) v.w = src[3]; }
-            }
-            ws[lx_c4][lr] = v.x; ws[lx_c4 + 1][lr] = v.y; ws[lx_c4 + 2][lr] = v.z; ws[lx_c4 + 3][lr] = v.w;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kRgK; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(&xs[k][tm]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&ws[k][tn]), b1 = *reinterpret_cast<const float4*>(&ws[k][tn + 4]);
-            const float av[4] = {a.x, a.y, a.z, a.w}, bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(bv[j], av[i], acc[i][j]);
-        }
-        __syncthreads();
-    }
-    bool bad = false;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t t = t0 + tm + i;
-        if (t >= tokens) continue;
-        float* orow = reinterpret_cast<float*>(reinterpret_cast<char*>(out) + t * out_stride);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const uint32_t r = r0 + tn + j;
-            if (r < rows) { bad |= !finite_f32(acc[i][j]); orow[r] = acc[i][j]; }
-            else if (r == rows && extra) { bad |= !finite_f32(acc[i][j]); extra_out[t] = acc[i][j]; }
-        }
-    }
-    if (bad) raise_error(error, TSP_ERR_NONFINITE);
-}
-
-// The same product for large batches: K steps of 16 double-buffered in shared memory, every shared-memory load 16 bytes and
-// conflict-free, FP32 FMA in ascending K order per output. Requires cols % 16 == 0 and 16-byte aligned rows; edge tiles are
-// predicated. (The 64 x 128 kernel above, no double buffering, ran at 15 TFLOP/s on 4096 x 512 x 2048: 0.574 ms.)
-constexpr int kSgT = 128, kSgK = 16, kSgThreads = 256;
-
-// One block: 128 token rows x 64 matrix rows, 8 x 4 outputs per thread, two blocks per SM. Measured on 4096 x 512 x 2048
-// (ms): this form 0.278; 128 x 128 tiles with 8 x 8 outputs (one block per SM, 128 blocks) 0.402; packed FP32 FMAs 0.280
-// (the kernel is not bound by issue slots); a warp-broadcast mapping with 16 x 4 outputs 0.415.
-__global__ void __launch_bounds__(kSgThreads, 2)
-router_sgemm_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, uint64_t x_stride, uint32_t tokens,
-                    float* __restrict__ out, uint64_t out_stride, uint32_t* error) {
-    pdl_launch_dependents();
-    pdl_wait();
-    constexpr int TN = 64;
-    __shared__ __align__(16) float xs[2][kSgK][kSgT];
-    __shared__ __align__(16) float ws[2][kSgK][TN];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t t0 = blockIdx.y * kSgT, r0 = blockIdx.x * TN;
-    // loaders: a warp takes 32 consecutive rows of a tile and one 4-wide K group; stores to [k][row] are then bank-conflict-free
-    const uint32_t l_row = lane + 32 * (warp & 3u), l_k = 4 * (warp >> 2);   // x: K groups l_k and l_k + 8
-    const uint32_t w_row = lane + 32 * (warp & 1u), w_k = 4 * (warp >> 1);   // w: 64 rows, one K group per warp
-    const float* xsrc = reinterpret_cast<const float*>(reinterpret_cast<const char*>(x) + static_cast<uint64_t>(min(t0 + l_row, tokens - 1)) * x_stride);
-    const float* wsrc = w + static_cast<uint64_t>(min(r0 + w_row, rows - 1)) * cols;
-    // outputs: token rows ty*4 + {0..3} and 64 + ty*4 + {0..3}, matrix rows tx*4 + {0..3}
-    const uint32_t ty = tid >> 4, tx = tid & 15u;
-    float acc[8][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    float4 gx[2], gw;
-    auto fetch = [&](uint32_t k0) {
-        gx[0] = *reinterpret_cast<const float4*>(xsrc + k0 + l_k); gx[1] = *reinterpret_cast<const float4*>(xsrc + k0 + l_k + 8);
-        gw = *reinterpret_cast<const float4*>(wsrc + k0 + w_k);
-    };
-    auto stash = [&](uint32_t b) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t k = l_k + 8 * h;
-            xs[b][k][l_row] = gx[h].x; xs[b][k + 1][l_row] = gx[h].y; xs[b][k + 2][l_row] = gx[h].z; xs[b][k + 3][l_row] = gx[h].w;
-        }
-        ws[b][w_k][w_row] = gw.x; ws[b][w_k + 1][w_row] = gw.y; ws[b][w_k + 2][w_row] = gw.z; ws[b][w_k + 3][w_row] = gw.w;
-    };
-    fetch(0);
-    stash(0);
-    __syncthreads();
-    uint32_t buf = 0;
-    for (uint32_t k0 = 0; k0 < cols; k0 += kSgK) {
-        const bool more = k0 + kSgK < cols;
-        if (more) fetch(k0 + kSgK);
-#pragma unroll
-        for (int k = 0; k < kSgK; ++k) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&xs[buf][k][ty * 4]), a1 = *reinterpret_cast<const float4*>(&xs[buf][k][64 + ty * 4]);
-            const float4 b0 = *reinterpret_cast<const float4*>(&ws[buf][k][tx * 4]);
-            const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w}, bv[4] = {b0.x, b0.y, b0.z, b0.w};
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(bv[j], av[i], acc[i][j]);
-        }
-        if (more) stash(buf ^ 1u);
-        __syncthreads();
-        buf ^= 1u;
-    }
-    bool bad = false;
-    const uint32_t r = r0 + tx * 4;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t t = t0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-        if (t >= tokens) continue;
-        float* orow = reinterpret_cast<float*>(reinterpret_cast<char*>(out) + t * out_stride);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) bad |= !finite_f32(acc[i][j]) && r + j < rows;
-        if (r + 4 <= rows && (reinterpret_cast<uintptr_t>(orow + r) & 15u) == 0) *reinterpret_cast<float4*>(orow + r) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        else
-            for (int j = 0; j < 4; ++j) if (r + j < rows) orow[r + j] = acc[i][j];
-    }
-    if (bad) raise_error(error, TSP_ERR_NONFINITE);
-}
+int launch_router_mma(const float*, uint32_t, uint32_t, const float*, uint64_t, uint32_t, float*, uint64_t, uint32_t*, cudaStream_t);
+// Fewest token rows for the tensor-core product (512 matrix rows): its one wave of blocks takes 18 us at 1024 columns and 32 us at
+// 2048 whatever the batch; one warp per output takes 15 us at 63 rows of 1024 columns, 15 us at 32 and 24 us at 63 rows of 2048.
+constexpr uint32_t kRouterMmaTokens = 96;
 
 int launch_gemv_f32(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x, uint64_t x_stride, uint32_t tokens, float* out,
                     uint64_t out_stride, float* extra_out, uint32_t* error, cudaStream_t st) {
-    if (tokens >= 256 && rows >= 64 && cols % kSgK == 0 && (reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x) | x_stride) % 16 == 0) {
-        // large batches: full 128 x 128 tiles; the extra row (one dot product per token) takes its own small launch
-        const dim3 grid((rows + 63) / 64, (tokens + kSgT - 1) / kSgT);
-        TSP_CUDA(launch_pdl(router_sgemm_kernel, grid, dim3(kSgThreads), 0, st, w, rows, cols, x, x_stride, tokens, out, out_stride, error));
+    if (tokens >= kRouterMmaTokens) {
+        // the extra row (one dot product per token) takes its own small launch
+        if (int rc = launch_router_mma(w, rows, cols, x, x_stride, tokens, out, out_stride, error, st)) return rc;
         if (extra) TSP_CUDA(launch_pdl(gemv_f32_kernel, dim3(static_cast<unsigned>((tokens + 7) / 8)), dim3(256), 0, st, extra, 1u, cols, x, x_stride, tokens, extra_out, sizeof(float), error));
-        return TSP_OK;
-    }
-    if (tokens >= 32) {   // batches: W is read once per 64 token rows
-        const dim3 grid((rows + (extra ? 1 : 0) + kRgN - 1) / kRgN, (tokens + kRgM - 1) / kRgM);
-        TSP_CUDA(launch_pdl(router_gemm_kernel, grid, dim3(kRgThreads), 0, st, w, rows, cols, extra, x, x_stride, tokens, out, out_stride, extra_out, error));
         return TSP_OK;
     }
     const uint64_t warps = static_cast<uint64_t>(rows) * tokens;
