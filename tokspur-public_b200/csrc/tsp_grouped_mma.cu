@@ -641,6 +641,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                             const uint32_t u16 = lane & 15u;
                             const uint32_t hpos = (u16 & 8u) | ((u16 & 4u) | ((u16 & 1u) << 1) | ((u16 & 2u) >> 1));
                             const bool low = lane < 16;
+                            float zero = 0.f, top = 0.f;   // NaN when a value is not finite; the largest magnitude
                             constexpr uint32_t RS = 48;   // tile row: 16 units x 2 B, padded so that the 16-byte reads below spread over the banks
 #pragma unroll
                             for (uint32_t a = 0; a < 16; ++a) {
@@ -651,7 +652,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                                 const float val = __fdividef(gv, 1.f + __expf(-gv)) * uv;   // silu(g) * u
                                 const __half hv = __float2half_rn(val);
                                 const uint32_t i = 2 * a + (low ? 0u : 1u);
-                                bad |= (j0 + i < cnt) && !finite_f32(__half2float(hv));
+                                zero = fmaf(val, 0.f, zero); top = fmaxf(top, fabsf(val));
                                 *reinterpret_cast<__half*>(etile + i * RS + hpos * 2) = hv;
                             }
                             __syncwarp();
@@ -660,14 +661,22 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                                 uint4* dst = reinterpret_cast<uint4*>(obase + static_cast<uint64_t>(t.row0 + j0 + lane) * ostride + (rb * 64u + quarter * 16u) * 2);
                                 dst[0] = o0; dst[1] = o1;
                             }
+                            // columns past cnt hold other experts' rows: only this item's values count, looked at one by one only when some
+                            // value of the batch is suspect (65520 rounds to infinity)
+                            if (__any_sync(0xffffffffu, zero != zero || top >= 65520.f) && j0 + lane < cnt)
+                                for (uint32_t i = 0; i < 16; ++i) bad |= !finite_f32(__half2float(*reinterpret_cast<const __half*>(etile + lane * RS + i * 2)));
                             __syncwarp();
                         } else {
                             const uint32_t wbase = rb * kRowsM + quarter * 32;   // first output channel of this warp
                             const bool f16 = !shared && p.out_f16;
-                            bool nf = false;
+                            float zero[4] = {0.f, 0.f, 0.f, 0.f};   // NaN when a value is not finite
 #pragma unroll
-                            for (uint32_t i = 0; i < 32; ++i) nf |= (j0 + i < cnt) && !finite_f32(__uint_as_float(v[i]));
-                            bad |= nf;
+                            for (uint32_t i = 0; i < 32; ++i) zero[i & 3u] = fmaf(__uint_as_float(v[i]), 0.f, zero[i & 3u]);
+                            const float all = (zero[0] + zero[1]) + (zero[2] + zero[3]);
+                            if (__any_sync(0xffffffffu, all != all)) {   // columns past cnt hold other experts' rows: look at this item's alone
+#pragma unroll
+                                for (uint32_t i = 0; i < 32; ++i) bad |= (j0 + i < cnt) && !finite_f32(__uint_as_float(v[i]));
+                            }
                             if (f16) {
                                 constexpr uint32_t RS = 80;   // 32 channels x 2 B + 16
 #pragma unroll
