@@ -275,7 +275,7 @@ def decode_record(args, dev, T, layers, etype, layout, full: bool):
     dn_bytes = (U0 + 1) * expert_down + T * (SELECTED + 1) * (HIDDEN * 4 + CHANNELS * 4)
     achieved = gu_bytes / (gu_ms * 1e-3) / 1e9
     kname = ("gemv3_kernel<planar, gate-up+SwiGLU> (routed experts + shared expert, one launch)" if etype == formats.Q4_K else
-             "gemv_k5_kernel<Q5_K, gate-up+SwiGLU> (routed experts) + gemv_kernel<Q8_0> (shared expert): two launches timed together" if etype == formats.Q5_K else
+             "gemv_k5_mma_kernel<Q5_K, gate-up+SwiGLU> (routed experts) + gemv_kernel<Q8_0> (shared expert): two launches timed together" if etype == formats.Q5_K else
              "gemv_kernel<Q8_0, gate-up+SwiGLU> (routed experts, then the shared expert: two launches timed together)")
     roofline = {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
                 "peak_kind": peak_kind, "timing": "average of a back-to-back loop of this launch alone over the rotating layers (CUDA events)",

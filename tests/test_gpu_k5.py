@@ -69,6 +69,37 @@ def test_dense_projection_against_oracle(oracle, type_, rows, cols, T):
     assert scaled_error(out.cpu().numpy(), want) <= 5e-5
 
 
+# The MMA kernel's edges: one warp's rows, a block's and more; tiles of up to four rows (low halves in the free columns) and of more; the
+# shortest K; activations far outside binary16's range. A value keeps 22 bits (high + low half) and an FP32 sum of n terms n * 2^-24 of its
+# magnitude sum, a term being the activation times the scaled code or the offset, each at most twice the largest weight; a tile's size
+# may not show in a row's result.
+@pytest.mark.parametrize("type_,rows,cols", [(formats.Q5_K, 16, 256), (formats.Q5_K, 144, 2048), (formats.Q5_1, 16, 128), (formats.Q5_1, 272, 512)])
+def test_dense_projection_tile_edges(oracle, type_, rows, cols):
+    w = formats.quantize(type_, synth.normal(81, (rows, cols), 0.02)).reshape(-1)
+    t = dev(w)
+    ms = L.matrix_set(t, type_, formats.GGUF, rows, cols, 1)
+    x = synth.normal(82, (8, cols), 1.0)
+    x[1] *= 1e30
+    x[2] *= 1e-25
+    x[3] = 0.0
+    x[4, 0] = 65000.0
+    w64 = oracle.dequantize(type_, w, rows * cols).astype(np.float64).reshape(rows, cols)
+    want = x.astype(np.float64) @ w64.T
+    magnitude = 4 * np.abs(w64).max() * np.abs(x.astype(np.float64)).sum(axis=1)[:, None]
+    dx, alone = dev(x), []
+    e = torch.zeros(1, dtype=torch.int32, device=DEV)
+    for T in (8, 5, 4, 1):
+        out = torch.zeros((T, rows), dtype=torch.float32, device=DEV)
+        capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, 1, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        assert np.all(np.abs(got - want[:T]) <= (cols + 8) * 2.0 ** -24 * magnitude[:T])
+        alone.append(got)
+    assert int(e.item()) == 0
+    for a in alone[1:]:
+        assert np.array_equal(a, alone[0][:len(a)])
+
+
 @pytest.mark.parametrize("T", [1, 8, 29, 64])
 @pytest.mark.parametrize("shared_type", [formats.Q8_0, formats.Q5_K])
 def test_layer_q5k_gate_up_q51_down(oracle, T, shared_type):
