@@ -93,3 +93,21 @@ def test_forced_route_fixture_ids_and_margins(oracle):
         assert tel.total_tokens == T and tel.total_layers == 1 and tel.violation_count == int((m <= 2e-4).sum())
         assert abs(tel.min_margin - float(m.min())) == 0 and abs(tel.sum_margin - float(m.astype(np.float64).sum())) <= 1e-9
         assert fb.value == int(tel.violation_count > 0) and tel.fallback_layers == fb.value
+
+
+# Register form of the selection (up to 512 experts): few distinct values, both zeros, experts not a multiple of 32, every expert selected
+@pytest.mark.parametrize("T,E,K", [(1, 512, 10), (9, 70, 64), (33, 512, 40), (64, 16, 16)])
+def test_route_ties_and_signed_zeros(oracle, T, E, K):
+    rng = np.random.default_rng(E + K)
+    logits = rng.choice(np.array([-0.0, 0.0, 1.5, -2.25], dtype=np.float32), size=(T, E))
+    lg = torch.from_numpy(logits).cuda()
+    ids = torch.zeros(T * K, dtype=torch.int32, device="cuda")
+    wt = torch.zeros(T * K, dtype=torch.float32, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for mode in (0, 1):
+        capi.call("tsp_moe_route", lg.data_ptr(), E * 4, T, E, K, mode, 1, ids.data_ptr(), wt.data_ptr(), err.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        oi, ow = oracle.route_rows(logits.astype(np.float64), K, mode, True)
+        assert np.array_equal(ids.cpu().numpy().view(np.uint32).reshape(T, K), oi)
+        assert np.max(np.abs(wt.cpu().numpy().reshape(T, K) - ow)) <= 1e-6
+    assert int(err.item()) == 0

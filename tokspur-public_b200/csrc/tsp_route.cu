@@ -107,14 +107,29 @@ __device__ __forceinline__ void route_row(float* row, const float* src, uint32_t
 __device__ __forceinline__ void route_row_regs(const float* src, uint32_t token, uint32_t experts, uint32_t selected,
                                                uint32_t mode, uint32_t* __restrict__ ids, float* __restrict__ weights, uint32_t* error,
                                                uint32_t lane) {
-    float v[16];
+    // Order-preserving 32-bit images (-0 counted as +0: equal logits tie by id), 0 = no expert or already taken. A round is one max over
+    // the lane's 16 images, one warp-wide max and one warp-wide min over the ids that reach it: two reductions instead of ten shuffles.
+    uint32_t k[16];
     bool bad = false;
 #pragma unroll
     for (uint32_t i = 0; i < 16; ++i) {
         const uint32_t e = lane + 32 * i;
-        v[i] = e < experts ? src[e] : -INFINITY;
-        bad |= e < experts && !finite_f32(v[i]);
+        const float f = e < experts ? src[e] : 0.f;
+        bad |= !finite_f32(f);
+        const uint32_t u = f == 0.f ? 0u : __float_as_uint(f);
+        k[i] = e < experts ? ((u & 0x80000000u) ? ~u : (u | 0x80000000u)) : 0u;
     }
+    auto lane_max = [&]() {
+        uint32_t m[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m[i] = max(k[i], k[i + 8]);
+#pragma unroll
+        for (int o = 4; o; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < o; ++i) m[i] = max(m[i], m[i + o]);
+        return m[0];
+    };
+    auto value = [](uint32_t image) { return __uint_as_float((image & 0x80000000u) ? image ^ 0x80000000u : ~image); };
     bad = __any_sync(0xffffffffu, bad);
     uint32_t* out_ids = ids + static_cast<uint64_t>(token) * selected;
     float* out_w = weights + static_cast<uint64_t>(token) * selected;
@@ -123,27 +138,21 @@ __device__ __forceinline__ void route_row_regs(const float* src, uint32_t token,
         for (uint32_t r = lane; r < selected; r += 32) { out_ids[r] = r; out_w[r] = 0.f; }
         return;
     }
-    float row_max = -INFINITY;
-#pragma unroll
-    for (uint32_t i = 0; i < 16; ++i) row_max = fmaxf(row_max, v[i]);
-    for (int o = 16; o; o >>= 1) row_max = fmaxf(row_max, __shfl_xor_sync(0xffffffffu, row_max, o));
+    float row_max = 0.f;
     float my_logit = 0.f, my_logit_hi = 0.f;
     for (uint32_t r = 0; r < selected; ++r) {
-        float best = -INFINITY;
-        uint32_t best_id = 0xffffffffu;
+        const uint32_t top = __reduce_max_sync(0xffffffffu, lane_max());
+        uint32_t mine = 0xffffffffu;
 #pragma unroll
-        for (uint32_t i = 0; i < 16; ++i)
-            if (v[i] > best) { best = v[i]; best_id = lane + 32 * i; }   // ascending scan keeps the lowest id on ties
-        for (int o = 16; o; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const uint32_t oi = __shfl_xor_sync(0xffffffffu, best_id, o);
-            if (ov > best || (ov == best && oi < best_id)) { best = ov; best_id = oi; }
-        }
+        for (int i = 15; i >= 0; --i) if (k[i] == top) mine = lane + 32 * i;   // the lane's lowest id
+        const uint32_t best_id = __reduce_min_sync(0xffffffffu, mine);
+        const float best = value(top);
+        if (r == 0) row_max = best;
         if ((r & 31u) == lane) { if (r < 32) my_logit = best; else my_logit_hi = best; }
         if (lane == 0) out_ids[r] = best_id;
-        if ((best_id & 31u) == lane) {
+        if (mine == best_id) {
 #pragma unroll
-            for (uint32_t i = 0; i < 16; ++i) if ((best_id >> 5) == i) v[i] = -INFINITY;
+            for (uint32_t i = 0; i < 16; ++i) if ((best_id >> 5) == i) k[i] = 0u;
         }
     }
     const double mx = row_max;
