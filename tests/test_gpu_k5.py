@@ -100,6 +100,25 @@ def test_dense_projection_tile_edges(oracle, type_, rows, cols):
         assert np.array_equal(a, alone[0][:len(a)])
 
 
+def test_every_kernel_gets_its_own_shared_memory_limit(oracle):
+    """Dense batches of 16 rows: the plain kernel and the gate-up kernel of one encoding both need more than the default 48 KB of shared
+    memory; the limit set for one says nothing about the other."""
+    rows, cols, T = 16, 2048, 16
+    w = formats.quantize(formats.Q5_K, synth.normal(91, (rows, cols), 0.02)).reshape(-1)
+    t = dev(w)
+    ms = L.matrix_set(t, formats.Q5_K, formats.GGUF, rows, cols, 1)
+    x = synth.normal(92, (T, cols), 1.0)
+    dx, e = dev(x), torch.zeros(1, dtype=torch.int32, device=DEV)
+    out, h = (torch.zeros((T, rows), dtype=torch.float32, device=DEV) for _ in range(2))
+    capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, 1, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+    capi.call("tsp_moe_gate_up_swiglu", C.byref(ms), C.byref(ms), dx.data_ptr(), cols * 4, T, 1, None, None, None, h.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+    torch.cuda.synchronize()
+    assert int(e.item()) == 0
+    want = np.stack([oracle.gemv(formats.Q5_K, w, cols, rows, x[i]) for i in range(T)]).astype(np.float64)
+    assert scaled_error(out.cpu().numpy(), want) <= 5e-5
+    assert scaled_error(h.cpu().numpy(), want / (1 + np.exp(-want)) * want) <= 5e-5
+
+
 @pytest.mark.parametrize("T", [1, 8, 29, 64])
 @pytest.mark.parametrize("shared_type", [formats.Q8_0, formats.Q5_K])
 def test_layer_q5k_gate_up_q51_down(oracle, T, shared_type):

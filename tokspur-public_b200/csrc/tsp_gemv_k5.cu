@@ -434,6 +434,14 @@ static int launch_km(const K5Params& p, size_t smem, int grid, cudaStream_t st) 
     return TSP_OK;
 }
 
+template <uint32_t TYPE, bool GATEUP, uint32_t MT>
+static int launch_k5(const K5Params& p, dim3 grid, size_t smem, cudaStream_t st) {
+    static thread_local SmemAttrCache configured;   // per kernel instantiation, keyed by device
+    TSP_CUDA(ensure_dynamic_smem(gemv_k5_kernel<TYPE, GATEUP, MT>, configured, smem));
+    TSP_CUDA(launch_pdl(gemv_k5_kernel<TYPE, GATEUP, MT>, grid, dim3(kK5Threads), smem, st, p));
+    return TSP_OK;
+}
+
 int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup, const float* x, uint64_t x_stride_bytes, uint32_t in_div,
                    uint32_t tokens, const uint32_t* token_map, const uint32_t* counts, const uint32_t* tasks, float* out,
                    uint64_t out_stride_bytes, int nc, uint32_t* error, cudaStream_t st) {
@@ -474,19 +482,13 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     const uint32_t dense_tiles = (tokens + p.tile_tokens - 1) / p.tile_tokens;
     const uint64_t routed_cap = static_cast<uint64_t>(tokens) * 64u;
     const uint32_t walkers = static_cast<uint32_t>(routed_cap < 4u * static_cast<uint32_t>(sms) ? routed_cap : 4u * static_cast<uint32_t>(sms));
-    const dim3 grid((a->rows + kK5BlockRows - 1) / kK5BlockRows, token_map ? walkers : (dense_tiles < 1024u ? dense_tiles : 1024u)), block(kK5Threads);
-    auto go = [&](auto kernel) -> int {
-        static thread_local SmemAttrCache configured;   // per kernel instantiation (one lambda instantiation each), keyed by device
-        TSP_CUDA(ensure_dynamic_smem(kernel, configured, smem));
-        TSP_CUDA(launch_pdl(kernel, grid, block, smem, st, p));
-        return TSP_OK;
-    };
+    const dim3 grid((a->rows + kK5BlockRows - 1) / kK5BlockRows, token_map ? walkers : (dense_tiles < 1024u ? dense_tiles : 1024u));
     if (a->type == TSP_TYPE_Q5_K) {
-        if (gateup) return nc == 1 ? go(gemv_k5_kernel<13u, true, 8u>) : go(gemv_k5_kernel<13u, true, 16u>);
-        return nc == 1 ? go(gemv_k5_kernel<13u, false, 8u>) : go(gemv_k5_kernel<13u, false, 16u>);
+        if (gateup) return nc == 1 ? launch_k5<13u, true, 8u>(p, grid, smem, st) : launch_k5<13u, true, 16u>(p, grid, smem, st);
+        return nc == 1 ? launch_k5<13u, false, 8u>(p, grid, smem, st) : launch_k5<13u, false, 16u>(p, grid, smem, st);
     }
-    if (gateup) return nc == 1 ? go(gemv_k5_kernel<7u, true, 8u>) : go(gemv_k5_kernel<7u, true, 16u>);
-    return nc == 1 ? go(gemv_k5_kernel<7u, false, 8u>) : go(gemv_k5_kernel<7u, false, 16u>);
+    if (gateup) return nc == 1 ? launch_k5<7u, true, 8u>(p, grid, smem, st) : launch_k5<7u, true, 16u>(p, grid, smem, st);
+    return nc == 1 ? launch_k5<7u, false, 8u>(p, grid, smem, st) : launch_k5<7u, false, 16u>(p, grid, smem, st);
 }
 
 }  // namespace tsp
