@@ -100,6 +100,29 @@ def test_dense_projection_tile_edges(oracle, type_, rows, cols):
         assert np.array_equal(a, alone[0][:len(a)])
 
 
+# Both kernels on the same eight rows (a batch of sixteen takes the FP32 FMA kernel): the split into binary16 halves and the sums of the MMA
+# kernel may not be further from 64-bit sums than the FP32 kernel's are. (Summed in one chain over K instead of step by step: 2.2e-7
+# against 1.6e-7 at 2048 columns. High halves alone: 2e-4.)
+@pytest.mark.parametrize("type_,rows,cols", [(formats.Q5_K, 256, 2048), (formats.Q5_K, 256, 256), (formats.Q5_1, 512, 512), (formats.Q5_1, 256, 2048), (formats.Q5_1, 256, 128)])
+def test_tiles_of_eight_rows_are_as_exact_as_fp32(oracle, type_, rows, cols):
+    w = formats.quantize(type_, synth.normal(81, (rows, cols), 0.02)).reshape(-1)
+    t = dev(w)
+    ms = L.matrix_set(t, type_, formats.GGUF, rows, cols, 1)
+    x = synth.normal(83, (16, cols), 1.0)
+    want = x.astype(np.float64) @ oracle.dequantize(type_, w, rows * cols).astype(np.float64).reshape(rows, cols).T
+    dx = dev(x)
+    e = torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def error(T, n):
+        out = torch.zeros((T, rows), dtype=torch.float32, device=DEV)
+        capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, 1, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        return float(np.linalg.norm(out.cpu().numpy()[:n].astype(np.float64) - want[:n]) / np.linalg.norm(want[:n]))
+    for T in (8, 3):   # low halves in a pass of their own; in the free columns
+        assert error(T, T) <= error(16, T)
+    assert int(e.item()) == 0
+
+
 def test_every_kernel_gets_its_own_shared_memory_limit(oracle):
     """Dense batches of 16 rows: the plain kernel and the gate-up kernel of one encoding both need more than the default 48 KB of shared
     memory; the limit set for one says nothing about the other."""
