@@ -123,6 +123,42 @@ def test_tiles_of_eight_rows_are_as_exact_as_fp32(oracle, type_, rows, cols):
     assert int(e.item()) == 0
 
 
+# An outlier that meets weights of zero (a block whose scale and offset are zero) leaves the other values as they are, however much larger it
+# is: n * 2^-24 of the sum of the terms' own magnitudes, as FP32 sums give it. Either side of the limit from which a row takes FP32 sums.
+@pytest.mark.parametrize("type_,rows,cols", [(formats.Q5_K, 16, 512), (formats.Q5_K, 144, 2048), (formats.Q5_1, 16, 128), (formats.Q5_1, 272, 512)])
+@pytest.mark.parametrize("gate_up", [False, True])
+def test_outliers_at_zero_weights(oracle, type_, rows, cols, gate_up):
+    w = formats.quantize(type_, synth.normal(84, (rows, cols), 0.02)).reshape(rows, -1).copy()
+    block, width = (176, 256) if type_ == formats.Q5_K else (24, 32)
+    w[:, :block] = 0
+    w = w.reshape(-1)
+    t = dev(w)
+    ms = L.matrix_set(t, type_, formats.GGUF, rows, cols, 1)
+    w64 = oracle.dequantize(type_, w, rows * cols).astype(np.float64).reshape(rows, cols)
+    assert not w64[:, :width].any()
+    x = synth.normal(85, (8, cols), 1.0)
+    for j in range(1, 8):
+        x[j, 3] = 2.0 ** (0, 8, 9, 11, 24, 39, 60, 120)[j]
+    x64 = x.astype(np.float64)
+    want = x64 @ w64.T
+    bound = (cols + 8) * 2.0 ** -24 * 4 * np.abs(w64).max() * np.abs(x64[:, width:]).sum(axis=1)[:, None]   # a term: see the tile edges above
+    if gate_up:
+        want, bound = want / (1 + np.exp(-want)) * want, bound * (2 * np.abs(want) + 2)
+    dx, e = dev(x), torch.zeros(1, dtype=torch.int32, device=DEV)
+    rows_of = {}
+    for T in (8, 4):
+        out = torch.zeros((T, rows), dtype=torch.float32, device=DEV)
+        if gate_up:
+            capi.call("tsp_moe_gate_up_swiglu", C.byref(ms), C.byref(ms), dx.data_ptr(), cols * 4, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        else:
+            capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, 1, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        rows_of[T] = out.cpu().numpy()
+        assert np.all(np.abs(rows_of[T] - want[:T]) <= bound[:T])
+    assert np.array_equal(rows_of[4], rows_of[8][:4])
+    assert int(e.item()) == 0
+
+
 def test_every_kernel_gets_its_own_shared_memory_limit(oracle):
     """Dense batches of 16 rows: the plain kernel and the gate-up kernel of one encoding both need more than the default 48 KB of shared
     memory; the limit set for one says nothing about the other."""

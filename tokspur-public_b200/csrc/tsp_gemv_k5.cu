@@ -80,6 +80,42 @@ template <> struct Group5<7u> {    // Q5_1: d, m, 32 fifth bits, 16 bytes of nib
     }
 };
 
+// The FP32 sums of one weight row (gate-up: gate and up row) per `lpr` lanes for `count` token rows: at(j, grp, i4) gives four activations,
+// put(j, v) takes a finished output on the row's first lane. Whole warps; a lane of no live row computes along.
+template <uint32_t TYPE, bool GATEUP, uint32_t MT, class At, class Put>
+__device__ __forceinline__ bool k5_row_f32(const uint8_t* rowA, const uint8_t* rowB, uint32_t groups, uint32_t lpr, uint32_t lig, uint32_t count, At at, Put put) {
+    bool ok = true;
+    float accA[MT], accB[GATEUP ? MT : 1];
+#pragma unroll
+    for (uint32_t j = 0; j < MT; ++j) { accA[j] = 0.f; if (GATEUP) accB[j] = 0.f; }
+    for (uint32_t grp = lig; grp < groups; grp += lpr) {
+        const Group5<TYPE> ga(rowA, grp), gb(rowB, grp);
+        ok &= ga.finite & gb.finite;
+#pragma unroll
+        for (uint32_t i4 = 0; i4 < 8; ++i4) {
+            float wa[4], wb[4] = {0.f, 0.f, 0.f, 0.f};
+            ga.get(i4, wa);
+            if (GATEUP) gb.get(i4, wb);
+#pragma unroll
+            for (uint32_t j = 0; j < MT; ++j) {
+                if (j >= count) break;
+                const float4 v = at(j, grp, i4);
+                accA[j] = fmaf(wa[0], v.x, accA[j]); accA[j] = fmaf(wa[1], v.y, accA[j]); accA[j] = fmaf(wa[2], v.z, accA[j]); accA[j] = fmaf(wa[3], v.w, accA[j]);
+                if (GATEUP) { accB[j] = fmaf(wb[0], v.x, accB[j]); accB[j] = fmaf(wb[1], v.y, accB[j]); accB[j] = fmaf(wb[2], v.z, accB[j]); accB[j] = fmaf(wb[3], v.w, accB[j]); }
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < MT; ++j) {
+        if (j >= count) break;
+        float a = accA[j], b = GATEUP ? accB[j] : 0.f;
+        for (uint32_t o = lpr >> 1; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); if (GATEUP) b += __shfl_xor_sync(0xffffffffu, b, o); }
+        // silu with the branch-stable sigmoid (operators.cpp:28-36)
+        if (lig == 0) put(j, GATEUP ? (a >= 0.f ? a / (1.f + expf(-a)) : a * expf(a) / (1.f + expf(a))) * b : a);
+    }
+    return ok;
+}
+
 // MT: token rows of a tile at most (8 for routed tiles, 16 for dense row batches of more than 8 rows).
 // Shared memory: the tile's rows as [token][group][9 float4] (eight of data, one of padding).
 template <uint32_t TYPE, bool GATEUP, uint32_t MT>
@@ -134,39 +170,13 @@ __global__ void __launch_bounds__(kK5Threads) gemv_k5_kernel(const K5Params p) {
             const bool live = r < p.rows && r < row0 + kK5BlockRows;
             const uint8_t* rowA = baseA + static_cast<uint64_t>(live ? r : rb) * p.row_bytes;
             const uint8_t* rowB = baseB + static_cast<uint64_t>(live ? r : rb) * p.row_bytes;
-            float accA[MT], accB[GATEUP ? MT : 1];
-#pragma unroll
-            for (uint32_t j = 0; j < MT; ++j) { accA[j] = 0.f; if (GATEUP) accB[j] = 0.f; }
-            for (uint32_t grp = lig; grp < groups; grp += lpr) {
-                const Group5<TYPE> ga(rowA, grp), gb(rowB, grp);
-                ok &= ga.finite & gb.finite;
-#pragma unroll
-                for (uint32_t i4 = 0; i4 < 8; ++i4) {
-                    float wa[4], wb[4] = {0.f, 0.f, 0.f, 0.f};
-                    ga.get(i4, wa);
-                    if (GATEUP) gb.get(i4, wb);
-#pragma unroll
-                    for (uint32_t j = 0; j < MT; ++j) {
-                        if (j >= count) break;
-                        const float4 v = k5_xs[(j * groups + grp) * 9u + i4];
-                        accA[j] = fmaf(wa[0], v.x, accA[j]); accA[j] = fmaf(wa[1], v.y, accA[j]); accA[j] = fmaf(wa[2], v.z, accA[j]); accA[j] = fmaf(wa[3], v.w, accA[j]);
-                        if (GATEUP) { accB[j] = fmaf(wb[0], v.x, accB[j]); accB[j] = fmaf(wb[1], v.y, accB[j]); accB[j] = fmaf(wb[2], v.z, accB[j]); accB[j] = fmaf(wb[3], v.w, accB[j]); }
-                    }
-                }
-            }
-            // A non-finite activation makes the sums it enters non-finite (0 * inf is NaN): the finished sums are checked
-#pragma unroll
-            for (uint32_t j = 0; j < MT; ++j) {
-                if (j >= count) break;
-                float a = accA[j], b = GATEUP ? accB[j] : 0.f;
-                for (uint32_t o = lpr >> 1; o > 0; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); if (GATEUP) b += __shfl_xor_sync(0xffffffffu, b, o); }
-                if (lig == 0 && live) {
-                    // silu with the branch-stable sigmoid (operators.cpp:28-36)
-                    const float v = GATEUP ? (a >= 0.f ? a / (1.f + expf(-a)) : a * expf(a) / (1.f + expf(a))) * b : a;
+            ok &= k5_row_f32<TYPE, GATEUP, MT>(
+                rowA, rowB, groups, lpr, lig, count, [&](uint32_t j, uint32_t grp, uint32_t i4) { return k5_xs[(j * groups + grp) * 9u + i4]; },
+                [&](uint32_t j, float v) {   // a non-finite activation makes the sums it enters non-finite (0 * inf is NaN)
+                    if (!live) return;
                     if (!finite_f32(v)) raise_error(p.error, TSP_ERR_NONFINITE);
                     s_out[j][r] = v;
-                }
-            }
+                });
         }
         if (!ok) raise_error(p.error, TSP_ERR_NONFINITE);
     }
@@ -185,7 +195,7 @@ __global__ void __launch_bounds__(kK5Threads) gemv_k5_kernel(const K5Params p) {
 // step ahead (a row's bytes are read by the four lanes that use them: 32-byte pieces); blocks of eight warps walk (tile, row block)
 // items, two blocks per SM, so that one streams while the other stages its rows.
 // The groups of a step are summed by themselves before they join the total: one chain over K of 2048 was further from 64-bit sums
-// (2.2e-7, relative 2-norm) than the FP32 kernel (1.6e-7); summed by steps it is 1.1e-7.
+// (2.1e-7, relative 2-norm) than the FP32 kernel (1.5e-7).
 // Measured, layer of 512 experts of 512 x 2048, 13 rows of ten: gate-up 115 -> 72 us, down 73 -> 63 us.
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t kKmWarps = 8;
@@ -263,6 +273,34 @@ template <> struct KmStep<7u> {
     }
 };
 
+// Rows that the split would not serve take the FP32 sums (k5_row_f32, one warp's rows and one token row at a time, straight from global
+// memory): rows with a run of eight values, not all zero, that are all below 2^4 after scaling (2^-10 of the row's largest). The halves
+// end at 2^-25, so what stays on the MMAs is good to 2^-29 of the largest value beside it, and an outlier more than 2^10 times larger that
+// meets weights of zero does not drown it. Infinities and NaN go the same way, and a row's path depends on that row alone.
+// Normally distributed rows never get there (2048 values: 1e-18 per row).
+constexpr float kKmNarrow = 16.f;
+
+// Out of line: the rare path takes no registers from the loop above it.
+template <uint32_t TYPE, bool GATEUP>
+__device__ __noinline__ void k5_wide_row(const uint8_t* rowsA, const uint8_t* rowsB, uint32_t row_bytes, uint32_t rows, uint32_t groups, uint32_t lpr, const float* x, float* out, uint32_t* error) {
+    const uint32_t lane = threadIdx.x & 31u, rpw = 32u / lpr, sub = lane / lpr, lig = lane & (lpr - 1u);
+    const float4* x4 = reinterpret_cast<const float4*>(x);
+    bool ok = true;
+    for (uint32_t rb = 0; rb < rows; rb += rpw) {
+        const uint32_t r = rb + sub;
+        const bool live = r < rows;
+        const uint32_t at = (live ? r : rb) * row_bytes;
+        ok &= k5_row_f32<TYPE, GATEUP, 1u>(
+            rowsA + at, rowsB + at, groups, lpr, lig, 1u, [&](uint32_t, uint32_t grp, uint32_t i4) { return x4[grp * 8u + i4]; },
+            [&](uint32_t, float v) {
+                if (!live) return;
+                ok &= finite_f32(v);
+                out[r] = v;
+            });
+    }
+    if (!ok) raise_error(error, TSP_ERR_NONFINITE);
+}
+
 // Shared memory: high halves [8][x_stride], low halves [8][x_stride], group sums [group][8] (of the scaled values)
 template <uint32_t TYPE, bool GATEUP>
 __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5Params p) {
@@ -271,6 +309,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
     __shared__ const float* s_x[8];
     __shared__ float* s_out[8];
     __shared__ float s_scale[8], s_inv[8];
+    __shared__ uint32_t s_wide[8];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t groups = p.cols / 32u, x_stride = p.cols * 2u + 64u;
     uint8_t* const xhi = km_smem;
@@ -314,7 +353,8 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
             }
             top = __reduce_max_sync(0xffffffffu, top) >> 23;   // biased exponent of the largest magnitude
             if (lane == 0) {
-                const uint32_t e = top >= 255u ? 127u : min(268u - top, 253u);   // not finite: left as it is
+                const uint32_t e = top >= 255u ? 127u : min(268u - top, 253u);   // not finite: a wide row
+                s_wide[warp] = top >= 255u;
                 s_scale[warp] = __uint_as_float(e << 23); s_inv[warp] = __uint_as_float((254u - e) << 23);
                 s_x[warp] = x;
                 s_out[warp] = reinterpret_cast<float*>(reinterpret_cast<char*>(p.out) + static_cast<uint64_t>(rid) * p.out_stride_bytes);
@@ -329,14 +369,16 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
             const float sc = s_scale[j];
             const float v[8] = {f0.x * sc, f0.z * sc, f0.y * sc, f0.w * sc, f1.x * sc, f1.z * sc, f1.y * sc, f1.w * sc};   // order 0,2,1,3
             uint32_t h[8], l[8];
-            float sum = 0.f;
+            float sum = 0.f, most = 0.f;
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
+                most = fmaxf(most, fabsf(v[q]));
                 const __half hv = __float2half_rn(v[q]);
                 h[q] = __half_as_ushort(hv);
                 l[q] = __half_as_ushort(__float2half_rn(v[q] - __half2float(hv)));
                 sum += v[q];
             }
+            if (most < kKmNarrow && most > 0.f) s_wide[j] = 1u;
             uint8_t* dst = xhi + j * x_stride + grp * 64u + tq * 16u;
             *reinterpret_cast<uint4*>(dst) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
             *reinterpret_cast<uint4*>(dst + (packed ? 4u : 8u) * x_stride) = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
@@ -394,7 +436,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
 #pragma unroll
         for (uint32_t q = 0; q < 2; ++q) {
             const uint32_t j = 2 * t + q;
-            if (j >= count) continue;
+            if (j >= count || s_wide[j]) continue;
             const float inv = s_inv[j], va = total[q] * inv, vb = total[2 + q] * inv;
             float* o = s_out[j] + r0 + g;
             if (GATEUP) {
@@ -406,6 +448,9 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
                 o[0] = va; o[8] = vb;
             }
         }
+        for (uint32_t j = 0; j < count; ++j)   // uniform over the block
+            if (s_wide[j]) k5_wide_row<TYPE, GATEUP>(wA - static_cast<uint64_t>(g) * p.row_bytes, GATEUP ? wB - static_cast<uint64_t>(g) * p.row_bytes : wA - static_cast<uint64_t>(g) * p.row_bytes,
+                                                        p.row_bytes, RW, groups, p.lanes_per_row, s_x[j], s_out[j] + r0, p.error);
     }
 }
 
@@ -471,6 +516,8 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     const uint32_t groups = a->cols / 32;
     const int sms = sm_count();
     if (sms <= 0) return fail(TSP_E_CUDA, "no usable CUDA device");
+    p.lanes_per_row = 1;
+    while (p.lanes_per_row * 2 <= groups && p.lanes_per_row < 32) p.lanes_per_row *= 2;
     // Tiles of up to 8 rows take the MMA kernel where a warp's rows are whole and two blocks' rows fit an SM's shared memory (up to 2944
     // columns); dense batches of more rows (16 per tile) and the other shapes keep the FP32 FMA kernel.
     const size_t km_smem = 16u * (a->cols * 2u + 64u) + groups * 32u;
@@ -478,8 +525,6 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
         if (a->type == TSP_TYPE_Q5_K) return gateup ? launch_km<13u, true>(p, km_smem, 2 * sms, st) : launch_km<13u, false>(p, km_smem, 2 * sms, st);
         return gateup ? launch_km<7u, true>(p, km_smem, 2 * sms, st) : launch_km<7u, false>(p, km_smem, 2 * sms, st);
     }
-    p.lanes_per_row = 1;
-    while (p.lanes_per_row * 2 <= groups && p.lanes_per_row < 32) p.lanes_per_row *= 2;
     const size_t smem = static_cast<size_t>(p.tile_tokens) * groups * 9 * sizeof(float4);
     if (smem > 200 * 1024) return fail(TSP_E_ARG, "five-bit projection: %u columns x %u token rows do not fit the activation staging", a->cols, p.tile_tokens);
     // routed launches learn their tile count on the device: a fixed number of block rows walks the tiles (a routed launch has at
