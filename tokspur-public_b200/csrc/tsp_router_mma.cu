@@ -1,9 +1,11 @@
 // Router projection for batches on the 5th-generation tensor cores (tcgen05) at FP32 precision:
 //   logits[t][e] = sum_c W[e][c] * x[t][c],  W and x FP32.
 //
-// Each FP32 value is the exact sum of three bfloat16 values (h = the top 16 bits, m = the top 16 bits of the rest, l = what is left:
-// 8 + 8 + 8 significant bits, truncated, so nothing overflows), and a product is taken as the six of its nine partial products that
-// reach 2^-24: hh + (hm + mh + mm + hl + lh). Products of bfloat16 values are exact in FP32. The tensor core adds into FP32 with truncation,
+// Each FP32 value is the exact sum of three bfloat16 values (h = the value rounded to nearest, m = the rest rounded to nearest, l = what is
+// left: 8 + 8 + 8 significant bits and their signs), and a product is taken as six of its nine partial products:
+// hh + (hm + mh + mm + hl + lh). |m| <= 2^-8 |v| and |l| <= 2^-17 |v|, so what is left out, ml + lm + ll, stays within 2^-24 of the product
+// (2^-28 on average) and has either sign. (Parts cut off instead of rounded leave out up to 2^-21, always towards zero.) Values below
+// 2^-109 lose low bits: the last part ends where bfloat16 does, at 2^-133. Products of bfloat16 values are exact in FP32. The tensor core adds into FP32 with truncation,
 // which over 2048 columns would cost more than the FP32 chain it replaces (128 truncated additions); so the hh sums run over 256
 // columns at most, in one of two accumulators that the epilogue warps empty into FP32 registers (rounded to nearest) while the other
 // fills. The five small products, 2^-8 of the result, share one accumulator for the whole K extent.
@@ -30,13 +32,18 @@ constexpr uint32_t kRmSmem = 1024 + kRmStages * 3 * kRmPlane + 1024;
 constexpr uint32_t kRmSmall = 2 * kRmN, kRmA = 3 * kRmN;
 static_assert(kRmA + kRmStages * 96 <= 512, "tensor memory");
 
-// two FP32 values -> their three bfloat16 parts as packed pairs
+// two FP32 values -> their three bfloat16 parts as packed pairs (`a` in the low half)
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
+}
 __device__ __forceinline__ void split3(float a, float b, uint32_t& h, uint32_t& m, uint32_t& l) {
-    const uint32_t ha = __float_as_uint(a) & 0xffff0000u, hb = __float_as_uint(b) & 0xffff0000u;
-    const float ra = a - __uint_as_float(ha), rb = b - __uint_as_float(hb);                      // exact
-    const uint32_t ma = __float_as_uint(ra) & 0xffff0000u, mb = __float_as_uint(rb) & 0xffff0000u;
-    const float la = ra - __uint_as_float(ma), lb = rb - __uint_as_float(mb);                    // exact, at most 8 bits left
-    h = __byte_perm(ha, hb, 0x7632); m = __byte_perm(ma, mb, 0x7632); l = __byte_perm(__float_as_uint(la), __float_as_uint(lb), 0x7632);
+    // the largest bfloat16 in the place of an infinity: a finite value above it keeps its rest, an infinity leaves one in `m`
+    asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(h) : "f"(b), "f"(a));
+    const float ra = a - __uint_as_float(h << 16), rb = b - __uint_as_float(h & 0xffff0000u);    // exact
+    m = bf16_pair(ra, rb);
+    l = bf16_pair(ra - __uint_as_float(m << 16), rb - __uint_as_float(m & 0xffff0000u));         // exact, at most 8 bits left
 }
 
 // 16 lanes x 16 columns: thread t holds columns 8 s + 2 (t % 4), + 1 of lanes t / 4 (r[4 s], r[4 s + 1]) and t / 4 + 8 (r[4 s + 2], r[4 s + 3])
