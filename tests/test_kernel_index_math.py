@@ -2,6 +2,9 @@
 tests do not reach (group counts that are not powers of two: the reference model's 2560 channels and 640 hidden units): every
 (row, group) pair of a block's rows is visited by exactly one lane, the lanes that share a row form one aligned run whose
 width the shuffle reduction covers, and the staged activation index stays inside the shared-memory extent the host sizes."""
+import os
+
+import numpy as np
 import pytest
 
 BLOCK_ROWS, WARPS = 64, 8
@@ -142,3 +145,30 @@ def test_five_bit_code_assembly():
             assert (q >> (8 * k)) & 255 == want
             bits = _byte_perm(q, 0x4B000000, 0x7440 + k)
             assert np.array([bits], dtype=np.uint32).view(np.float32)[0] - np.float32(8388608.0) == want
+
+
+@pytest.mark.parametrize("vocab", [4096, 20000, 32000, 50257, 151936, 248320])
+def test_topk_merge_candidates_pass_a_tight_bound(vocab):
+    """The merge of the sampler's top-64 rows ranks what passes the warps' bound by counting and falls back to a radix select where more
+    than kTopkCand keys pass: ordinary logits may not get there, and every candidate is visited once."""
+    import re
+    src = open(os.path.join(os.path.dirname(__file__), "..", "tokspur-public_b200", "csrc", "tsp_topk.cu")).read()
+    spread = re.search(r"kTopkSpread = (\d+);", src)
+    spread, limit, cap, threads = int(spread.group(1)) if spread else 0, int(re.search(r"kTopkCand = (\d+);", src).group(1)), 64, 256
+    tiles = (vocab + 4095) // 4096
+    i = np.arange(tiles * cap)
+    t = i // cap
+    s = (i ^ (t * spread)) % cap
+    assert np.array_equal(np.sort(t * cap + s), i)
+    for seed in range(5):
+        v = np.random.default_rng(seed).standard_normal(vocab).astype(np.float32)
+        part = np.full((tiles, cap), -np.inf, dtype=np.float32)
+        for k in range(tiles):
+            best = np.sort(v[k * 4096:(k + 1) * 4096])[::-1][:cap]
+            part[k, :len(best)] = best
+        key = np.full(-(-len(i) // threads) * threads, -np.inf, dtype=np.float32)
+        key[:len(i)] = part[t, s]
+        lanes = key.reshape(-1, threads).max(axis=0).reshape(-1, 32)          # every lane's largest
+        bound = np.sort(lanes, axis=1)[:, -8].min()                           # the smallest of the warps' eighth-largest
+        passed = int((key >= max(bound, np.finfo(np.float32).min)).sum())
+        assert min(64, vocab) <= passed <= limit

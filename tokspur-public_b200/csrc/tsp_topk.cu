@@ -33,6 +33,7 @@ constexpr uint32_t kTopkZero = 0x80000000u;
 __device__ __forceinline__ uint32_t topk_bits(uint32_t image) { return (image & 0x80000000u) ? image ^ 0x80000000u : ~image; }
 
 constexpr uint32_t kTopkCand = 512;   // candidates ranked by counting at most
+constexpr uint32_t kTopkSpread = 7;   // merge: slot s of tile t goes to lane (s ^ 7 t) % 64 of its 64
 struct TopkShared {
     uint32_t hist[256];
     unsigned long long sel[kTopkCand];
@@ -228,10 +229,12 @@ logit_topk_merge_kernel(const uint32_t* partial, uint32_t vocabulary, uint32_t t
     if (valid) atomicAdd(&sh.valid, valid);
     __syncthreads();
     const uint32_t count = min(sh.valid, kTopkCap);
-    // candidates: slot s of tile t is live when s < that tile's count; key = value image above the inverted column (64 bits)
+    // candidates: slot s of tile t is live when s < that tile's count; key = value image above the inverted column (64 bits). A tile's slots are
+    // in descending order: taken in that order every other warp would see slots 32..63 alone, its bound would lie near slot 40 and 1200 to
+    // 2100 keys of a vocabulary of 150 000 to 250 000 would pass. So each tile's slots go round the lanes by an offset of its own.
     const uint32_t cands = tiles * kTopkCap;
     auto key_at = [&](uint32_t i) -> unsigned long long {
-        const uint32_t t = i / kTopkCap, s = i % kTopkCap;
+        const uint32_t t = i / kTopkCap, s = (i ^ (t * kTopkSpread)) % kTopkCap;
         const uint32_t* h = src + static_cast<uint64_t>(t) * kTopkRowWords;
         const uint32_t live = h[1], id = h[4 + s], bits = h[4 + kTopkCap + s];   // three independent loads (every slot of a row exists)
         if (s >= min(live, kTopkCap)) return 0ull;
