@@ -47,3 +47,20 @@ def test_residual_read_write_rows(oracle, tokens, branches, channels, rank):
         want = oracle.residual_write(streams[t], ffn[t], sc32[t])
         assert np.max(np.abs(dst[t].cpu().numpy() - want) / np.maximum(1.0, np.abs(want))) <= 1e-6
     assert int(err.item()) == 0
+
+
+# The write's forms: one branch or four per thread (the last group short), rows of whole 16-byte units and not, in place and not. One FMA per
+# value: within one rounding of the 64-bit result, whose product alone is rounded once more here.
+@pytest.mark.parametrize("tokens,branches,channels", [(1, 4, 2048), (1, 3, 1025), (300, 5, 516), (70, 6, 1025), (257, 1, 2052)])
+def test_residual_write_forms(tokens, branches, channels):
+    g = torch.Generator().manual_seed(tokens + branches)
+    streams, ffn, scales = torch.randn(tokens, branches, channels, generator=g), torch.randn(tokens, channels, generator=g), torch.randn(tokens, branches, generator=g)
+    want = streams.double() + scales.double()[:, :, None] * ffn.double()[:, None, :]
+    ds, df, dc = streams.cuda(), ffn.cuda(), scales.cuda()
+    dst, err = torch.zeros_like(ds), torch.zeros(1, dtype=torch.int32, device="cuda")
+    for out in (dst, ds):
+        capi.call("tsp_residual_write", ds.data_ptr(), df.data_ptr(), dc.data_ptr(), branches, channels, tokens, out.data_ptr(), err.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        got = out.cpu().double()
+        assert torch.all((got - want).abs() <= 2.0 ** -23 * want.abs() + 1e-30)
+    assert int(err.item()) == 0

@@ -72,36 +72,35 @@ residual_read_kernel(const float* normalized, const float* scores, const float* 
 }
 
 // destination[t][b][c] = streams[t][b][c] + scales[t][b] * output[t][c]      (destination may be streams: a thread writes what it read)
-template <uint32_t V>
-__global__ void __launch_bounds__(kResThreads)
+// A thread takes NB branches of one unit; blockIdx.x counts (run of units, group of branches).
+template <uint32_t V, uint32_t NB>
+__global__ void __launch_bounds__(V == 4 ? 128 : 256)
 residual_write_kernel(const float* streams, const float* output, const float* scales, uint32_t branches,
                       uint32_t channels, float* destination, uint32_t* error) {
     using T = typename Chan<V>::T;
     pdl_launch_dependents();
     pdl_wait();
-    const uint32_t t = blockIdx.y, units = channels / V;
+    const uint32_t t = blockIdx.y, units = channels / V, groups = (branches + NB - 1) / NB;
+    const uint32_t run = blockIdx.x / groups, b0 = (blockIdx.x - run * groups) * NB, u = run * blockDim.x + threadIdx.x;
+    if (u >= units) return;
     const uint64_t row = static_cast<uint64_t>(t) * branches * units;
     bool bad = false;
-    for (uint32_t u = blockIdx.x * kResThreads + threadIdx.x; u < units; u += gridDim.x * kResThreads) {
-        T o = reinterpret_cast<const T*>(output)[static_cast<uint64_t>(t) * units + u];
-        for (uint32_t b0 = 0; b0 < branches; b0 += kResBranches) {
-            T s[kResBranches];
-            float f[kResBranches];
+    T o = reinterpret_cast<const T*>(output)[static_cast<uint64_t>(t) * units + u];
+    T s[NB];
+    float f[NB];
 #pragma unroll
-            for (uint32_t b = 0; b < kResBranches; ++b) {
-                const uint32_t bb = min(b0 + b, branches - 1);
-                s[b] = reinterpret_cast<const T*>(streams)[row + static_cast<uint64_t>(bb) * units + u];
-                f[b] = scales[static_cast<uint64_t>(t) * branches + bb];
-            }
+    for (uint32_t b = 0; b < NB; ++b) {
+        const uint32_t bb = min(b0 + b, branches - 1);
+        s[b] = reinterpret_cast<const T*>(streams)[row + static_cast<uint64_t>(bb) * units + u];
+        f[b] = scales[static_cast<uint64_t>(t) * branches + bb];
+    }
 #pragma unroll
-            for (uint32_t b = 0; b < kResBranches; ++b) {
-                if (b0 + b >= branches) break;
-                T v;
+    for (uint32_t b = 0; b < NB; ++b) {
+        if (b0 + b >= branches) break;
+        T v;
 #pragma unroll
-                for (uint32_t i = 0; i < V; ++i) { chan_at(v, i) = fmaf(f[b], chan_at(o, i), chan_at(s[b], i)); bad |= !finite_f32(chan_at(v, i)); }
-                reinterpret_cast<T*>(destination)[row + static_cast<uint64_t>(b0 + b) * units + u] = v;
-            }
-        }
+        for (uint32_t i = 0; i < V; ++i) { chan_at(v, i) = fmaf(f[b], chan_at(o, i), chan_at(s[b], i)); bad |= !finite_f32(chan_at(v, i)); }
+        reinterpret_cast<T*>(destination)[row + static_cast<uint64_t>(b0 + b) * units + u] = v;
     }
     if (bad) raise_error(error, TSP_ERR_NONFINITE);
 }
@@ -125,10 +124,13 @@ int launch_residual_read(const float* normalized, const float* scores, const flo
 int launch_residual_write(const float* streams, const float* output, const float* scales, uint32_t branches, uint32_t channels, uint32_t tokens,
                           float* destination, uint32_t* error, cudaStream_t st) {
     const bool v4 = whole_units(channels, {streams, output, destination});
-    const uint32_t units = v4 ? channels / 4 : channels;
-    const dim3 grid((units + kResThreads - 1) / kResThreads, tokens);
-    TSP_CUDA(launch_pdl(v4 ? residual_write_kernel<4> : residual_write_kernel<1>, grid, dim3(kResThreads), 0, st, streams, output, scales, branches, channels,
-                        destination, error));
+    const uint32_t threads = v4 ? 128 : 256, units = v4 ? channels / 4 : channels, runs = (units + threads - 1) / threads;
+    // One branch per thread while that is about one wave of blocks: 64 rows of 4 x 2560 1.7 us against 2.0 with four branches per thread, 256
+    // rows of 4 x 2048 4.8 us against 3.5. (Every branch in one thread: 64 rows of 16 x 4096 7.2 us, now 4.2; 2000 rows of 4 x 2050 43 us, now 27.)
+    const bool single = static_cast<uint64_t>(runs) * branches * tokens <= 8u * 148u;
+    const dim3 grid(runs * (single ? branches : (branches + 3) / 4), tokens);
+    auto kernel = v4 ? (single ? residual_write_kernel<4, 1> : residual_write_kernel<4, 4>) : (single ? residual_write_kernel<1, 1> : residual_write_kernel<1, 4>);
+    TSP_CUDA(launch_pdl(kernel, grid, dim3(threads), 0, st, streams, output, scales, branches, channels, destination, error));
     return TSP_OK;
 }
 
