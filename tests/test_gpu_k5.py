@@ -216,3 +216,25 @@ def test_nonfinite_scale_sets_the_error_word():
     capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), 256, 1, 1, 1, None, None, None, out.data_ptr(), 64, 0, e.data_ptr(), L.stream_ptr())
     torch.cuda.synchronize()
     assert int(e.item()) & capi.ERR_NONFINITE
+
+
+# Infinities and NaN in a token row, on the MMA kernel's tiles (8 rows) and the FP32 kernel's (16): reported, and every other row as without them
+@pytest.mark.parametrize("T", [3, 8, 16])
+@pytest.mark.parametrize("type_,rows,cols", [(formats.Q5_K, 32, 512), (formats.Q5_1, 32, 128)])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_nonfinite_activation_row(type_, rows, cols, T, bad):
+    w = formats.quantize(type_, synth.normal(95, (rows, cols), 0.02)).reshape(-1)
+    t = dev(w)
+    ms = L.matrix_set(t, type_, formats.GGUF, rows, cols, 1)
+    x = synth.normal(96, (T, cols), 1.0)
+    outs = []
+    for value in (x[1, 5], bad):
+        x[1, 5] = value
+        dx, out, e = dev(x), torch.zeros((T, rows), dtype=torch.float32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, 1, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        assert bool(int(e.item()) & capi.ERR_NONFINITE) == (not np.isfinite(value))
+        outs.append(out.cpu().numpy())
+    others = [i for i in range(T) if i != 1]
+    assert np.array_equal(outs[0][others], outs[1][others])
+    assert not np.isfinite(outs[1][1]).any()

@@ -290,13 +290,14 @@ __device__ __noinline__ void k5_wide_row(const uint8_t* rowsA, const uint8_t* ro
         const uint32_t r = rb + sub;
         const bool live = r < rows;
         const uint32_t at = (live ? r : rb) * row_bytes;
-        ok &= k5_row_f32<TYPE, GATEUP, 1u>(
+        const bool weights = k5_row_f32<TYPE, GATEUP, 1u>(
             rowsA + at, rowsB + at, groups, lpr, lig, 1u, [&](uint32_t, uint32_t grp, uint32_t i4) { return x4[grp * 8u + i4]; },
             [&](uint32_t, float v) {
                 if (!live) return;
-                ok &= finite_f32(v);
+                ok = ok && finite_f32(v);
                 out[r] = v;
             });
+        ok = ok && weights;
     }
     if (!ok) raise_error(error, TSP_ERR_NONFINITE);
 }
