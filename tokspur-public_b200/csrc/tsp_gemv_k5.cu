@@ -310,7 +310,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
     __shared__ const float* s_x[8];
     __shared__ float* s_out[8];
     __shared__ float s_scale[8], s_inv[8];
-    __shared__ uint32_t s_wide[8];
+    __shared__ __align__(8) uint8_t s_wide[8];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t groups = p.cols / 32u, x_stride = p.cols * 2u + 64u;
     uint8_t* const xhi = km_smem;
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
                 s_x[warp] = x;
                 s_out[warp] = reinterpret_cast<float*>(reinterpret_cast<char*>(p.out) + static_cast<uint64_t>(rid) * p.out_stride_bytes);
             }
-        }
+        } else if (lane == 0) s_wide[warp] = 0;
         __syncthreads();
         // stage: a thread takes the eight values that lane tq of a group multiplies, in the MMA's order
         for (uint32_t i = threadIdx.x; i < count * groups * 4u; i += kKmWarps * 32) {
@@ -370,16 +370,17 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
             const float sc = s_scale[j];
             const float v[8] = {f0.x * sc, f0.z * sc, f0.y * sc, f0.w * sc, f1.x * sc, f1.z * sc, f1.y * sc, f1.w * sc};   // order 0,2,1,3
             uint32_t h[8], l[8];
-            float sum = 0.f, most = 0.f;
+            float sum = 0.f;
+            const float most = fmaxf(fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3]))),
+                                     fmaxf(fmaxf(fabsf(v[4]), fabsf(v[5])), fmaxf(fabsf(v[6]), fabsf(v[7]))));
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                most = fmaxf(most, fabsf(v[q]));
                 const __half hv = __float2half_rn(v[q]);
                 h[q] = __half_as_ushort(hv);
                 l[q] = __half_as_ushort(__float2half_rn(v[q] - __half2float(hv)));
                 sum += v[q];
             }
-            if (most < kKmNarrow && most > 0.f) s_wide[j] = 1u;
+            if (most < kKmNarrow && most > 0.f) s_wide[j] = 1;
             uint8_t* dst = xhi + j * x_stride + grp * 64u + tq * 16u;
             *reinterpret_cast<uint4*>(dst) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
             *reinterpret_cast<uint4*>(dst + (packed ? 4u : 8u) * x_stride) = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
@@ -394,6 +395,8 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
         }
         __syncthreads();
         if (!live) continue;
+        const uint2 wide8 = *reinterpret_cast<const uint2*>(s_wide);
+        const bool wide = (wide8.x | wide8.y) != 0;   // some row of the tile
         float total[4] = {0.f, 0.f, 0.f, 0.f}, low[4] = {0.f, 0.f, 0.f, 0.f};   // low: the low halves' sums of a tile that is not packed
         bool ok = true;
         const uint8_t* xh = xhi + g * x_stride + t * 16u;
@@ -437,7 +440,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
 #pragma unroll
         for (uint32_t q = 0; q < 2; ++q) {
             const uint32_t j = 2 * t + q;
-            if (j >= count || s_wide[j]) continue;
+            if (j >= count || (wide && s_wide[j])) continue;
             const float inv = s_inv[j], va = total[q] * inv, vb = total[2 + q] * inv;
             float* o = s_out[j] + r0 + g;
             if (GATEUP) {
@@ -449,7 +452,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
                 o[0] = va; o[8] = vb;
             }
         }
-        for (uint32_t j = 0; j < count; ++j)   // uniform over the block
+        for (uint32_t j = 0; wide && j < count; ++j)   // uniform over the block
             if (s_wide[j]) k5_wide_row<TYPE, GATEUP>(wA - static_cast<uint64_t>(g) * p.row_bytes, GATEUP ? wB - static_cast<uint64_t>(g) * p.row_bytes : wA - static_cast<uint64_t>(g) * p.row_bytes,
                                                         p.row_bytes, RW, groups, p.lanes_per_row, s_x[j], s_out[j] + r0, p.error);
     }
