@@ -238,3 +238,21 @@ def test_nonfinite_activation_row(type_, rows, cols, T, bad):
     others = [i for i in range(T) if i != 1]
     assert np.array_equal(outs[0][others], outs[1][others])
     assert not np.isfinite(outs[1][1]).any()
+
+
+@pytest.mark.parametrize("T", [1, 5])
+def test_rows_do_not_depend_on_how_a_dense_launch_is_split(T):
+    """Dense launches of 16, 2400, 4800 and 9616 rows take one, two, four and eight warps per block's item: a row comes out the same."""
+    rows, cols = 9616, 128
+    w = formats.quantize(formats.Q5_1, synth.normal(97, (rows, cols), 0.02)).reshape(rows, -1)
+    dx, e, outs = dev(synth.normal(98, (T, cols), 1.0)), torch.zeros(1, dtype=torch.int32, device=DEV), []
+    for n in (9616, 4800, 2400, 16):
+        t = dev(w[:n].reshape(-1))
+        ms = L.matrix_set(t, formats.Q5_1, formats.GGUF, n, cols, 1)
+        out = torch.zeros((T, n), dtype=torch.float32, device=DEV)
+        capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, 1, T, 1, None, None, None, out.data_ptr(), n * 4, 0, e.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        outs.append(out.cpu().numpy())
+    assert int(e.item()) == 0
+    for o in outs[1:]:
+        assert np.array_equal(o, outs[0][:, :o.shape[1]])

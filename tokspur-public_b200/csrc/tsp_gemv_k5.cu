@@ -24,6 +24,7 @@ struct K5Params {
     const float* x; uint64_t x_stride_bytes; uint32_t in_div;
     const uint32_t* token_map; const uint32_t* counts; const uint32_t* tasks;
     uint32_t tokens, tile_tokens;
+    uint32_t item_warps;      // MMA kernel, SPLIT: warps of a block that take rows of an item
     uint32_t lanes_per_row;   // lanes that share one weight row: the largest power of two <= min(32, groups)
     float* out; uint64_t out_stride_bytes;
     uint32_t* error;
@@ -303,7 +304,8 @@ __device__ __noinline__ void k5_wide_row(const uint8_t* rowsA, const uint8_t* ro
 }
 
 // Shared memory: high halves [8][x_stride], low halves [8][x_stride], group sums [group][8] (of the scaled values)
-template <uint32_t TYPE, bool GATEUP>
+// SPLIT: only the first item_warps warps of a block take rows (all of them stage).
+template <uint32_t TYPE, bool GATEUP, bool SPLIT>
 __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5Params p) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) uint8_t km_smem[];
@@ -320,10 +322,10 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
     const uint32_t steps = groups / Step::kGroups;
     pdl_wait();
     const uint32_t n_tiles = p.token_map ? p.tasks[0] : (p.tokens + 7u) / 8u;
-    const uint32_t row_items = (p.rows + RW * kKmWarps - 1) / (RW * kKmWarps);
+    const uint32_t item_rows = RW * (SPLIT ? p.item_warps : kKmWarps), row_items = (p.rows + item_rows - 1) / item_rows;
     const uint32_t n_items = n_tiles * row_items;
     for (uint32_t item = blockIdx.x; item < n_items; item += gridDim.x) {   // uniform over the block
-        const uint32_t tile = item / row_items, r0 = (item - tile * row_items) * (RW * kKmWarps) + warp * RW;
+        const uint32_t tile = item / row_items, r0 = (item - tile * row_items) * item_rows + warp * RW;
         uint32_t expert = 0, start = tile * 8u, count = 0;
         if (p.token_map) {
             expert = p.tasks[2 + 2 * tile];
@@ -336,13 +338,13 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
         const bool hi = expert >= p.split;
         const uint64_t eoff = static_cast<uint64_t>(hi ? expert - p.split : expert) * p.expert_stride;
         const uint8_t* baseA = (hi ? p.a_base_hi : p.a_base) + eoff;
-        const bool live = r0 < p.rows;   // whole warps: rows are a multiple of RW
+        const bool live = (!SPLIT || warp < p.item_warps) && r0 < p.rows;   // whole warps: rows are a multiple of RW
         const uint32_t rowA = (live ? r0 : 0u) + g;
         const uint8_t* wA = baseA + static_cast<uint64_t>(rowA) * p.row_bytes;
         const uint8_t* wB = GATEUP ? (hi ? p.b_base_hi : p.b_base) + eoff + static_cast<uint64_t>(rowA) * p.row_bytes
                                    : baseA + static_cast<uint64_t>(rowA + 8u) * p.row_bytes;
         Step nA, nB;
-        nA.load(wA, t); nB.load(wB, t);   // on their way while the rows are staged
+        if (!SPLIT || live) { nA.load(wA, t); nB.load(wB, t); }   // on their way while the rows are staged
         __syncthreads();                  // the previous item's rows are no longer read
         if (warp < count) {               // warp j: route id and scale of token row j
             const uint32_t rid = p.token_map ? p.token_map[static_cast<uint64_t>(expert) * p.tokens + start + warp] : start + warp;
@@ -480,12 +482,16 @@ int launch_dequant_k5(uint32_t type, const uint8_t* m, uint64_t elements, float*
     return TSP_OK;
 }
 
+template <uint32_t TYPE, bool GATEUP, bool SPLIT>
+static int launch_km_t(const K5Params& p, size_t smem, int grid, cudaStream_t st) {
+    static thread_local SmemAttrCache configured;   // per kernel instantiation, keyed by device
+    TSP_CUDA(ensure_dynamic_smem(gemv_k5_mma_kernel<TYPE, GATEUP, SPLIT>, configured, smem));
+    TSP_CUDA(launch_pdl(gemv_k5_mma_kernel<TYPE, GATEUP, SPLIT>, dim3(grid), dim3(kKmWarps * 32), smem, st, p));
+    return TSP_OK;
+}
 template <uint32_t TYPE, bool GATEUP>
 static int launch_km(const K5Params& p, size_t smem, int grid, cudaStream_t st) {
-    static thread_local SmemAttrCache configured;   // per kernel instantiation, keyed by device
-    TSP_CUDA(ensure_dynamic_smem(gemv_k5_mma_kernel<TYPE, GATEUP>, configured, smem));
-    TSP_CUDA(launch_pdl(gemv_k5_mma_kernel<TYPE, GATEUP>, dim3(grid), dim3(kKmWarps * 32), smem, st, p));
-    return TSP_OK;
+    return p.item_warps < kKmWarps ? launch_km_t<TYPE, GATEUP, true>(p, smem, grid, st) : launch_km_t<TYPE, GATEUP, false>(p, smem, grid, st);
 }
 
 template <uint32_t TYPE, bool GATEUP, uint32_t MT>
@@ -524,6 +530,11 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     while (p.lanes_per_row * 2 <= groups && p.lanes_per_row < 32) p.lanes_per_row *= 2;
     // Tiles of up to 8 rows take the MMA kernel where a warp's rows are whole and two blocks' rows fit an SM's shared memory (up to 2944
     // columns); dense batches of more rows (16 per tile) and the other shapes keep the FP32 FMA kernel.
+    // A dense launch of fewer than half as many items as SMs takes fewer warps per item: eight would leave most SMs idle (one row of Q5_1
+    // 2048 x 512: 7.0 us on 16 SMs, the FP32 kernel's 32 blocks 5.5; 4.3 us on 128). Routed launches learn their items on the device; with the
+    // count of warps a variable there, too, a layer of 64 rows took 506 us instead of 491.
+    const uint32_t row_warps = (a->rows + (gateup ? 7u : 15u)) / (gateup ? 8u : 16u), dense_tiles = (tokens + p.tile_tokens - 1) / p.tile_tokens;
+    for (p.item_warps = kKmWarps; !token_map && p.item_warps > 1 && 2ull * dense_tiles * ((row_warps + p.item_warps - 1) / p.item_warps) <= static_cast<uint32_t>(sms);) p.item_warps /= 2;
     const size_t km_smem = 16u * (a->cols * 2u + 64u) + groups * 32u;
     if (nc == 1 && a->rows % (gateup ? 8 : 16) == 0 && groups % (a->type == TSP_TYPE_Q5_K ? 8 : 4) == 0 && km_smem <= 110 * 1024) {
         if (a->type == TSP_TYPE_Q5_K) return gateup ? launch_km<13u, true>(p, km_smem, 2 * sms, st) : launch_km<13u, false>(p, km_smem, 2 * sms, st);
@@ -533,7 +544,6 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     if (smem > 200 * 1024) return fail(TSP_E_ARG, "five-bit projection: %u columns x %u token rows do not fit the activation staging", a->cols, p.tile_tokens);
     // routed launches learn their tile count on the device: a fixed number of block rows walks the tiles (a routed launch has at
     // most 64 routes per token row, one tile each at worst)
-    const uint32_t dense_tiles = (tokens + p.tile_tokens - 1) / p.tile_tokens;
     const uint64_t routed_cap = static_cast<uint64_t>(tokens) * 64u;
     const uint32_t walkers = static_cast<uint32_t>(routed_cap < 4u * static_cast<uint32_t>(sms) ? routed_cap : 4u * static_cast<uint32_t>(sms));
     const dim3 grid((a->rows + kK5BlockRows - 1) / kK5BlockRows, token_map ? walkers : (dense_tiles < 1024u ? dense_tiles : 1024u));
