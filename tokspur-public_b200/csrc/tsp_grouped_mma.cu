@@ -67,7 +67,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // One K chunk of 64: four D[tmem] (+)= A[tmem] * B[smem], kind::f16, one CTA, then a commit on `bar` (it completes when the MMAs have
 // read their operands). Called by a whole warp with uniform arguments; one elected lane issues. (A lane picked by `lane == 0` in
@@ -898,7 +897,8 @@ int launch_grouped(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     TSP_REQUIRE(a->rows % rm == 0 && a->cols % 256 == 0, "grouped GEMM: rows must be a multiple of %u and columns of 256", rm);
     GroupedParams p{};
     const uint32_t nblk = q8 ? a->cols / 128 : a->cols / 256;
-    TSP_REQUIRE(a->cols / 256 <= 32, "grouped GEMM: K extent too large");
+    // Q4_K up to 2048 columns: the rows that this kernel has been run on (more would need another look at the (d, dmin) ring beside the stages)
+    TSP_REQUIRE(a->cols / 256 <= (q8 ? 32u : 8u), "grouped GEMM: at most %u columns in this encoding", q8 ? 8192u : 2048u);
     p.split = a->split < a->experts ? a->split : a->experts;
     p.experts = a->experts;
     p.nblk = nblk; p.chunks = a->cols / 64; p.row_blocks = a->rows / rm;
@@ -926,7 +926,7 @@ int launch_grouped(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
         smem = p.off_ep + kEpWarps * ep_tile_bytes(gateup) + 1024;
         if (smem <= 227 * 1024) break;
     }
-    TSP_REQUIRE(p.d_stage_bytes <= 4096 && smem <= 227 * 1024, "grouped GEMM: K extent needs more shared memory than one SM has");
+    TSP_REQUIRE(smem <= 227 * 1024, "grouped GEMM: %zu bytes of shared memory are more than one SM has", smem);
 
     // gate and up of an expert at one constant distance: one copy per plane brings both
     auto mergeable = [](const uint8_t* first, const uint8_t* second, uint64_t* delta) {
