@@ -101,3 +101,26 @@ def test_staged_weight_values_against_rounded_reference(oracle):
     dev = (np.abs(got - once).reshape(rows, cols // 32, 32) / np.maximum(group_max, 1e-30)).max()
     print(f"staged weights: rel-L2 vs exact {rel:.3e} (one rounding: {rel_once:.3e}), worst deviation from RN16 {dev:.3e} of the group maximum")
     assert rel <= 4e-4 and dev <= 2.0 ** -10
+
+
+def test_overflowing_hidden_row_is_reported_and_stays_alone(oracle):
+    """Finite input rows whose hidden values pass binary16's range (the gate-up epilogue's test, with the columns past an expert's last route
+    holding other experts' rows): reported; every other token row comes out as without them. One step below, nothing is reported."""
+    Cn, H, E, K, T = 256, 256, 4, 2, 150
+    host = L.synth_host_layer(23, Cn, H, E, K, expert_type=formats.Q4_K)
+    x16, logits = synth.activations_f16(24, T, Cn), synth.router_logits(25, T, E)
+    outs = []
+    for scale in (1.0, 64.0, 16384.0):   # hidden values of the row about 0.1, 400 and 3e7
+        x = x16.copy()
+        x[77] = (x[77].astype(np.float32) * scale).clip(-60000, 60000).astype(np.float16)
+        assert np.isfinite(x).all()
+        dl = L.DeviceLayer(host, formats.PLANAR, "cuda")
+        ps = L.PrefillScratch(Cn, H, E, K, T, "cuda")
+        out = torch.zeros((T, Cn), dtype=torch.float32, device="cuda")
+        L.moe_layer_prefill(dl, ps, torch.from_numpy(x.astype(np.float32)).cuda(), torch.from_numpy(logits).cuda(), out)
+        torch.cuda.synchronize()
+        assert bool(ps.base.error_word() & capi.ERR_NONFINITE) == (scale > 1000)
+        outs.append(out.cpu().numpy())
+    others = np.arange(T) != 77
+    assert np.array_equal(outs[0][others], outs[1][others]) and np.array_equal(outs[0][others], outs[2][others])
+    assert np.isfinite(outs[1]).all() and not np.isfinite(outs[2][77]).all()

@@ -139,3 +139,24 @@ def test_route_ties_and_signed_zeros(oracle, T, E, K):
         assert np.array_equal(ids.cpu().numpy().view(np.uint32).reshape(T, K), oi)
         assert np.max(np.abs(wt.cpu().numpy().reshape(T, K) - ow)) <= 1e-6
     assert int(err.item()) == 0
+
+
+# Infinities and NaN go through the three parts of the tensor-core product (130 rows) as through the FP32 chain (5): reported, and every other
+# output as without them
+@pytest.mark.parametrize("T", [5, 130])
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+def test_nonfinite_router_inputs(T, bad):
+    rows, cols = 70, 256
+    w, x = synth.normal(31, (rows, cols), 0.05), synth.normal(32, (T, cols))
+    clean, _ = project(w, x)
+    xb, wb = x.copy(), w.copy()
+    xb[3, 9] = bad
+    wb[66, 100] = bad
+    for ww, xx, keep in ((w, xb, (np.arange(T) != 3)[:, None] & np.ones(rows, bool)), (wb, x, (np.arange(rows) != 66) & np.ones((T, 1), bool))):
+        dw, dx = torch.from_numpy(ww).cuda(), torch.from_numpy(xx).cuda()
+        out, err = torch.zeros((T, rows), dtype=torch.float32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        capi.call("tsp_router_project", dw.data_ptr(), rows, cols, None, dx.data_ptr(), cols * 4, T, out.data_ptr(), rows * 4, None, err.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        assert int(err.item()) & capi.ERR_NONFINITE
+        assert np.array_equal(got[keep], clean[keep]) and not np.isfinite(got[~keep]).any()
