@@ -620,8 +620,8 @@ def run_ours(args):
                                  "h2d_bytes_per_step": rec["h2d_bytes_per_step"], "d2h_bytes_per_step": rec["d2h_bytes_per_step"]},
                          "gpu_launches": 9 * max(4, args.steps // 4),
                          "roofline": {"bound": "tensor", "kernel": "grouped_mma_kernel<gate-up> (routed experts + shared expert, tcgen05)", "achieved": rec["gate_up_launch_tflops"],
-                                      "peak": tf_peak, "unit": "TFLOP/s", "frac": rec["gate_up_launch_frac_of_bf16_peak"], "peak_kind": peak_kind, "traffic": 478.4e6 if Tp == 4096 else None,
-                                      "traffic_source": "profiles/grouped_mma_prefill_T4096.md (ncu: DRAM throughput x duration of the gate-up launch)",
+                                      "peak": tf_peak, "unit": "TFLOP/s", "frac": rec["gate_up_launch_frac_of_bf16_peak"], "peak_kind": peak_kind, "traffic": 471.3e6 if Tp == 4096 and p_layout == formats.PLANAR and sh_type is None else None,
+                                      "traffic_source": "profiles/grouped_mma_prefill_T4096.md (ncu: DRAM bytes read and written by the gate-up launch)",
                                       "launch_ms": rec["stage_ms"]["gate_up_ms"]},
                          "cpu_baseline": cpu, "extra": {"prefill": rec}})
         else:

@@ -267,7 +267,7 @@ int tsp_gemv_f32(const float* d_w, uint32_t rows, uint32_t cols, const float* d_
  * of the shared-router vector as a launch of its own, d_extra_out[t] = sum_c d_extra_row[c] x[t][c] (both NULL: none).
  * The ids chosen from these logits have to follow the reference's double-precision logits, so the error is that of FP32 sums or
  * less: up to 95 token rows one FP32 FMA chain per lane, from 96 on tensor-core products of the three bfloat16 parts that each
- * FP32 value splits into exactly (a term's error stays within 2^-24 of it, 3.4e-7 for 2048 columns in the relative 2-norm, an FP32
+ * FP32 value splits into exactly (a term's error stays within 2^-24 of it, 2.4e-7 for 2048 columns in the relative 2-norm, one FP32
  * chain 8.1e-7; magnitudes below 2^-109 keep fewer bits). tsp_moe_route_audit tells how close each row's selection is to changing. */
 int tsp_router_project(const float* d_w, uint32_t rows, uint32_t cols, const float* d_extra_row, const float* d_x, uint64_t x_stride_bytes,
                        uint32_t tokens, float* d_out, uint64_t out_stride_bytes, float* d_extra_out, uint32_t* d_error, void* stream);

@@ -1,14 +1,16 @@
 // Decode-size routed / dense projections over the five-bit encodings of the reference's model: Q5_K (176-byte super-blocks of
 // 256 weights; gate and up tensors) and Q5_1 (24-byte blocks of 32 weights; down tensors), plain GGUF rows.
 //
+// Two kernels: tiles of up to eight token rows (every routed launch) take warp-level MMAs on the five-bit codes (gemv_k5_mma_kernel, below);
+// dense batches of more rows and shapes that are not whole warps or too long take FP32 FMAs on exactly rounded weights:
+//
 // A block takes one token tile and a run of weight rows. It first stages the tile's FP32 activation rows in shared memory
 // (32-value groups padded to 36 values, so that 32 lanes reading 16 bytes each at a group stride touch every bank equally). Then
 // the lanes of a warp spread over the K extent of one weight row (gate-up: the gate row and the up row of one hidden unit): a
 // lane takes one 32-weight group at a time with 16-byte loads that are contiguous across the warp, decodes it to the exactly
 // rounded FP32 weights (numeric.cpp:38-50: d * sc * q and dmin * mn are exact in FP32, so one FMA gives the reference's rounded
 // value), multiplies with the staged activations and keeps one FP32 sum per token; the lanes' sums are added with shuffles.
-// Weight bytes are read once per (tile, row). FP32 FMAs, no tensor cores, no copy pipeline: a plain path for the encodings the
-// benchmark configurations do not use.
+// Weight bytes are read once per (tile, row).
 #include "tsp_common.cuh"
 
 namespace tsp {
@@ -190,14 +192,14 @@ __global__ void __launch_bounds__(kK5Threads) gemv_k5_kernel(const K5Params p) {
 // dependent load latencies. Here the five-bit codes enter the MMA as binary16 integers code - 16 (three or four operations per pair),
 // the group's scale s and offset 16 s + m are applied to FP32 sums, the offset through the group's FP32 activation sum. Centred codes
 // keep both terms as small as the weights themselves; with codes 0..31 a weight near zero is the difference of two large terms.
-// Activations enter as binary16 high + low halves after a power-of-two scaling of their row to [2^14, 2^15): the pair keeps 22 bits of
-// every value and an absolute 2^-40 of the row's largest, for rows anywhere in FP32's range.
+// Activations enter as binary16 high + low halves after a power-of-two scaling of the row's largest to [2^14, 2^15): the pair keeps 22 bits of
+// every value, down to 2^-25 after scaling (2^-39 of the row's largest), for rows anywhere in FP32's range.
 // A warp owns 8 hidden units (8 gate + 8 up rows) or 16 plain rows over the whole K, its weights loaded straight into registers one
 // step ahead (a row's bytes are read by the four lanes that use them: 32-byte pieces); blocks of eight warps walk (tile, row block)
 // items, two blocks per SM, so that one streams while the other stages its rows.
 // The groups of a step are summed by themselves before they join the total: one chain over K of 2048 was further from 64-bit sums
 // (2.1e-7, relative 2-norm) than the FP32 kernel (1.5e-7).
-// Measured, layer of 512 experts of 512 x 2048, 13 rows of ten: gate-up 115 -> 72 us, down 73 -> 63 us.
+// Measured against the FP32 kernel, whole layer of 512 experts of 512 x 2048, ten per token: 13 rows 228 -> 187 us, 64 rows 644 -> 492 us.
 // ---------------------------------------------------------------------------------------------
 constexpr uint32_t kKmWarps = 8;
 
@@ -528,7 +530,7 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     if (sms <= 0) return fail(TSP_E_CUDA, "no usable CUDA device");
     p.lanes_per_row = 1;
     while (p.lanes_per_row * 2 <= groups && p.lanes_per_row < 32) p.lanes_per_row *= 2;
-    // Tiles of up to 8 rows take the MMA kernel where a warp's rows are whole and two blocks' rows fit an SM's shared memory (up to 2944
+    // Tiles of up to 8 rows take the MMA kernel where a warp's rows are whole and two blocks' rows fit an SM's shared memory (up to 3328
     // columns); dense batches of more rows (16 per tile) and the other shapes keep the FP32 FMA kernel.
     // A dense launch of fewer than half as many items as SMs takes fewer warps per item: eight would leave most SMs idle (one row of Q5_1
     // 2048 x 512: 7.0 us on 16 SMs, the FP32 kernel's 32 blocks 5.5; 4.3 us on 128). Routed launches learn their items on the device; with the

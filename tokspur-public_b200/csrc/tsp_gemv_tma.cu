@@ -480,7 +480,7 @@ __global__ void __launch_bounds__((W + kProd3) * 32, 1) gemv3_kernel(const __gri
                 }
                 const uint8_t* sb = my_stage0 + s * p.stage_bytes;
                 // rolled: four copies of the body are 17 KB of code (22 KB with the low-half pass); eight warps at different points of it wait
-                // for instructions (decode layer: 1 row 139 -> 131 us for four layers, 8 rows 154 -> 141 us for two, 64 rows 196 -> 189 us)
+                // for instructions (unrolled / rolled: 1 row 154 / 140 us for four layers, 8 rows 141 / 132 us for two, 64 rows 196 / 193 us)
                 if (ok)
 #pragma unroll 1
                 for (uint32_t bl = 0; bl < KB; ++bl) {

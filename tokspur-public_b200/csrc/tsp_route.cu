@@ -604,8 +604,10 @@ gemv_f32_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, ui
 }
 
 int launch_router_mma(const float*, uint32_t, uint32_t, const float*, uint64_t, uint32_t, float*, uint64_t, uint32_t*, cudaStream_t);
-// Fewest token rows for the tensor-core product (512 matrix rows): its one wave of blocks takes 18 us at 1024 columns and 32 us at
-// 2048 whatever the batch; one warp per output takes 15 us at 63 rows of 1024 columns, 15 us at 32 and 24 us at 63 rows of 2048.
+// Fewest token rows for the tensor-core product, from 512 matrix rows: its one wave of blocks takes 18 us at 1024 columns and 28 us at 2048
+// whatever the batch; one warp per output takes 15 us at 63 rows of 1024 columns, 20 us at 64 and 28 us at 95 rows of 2048. The warp form scales
+// with matrix rows x token rows (64 matrix rows: 8 us at 95 token rows of 2048 columns), the other does not (28 us at 96), so a matrix of fewer
+// rows would change over later: about 48 k outputs.
 constexpr uint32_t kRouterMmaTokens = 96;
 
 int launch_gemv_f32(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x, uint64_t x_stride, uint32_t tokens, float* out,

