@@ -138,7 +138,7 @@ def test_outliers_at_zero_weights(oracle, type_, rows, cols, gate_up):
     assert not w64[:, :width].any()
     x = synth.normal(85, (8, cols), 1.0)
     for j in range(1, 8):
-        x[j, 3] = 2.0 ** (0, 8, 9, 11, 24, 39, 60, 120)[j]
+        x[j, 3] = 2.0 ** (0, 8, 13, 16, 24, 39, 60, 120)[j]
     x64 = x.astype(np.float64)
     want = x64 @ w64.T
     bound = (cols + 8) * 2.0 ** -24 * 4 * np.abs(w64).max() * np.abs(x64[:, width:]).sum(axis=1)[:, None]   # a term: see the tile edges above

@@ -276,33 +276,47 @@ template <> struct KmStep<7u> {
     }
 };
 
-// Rows that the split would not serve take the FP32 sums (k5_row_f32, one warp's rows and one token row at a time, straight from global
-// memory): rows with a run of eight values, not all zero, that are all below 2^4 after scaling (2^-10 of the row's largest). The halves
-// end at 2^-25, so what stays on the MMAs is good to 2^-29 of the largest value beside it, and an outlier more than 2^10 times larger that
-// meets weights of zero does not drown it. Infinities and NaN go the same way, and a row's path depends on that row alone.
-// Normally distributed rows never get there (2048 values: 1e-18 per row).
-constexpr float kKmNarrow = 16.f;
+// Rows that the split would not serve take the FP32 sums (k5_row_f32, by the warp that has the matrix rows, straight from global memory): rows
+// with a run of eight values, not all zero, that are all below 1 after scaling (2^-14 of the row's largest or less). The halves end at
+// 2^-25, so in every run that stays on the MMAs the values are good to 2^-25 of its largest, as good as FP32's own rounding of that one,
+// whatever outlier is beside it. Infinities and NaN go the same way, and a row's path depends on that row alone. Normally distributed rows never
+// get there. Layers whose input rows all hold an outlier of 5000 (the limit at 2^-10 and one row at a time / now / the FP32 kernel): 13 rows
+// 492 / 264 / 231 us, 64 rows on 16 experts 949 / 297 / 323 us.
+constexpr float kKmNarrow = 1.f;
 
-// Out of line: the rare path takes no registers from the loop above it.
+// What a tile's rows need in shared memory, and what the rare path below reads of the launch (from here, so that the kernel keeps nothing for it)
+struct KmTile {
+    const float* x[8]; float* out[8]; float scale[8], inv[8];
+    alignas(8) uint8_t wide[8];   // rows that take FP32 sums
+    uint32_t row_bytes, groups, lanes_per_row; uint32_t* error;
+};
+
+// Out of line: the rare path takes no registers from the loop above it. Up to four token rows at a time; out row r of the warp's `rows` at r0 + r.
 template <uint32_t TYPE, bool GATEUP>
-__device__ __noinline__ void k5_wide_row(const uint8_t* rowsA, const uint8_t* rowsB, uint32_t row_bytes, uint32_t rows, uint32_t groups, uint32_t lpr, const float* x, float* out, uint32_t* error) {
+__device__ __noinline__ void k5_wide_rows(const KmTile* tile, const uint8_t* rowsA, const uint8_t* rowsB, uint32_t count, uint32_t r0) {
+    const uint32_t lpr = tile->lanes_per_row, groups = tile->groups, row_bytes = tile->row_bytes, rows = GATEUP ? 8u : 16u;
     const uint32_t lane = threadIdx.x & 31u, rpw = 32u / lpr, sub = lane / lpr, lig = lane & (lpr - 1u);
-    const float4* x4 = reinterpret_cast<const float4*>(x);
     bool ok = true;
-    for (uint32_t rb = 0; rb < rows; rb += rpw) {
-        const uint32_t r = rb + sub;
-        const bool live = r < rows;
-        const uint32_t at = (live ? r : rb) * row_bytes;
-        const bool weights = k5_row_f32<TYPE, GATEUP, 1u>(
-            rowsA + at, rowsB + at, groups, lpr, lig, 1u, [&](uint32_t, uint32_t grp, uint32_t i4) { return x4[grp * 8u + i4]; },
-            [&](uint32_t, float v) {
-                if (!live) return;
-                ok = ok && finite_f32(v);
-                out[r] = v;
-            });
-        ok = ok && weights;
+    for (uint32_t j = 0; j < count;) {
+        uint32_t n = 0, list = 0;   // the next wide rows, four bits each
+        for (; j < count && n < 4; ++j) if (tile->wide[j]) list |= j << (4u * n++);
+        if (!n) break;
+        for (uint32_t rb = 0; rb < rows; rb += rpw) {
+            const uint32_t r = rb + sub;
+            const bool live = r < rows;
+            const uint32_t at = (live ? r : rb) * row_bytes;
+            const bool weights = k5_row_f32<TYPE, GATEUP, 4u>(
+                rowsA + at, rowsB + at, groups, lpr, lig, n,
+                [&](uint32_t k, uint32_t grp, uint32_t i4) { return reinterpret_cast<const float4*>(tile->x[(list >> (4u * k)) & 15u])[grp * 8u + i4]; },
+                [&](uint32_t k, float v) {
+                    if (!live) return;
+                    ok = ok && finite_f32(v);
+                    tile->out[(list >> (4u * k)) & 15u][r0 + r] = v;
+                });
+            ok = ok && weights;
+        }
     }
-    if (!ok) raise_error(error, TSP_ERR_NONFINITE);
+    if (!ok) raise_error(tile->error, TSP_ERR_NONFINITE);
 }
 
 // Shared memory: high halves [8][x_stride], low halves [8][x_stride], group sums [group][8] (of the scaled values)
@@ -311,10 +325,8 @@ template <uint32_t TYPE, bool GATEUP, bool SPLIT>
 __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5Params p) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) uint8_t km_smem[];
-    __shared__ const float* s_x[8];
-    __shared__ float* s_out[8];
-    __shared__ float s_scale[8], s_inv[8];
-    __shared__ __align__(8) uint8_t s_wide[8];
+    __shared__ KmTile tl;
+    if (threadIdx.x == 0) { tl.row_bytes = p.row_bytes; tl.groups = p.cols / 32u; tl.lanes_per_row = p.lanes_per_row; tl.error = p.error; }   // read behind barriers
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t groups = p.cols / 32u, x_stride = p.cols * 2u + 64u;
     uint8_t* const xhi = km_smem;
@@ -359,19 +371,19 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
             top = __reduce_max_sync(0xffffffffu, top) >> 23;   // biased exponent of the largest magnitude
             if (lane == 0) {
                 const uint32_t e = top >= 255u ? 127u : min(268u - top, 253u);   // not finite: a wide row
-                s_wide[warp] = top >= 255u;
-                s_scale[warp] = __uint_as_float(e << 23); s_inv[warp] = __uint_as_float((254u - e) << 23);
-                s_x[warp] = x;
-                s_out[warp] = reinterpret_cast<float*>(reinterpret_cast<char*>(p.out) + static_cast<uint64_t>(rid) * p.out_stride_bytes);
+                tl.wide[warp] = top >= 255u;
+                tl.scale[warp] = __uint_as_float(e << 23); tl.inv[warp] = __uint_as_float((254u - e) << 23);
+                tl.x[warp] = x;
+                tl.out[warp] = reinterpret_cast<float*>(reinterpret_cast<char*>(p.out) + static_cast<uint64_t>(rid) * p.out_stride_bytes);
             }
-        } else if (lane == 0) s_wide[warp] = 0;
+        } else if (lane == 0) tl.wide[warp] = 0;
         __syncthreads();
         // stage: a thread takes the eight values that lane tq of a group multiplies, in the MMA's order
         for (uint32_t i = threadIdx.x; i < count * groups * 4u; i += kKmWarps * 32) {
             const uint32_t j = i / (groups * 4u), rem = i - j * groups * 4u, grp = rem >> 2, tq = rem & 3u;
-            const float4* src = reinterpret_cast<const float4*>(s_x[j] + grp * 32u);
+            const float4* src = reinterpret_cast<const float4*>(tl.x[j] + grp * 32u);
             const float4 f0 = src[TYPE == 13u ? 2 * tq : tq], f1 = src[TYPE == 13u ? 2 * tq + 1 : 4 + tq];
-            const float sc = s_scale[j];
+            const float sc = tl.scale[j];
             const float v[8] = {f0.x * sc, f0.z * sc, f0.y * sc, f0.w * sc, f1.x * sc, f1.z * sc, f1.y * sc, f1.w * sc};   // order 0,2,1,3
             uint32_t h[8], l[8];
             float sum = 0.f;
@@ -384,7 +396,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
                 l[q] = __half_as_ushort(__float2half_rn(v[q] - __half2float(hv)));
                 sum += v[q];
             }
-            if (most < kKmNarrow && most > 0.f) s_wide[j] = 1;
+            if (most < kKmNarrow && most > 0.f) tl.wide[j] = 1;
             uint8_t* dst = xhi + j * x_stride + grp * 64u + tq * 16u;
             *reinterpret_cast<uint4*>(dst) = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
             *reinterpret_cast<uint4*>(dst + (packed ? 4u : 8u) * x_stride) = make_uint4(l[0] | (l[1] << 16), l[2] | (l[3] << 16), l[4] | (l[5] << 16), l[6] | (l[7] << 16));
@@ -399,7 +411,7 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
         }
         __syncthreads();
         if (!live) continue;
-        const uint2 wide8 = *reinterpret_cast<const uint2*>(s_wide);
+        const uint2 wide8 = *reinterpret_cast<const uint2*>(tl.wide);
         const bool wide = (wide8.x | wide8.y) != 0;   // some row of the tile
         float total[4] = {0.f, 0.f, 0.f, 0.f}, low[4] = {0.f, 0.f, 0.f, 0.f};   // low: the low halves' sums of a tile that is not packed
         bool ok = true;
@@ -444,9 +456,9 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
 #pragma unroll
         for (uint32_t q = 0; q < 2; ++q) {
             const uint32_t j = 2 * t + q;
-            if (j >= count || (wide && s_wide[j])) continue;
-            const float inv = s_inv[j], va = total[q] * inv, vb = total[2 + q] * inv;
-            float* o = s_out[j] + r0 + g;
+            if (j >= count || (wide && tl.wide[j])) continue;
+            const float inv = tl.inv[j], va = total[q] * inv, vb = total[2 + q] * inv;
+            float* o = tl.out[j] + r0 + g;
             if (GATEUP) {
                 const float v = (va >= 0.f ? va / (1.f + expf(-va)) : va * expf(va) / (1.f + expf(va))) * vb;
                 if (!finite_f32(v)) raise_error(p.error, TSP_ERR_NONFINITE);
@@ -456,9 +468,8 @@ __global__ void __launch_bounds__(kKmWarps * 32, 2) gemv_k5_mma_kernel(const K5P
                 o[0] = va; o[8] = vb;
             }
         }
-        for (uint32_t j = 0; wide && j < count; ++j)   // uniform over the block
-            if (s_wide[j]) k5_wide_row<TYPE, GATEUP>(wA - static_cast<uint64_t>(g) * p.row_bytes, GATEUP ? wB - static_cast<uint64_t>(g) * p.row_bytes : wA - static_cast<uint64_t>(g) * p.row_bytes,
-                                                        p.row_bytes, RW, groups, p.lanes_per_row, s_x[j], s_out[j] + r0, p.error);
+        if (wide)   // uniform over the block
+            k5_wide_rows<TYPE, GATEUP>(&tl, wA - static_cast<uint64_t>(g) * p.row_bytes, (GATEUP ? wB : wA) - static_cast<uint64_t>(g) * p.row_bytes, count, r0);
     }
 }
 
