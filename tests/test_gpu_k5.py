@@ -256,3 +256,58 @@ def test_rows_do_not_depend_on_how_a_dense_launch_is_split(T):
     assert int(e.item()) == 0
     for o in outs[1:]:
         assert np.array_equal(o, outs[0][:, :o.shape[1]])
+
+
+# How the MMA kernel cuts its work: one warp per unit of rows (three steps of K), two, four and eight, two steps a warp (sixteen), rows whose
+# unit takes two copies (more than 256 lines), a unit count that the blocks do not share evenly. An FP32 sum of n terms: see the tile edges above.
+@pytest.mark.parametrize("type_,rows,cols", [(formats.Q5_K, 48, 768), (formats.Q5_K, 2400, 512), (formats.Q5_K, 32, 3072), (formats.Q5_1, 3008, 384), (formats.Q5_1, 48, 2944),
+                                             (formats.Q5_1, 32, 2048)])
+@pytest.mark.parametrize("gate_up", [False, True])
+def test_unit_geometry(oracle, type_, rows, cols, gate_up):
+    w = formats.quantize(type_, synth.normal(101, (rows, cols), 0.02)).reshape(-1)
+    t = dev(w)
+    ms = L.matrix_set(t, type_, formats.GGUF, rows, cols, 1)
+    x = synth.normal(102, (7, cols), 1.0)
+    w64 = oracle.dequantize(type_, w, rows * cols).astype(np.float64).reshape(rows, cols)
+    want = x.astype(np.float64) @ w64.T
+    bound = (cols + 8) * 2.0 ** -24 * 4 * np.abs(w64).max() * np.abs(x.astype(np.float64)).sum(axis=1)[:, None]
+    if gate_up:
+        want, bound = want / (1 + np.exp(-want)) * want, bound * (2 * np.abs(want) + 2)
+    dx, e = dev(x), torch.zeros(1, dtype=torch.int32, device=DEV)
+    for T in (7, 2):
+        out = torch.full((T, rows), np.nan, dtype=torch.float32, device=DEV)
+        if gate_up:
+            capi.call("tsp_moe_gate_up_swiglu", C.byref(ms), C.byref(ms), dx.data_ptr(), cols * 4, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        else:
+            capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, 1, T, 1, None, None, None, out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        assert np.all(np.abs(out.cpu().numpy() - want[:T]) <= bound[:T])
+    assert int(e.item()) == 0
+
+
+@pytest.mark.parametrize("tokens,experts,selected", [(1500, 512, 8), (2048, 4096, 32)])
+def test_many_tiles_per_block(oracle, tokens, experts, selected):
+    """Blocks that walk more tiles than their routing table holds (32), with the experts in two address ranges."""
+    rows, cols = 16, 128
+    rng = np.random.default_rng(7)
+    w = rng.integers(0, 256, (experts, rows * cols // 32 * 24), dtype=np.uint8)
+    w.reshape(experts, -1, 24)[:, :, 0:4] = np.array([0x00, 0x24, 0x00, 0xa4], dtype=np.uint8)   # d = 2^-6, m = -2^-6
+    t = dev(w.reshape(-1))
+    half = experts // 2
+    ms = L.matrix_set(t, formats.Q5_1, formats.GGUF, rows, cols, experts, base_hi=t.reshape(experts, -1)[half:].reshape(-1), split=half)
+    ids = np.argsort(rng.random((tokens, experts)), axis=1)[:, :selected].astype(np.int32)
+    x = synth.normal(103, (tokens, cols), 1.0)
+    dx, dids, e = dev(x), dev(ids), torch.zeros(1, dtype=torch.int32, device=DEV)
+    tmap, counts = torch.empty(experts * tokens, dtype=torch.int32, device=DEV), torch.empty(experts, dtype=torch.int32, device=DEV)
+    tasks = torch.empty(capi.lib().tsp_moe_tasks_words(tokens, experts, selected, 8), dtype=torch.int32, device=DEV)
+    out = torch.full((tokens * selected, rows), np.nan, dtype=torch.float32, device=DEV)
+    capi.call("tsp_moe_permute", dids.data_ptr(), tokens, experts, selected, 8, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(), e.data_ptr(), L.stream_ptr())
+    capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, selected, tokens, selected, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(),
+              out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+    torch.cuda.synchronize()
+    assert int(e.item()) == 0 and int(tasks[0]) > 32 * 16
+    w64 = oracle.dequantize(formats.Q5_1, w.reshape(-1), experts * rows * cols).astype(np.float64).reshape(experts, rows, cols)
+    want = np.einsum("tkrc,tc->tkr", w64[ids[::16]], x[::16].astype(np.float64))
+    got = out.cpu().numpy().reshape(tokens, selected, rows)[::16]
+    bound = (cols + 8) * 2.0 ** -24 * 4 * np.abs(w64).max() * np.abs(x[::16].astype(np.float64)).sum(axis=1)[:, None, None]
+    assert np.isfinite(out.cpu().numpy()).all() and np.all(np.abs(got - want) <= bound)
