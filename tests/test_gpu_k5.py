@@ -258,10 +258,12 @@ def test_rows_do_not_depend_on_how_a_dense_launch_is_split(T):
         assert np.array_equal(o, outs[0][:, :o.shape[1]])
 
 
-# How the MMA kernel cuts its work: one warp per unit of rows (three steps of K), two, four and eight, two steps a warp (sixteen), rows whose
+# How the MMA kernel cuts its work: two warps per unit of rows with uneven parts (three steps of K), two, four and eight, two steps a warp (sixteen), rows whose
 # unit takes two copies (more than 256 lines), a unit count that the blocks do not share evenly. An FP32 sum of n terms: see the tile edges above.
 @pytest.mark.parametrize("type_,rows,cols", [(formats.Q5_K, 48, 768), (formats.Q5_K, 2400, 512), (formats.Q5_K, 32, 3072), (formats.Q5_1, 3008, 384), (formats.Q5_1, 48, 2944),
-                                             (formats.Q5_1, 32, 2048)])
+                                             (formats.Q5_1, 32, 2048),
+                                             # enough units per block to go round the ring of stages: one, two and four warps per unit
+                                             (formats.Q5_K, 47360, 256), (formats.Q5_K, 28416, 768), (formats.Q5_1, 47360, 128), (formats.Q5_1, 47360, 640)])
 @pytest.mark.parametrize("gate_up", [False, True])
 def test_unit_geometry(oracle, type_, rows, cols, gate_up):
     w = formats.quantize(type_, synth.normal(101, (rows, cols), 0.02)).reshape(-1)

@@ -32,7 +32,7 @@ struct K5Params {
     const uint32_t* token_map; const uint32_t* counts; const uint32_t* tasks;
     uint32_t tokens, tile_tokens;
     // MMA kernel
-    uint32_t wpu;             // warps that share a unit, each with a part of its K extent (a power of two that divides the K steps)
+    uint32_t wpu;             // warps that share a unit, each with a part of its K extent (a power of two, no more than there are K steps)
     uint32_t slots;           // (unit, K part) sums of a batch that shared memory holds
     uint32_t copies, copy_lines, mat_bytes, stage_bytes, stages;   // a unit's matrix: copies of copy_lines lines, padded to mat_bytes; ring of stages
     uint32_t off_sx, off_red, off_stage;
@@ -219,7 +219,7 @@ constexpr uint32_t kKmWarps = 16, kKmThreads = (kKmWarps + 4) * 32;   // consume
 // kKmWarps * (kKmConsRegs - launch) <= 4 * (launch - kKmProdRegs) must hold for the count at launch (96). launch_km() checks the compiled kernel.
 constexpr int kKmConsRegs = 112, kKmProdRegs = 24;
 constexpr uint32_t kKmParts = 8;       // warps that share a unit at most
-constexpr uint32_t kKmStages = 8;      // units in flight at most
+constexpr uint32_t kKmStages = 16;     // units in flight at most
 constexpr uint32_t kKmTable = 32;      // tiles whose routing data a block keeps in shared memory
 struct alignas(64) K5Maps { CUtensorMap m[4]; };   // matrix A low ids, high ids, matrix B the same: [128 B][line][expert]
 
@@ -331,10 +331,10 @@ struct KmTile {
 };
 
 // Out of line: the rare path takes no registers from the loop above it. This warp's part of K of one unit for the wide rows of the tile, up to four
-// at a time, into their places of the unit's sums. linA, linB: the lane's rows' first bytes of that part; col0 its first column.
+// at a time, into their places of the unit's sums. linA, linB: the lane's rows' first bytes.
 template <uint32_t TYPE>
-__device__ __noinline__ void k5_wide_unit(const KmTile* tile, const uint8_t* mA, const uint8_t* mB, uint32_t linA, uint32_t linB, uint32_t col0, uint32_t steps,
-                                          uint32_t count, float* sums) {
+__device__ __noinline__ void k5_wide_unit(const KmTile* tile, const uint8_t* mA, const uint8_t* mB, uint32_t linA, uint32_t linB, uint32_t part, uint32_t wpu,
+                                          uint32_t steps, uint32_t count, float* sums) {
     using Step = KmStep<TYPE>;
     const uint32_t lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
     for (uint32_t j = 0; j < count;) {
@@ -342,7 +342,7 @@ __device__ __noinline__ void k5_wide_unit(const KmTile* tile, const uint8_t* mA,
         for (; j < count && n < 4; ++j) if (tile->wide[j]) list |= j << (4u * n++);
         if (!n) break;
         float acc[4][2] = {};
-        for (uint32_t st = 0; st < steps; ++st) {
+        for (uint32_t st = part; st < steps; st += wpu) {
             uint32_t at[Step::kLoads];
             Step a, b;
             Step::offsets(linA + st * Step::kBytes, t, at); a.load(mA, at);
@@ -363,7 +363,7 @@ __device__ __noinline__ void k5_wide_unit(const KmTile* tile, const uint8_t* mA,
 #pragma unroll
                 for (uint32_t k = 0; k < 4; ++k) {
                     if (k >= n) break;
-                    const float4* src = reinterpret_cast<const float4*>(tile->x[(list >> (4u * k)) & 15u] + col0 + (st * Step::kGroups + G) * 32u);
+                    const float4* src = reinterpret_cast<const float4*>(tile->x[(list >> (4u * k)) & 15u] + (st * Step::kGroups + G) * 32u);
                     const float4 x0 = src[TYPE == 13u ? 2 * t : t], x1 = src[TYPE == 13u ? 2 * t + 1 : 4 + t];
                     const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(kKmThreads, 1) gemv_k5_mma_kernel(const __grid
     uint8_t* const km = km_raw + ((1024u - (smem_u32(km_raw) & 1023u)) & 1023u);
     uint64_t* const full = reinterpret_cast<uint64_t*>(km);
     uint64_t* const empty = full + kKmStages;
-    uint32_t* const tt = reinterpret_cast<uint32_t*>(km + 128);             // [kKmTable + 1][12]: expert, first route, count, -, route ids; the last for a tile beyond
+    uint32_t* const tt = reinterpret_cast<uint32_t*>(km + 256);             // [kKmTable + 1][12]: expert, first route, count, -, route ids; the last for a tile beyond
     uint8_t* const xhi = km + 2048;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u, g = lane >> 2, t = lane & 3u;
     const uint32_t groups = p.cols / 32u, x_stride = p.cols * 2u + 64u;
@@ -478,13 +478,13 @@ __global__ void __launch_bounds__(kKmThreads, 1) gemv_k5_mma_kernel(const __grid
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kKmConsRegs));
     constexpr uint32_t CT = kKmWarps * 32;
     const uint32_t steps = groups / Step::kGroups, wpu = p.wpu, part = warp & (wpu - 1u), ngroups = kKmWarps / wpu;
-    const uint32_t my_steps = steps / wpu, batch = p.slots / wpu, st0 = part * my_steps;   // K steps st0 .. st0 + my_steps - 1
+    const uint32_t my_steps = (steps - part + wpu - 1u) / wpu, batch = p.slots / wpu;   // K steps part, part + wpu, ...
     uint32_t mine = warp / wpu;                  // this warp's next unit of the run
     uint32_t filled = 0;                         // units brought before this tile's
     bool ready = true;                           // no wait has expired
     uint32_t atA[Step::kLoads], atB[Step::kLoads];   // (gate-up: the same for both matrices)
-    Step::offsets(g * p.row_bytes + st0 * Step::kBytes, t, atA);
-    if (!GATEUP) Step::offsets((g + 8u) * p.row_bytes + st0 * Step::kBytes, t, atB);
+    Step::offsets(g * p.row_bytes + part * Step::kBytes, t, atA);
+    if (!GATEUP) Step::offsets((g + 8u) * p.row_bytes + part * Step::kBytes, t, atB);
     uint32_t tile = tile0, first = first0;
     for (uint32_t done = 0; done < units; ++tile, first = 0) {   // uniform over the block
         const uint32_t seg = done, row0 = first;
@@ -579,9 +579,10 @@ __global__ void __launch_bounds__(kKmThreads, 1) gemv_k5_mma_kernel(const __grid
                 auto work = [&](auto packed_tile) {   // two copies: as a run-time choice the second pass was predicated and issued all the same
                     constexpr bool PACKED = decltype(packed_tile)::value != 0;
                     for (uint32_t st = 0; st < my_steps; ++st) {
+                        const uint32_t step = part + st * wpu;
                         if (my_steps > 1) {
-                            Step::offsets(g * p.row_bytes + (st0 + st) * Step::kBytes, t, atA);
-                            if (!GATEUP) Step::offsets((g + 8u) * p.row_bytes + (st0 + st) * Step::kBytes, t, atB);
+                            Step::offsets(g * p.row_bytes + step * Step::kBytes, t, atA);
+                            if (!GATEUP) Step::offsets((g + 8u) * p.row_bytes + step * Step::kBytes, t, atB);
                         }
                         Step a, b;
                         a.load(mA, atA); b.load(mB, GATEUP ? atA : atB);
@@ -592,7 +593,7 @@ __global__ void __launch_bounds__(kKmThreads, 1) gemv_k5_mma_kernel(const __grid
                             uint32_t ca[4], cb[4];
                             float fa, ma, fb, mb, acc[4];
                             a.template get<G>(t, ca, fa, ma); b.template get<G>(t, cb, fb, mb);
-                            const uint32_t grp = (st0 + st) * Step::kGroups + G;
+                            const uint32_t grp = step * Step::kGroups + G;
                             k5_group_mma(acc, ca, cb, xh + grp * 64u);
                             if (!PACKED) {
                                 float al[4];
@@ -617,8 +618,7 @@ __global__ void __launch_bounds__(kKmThreads, 1) gemv_k5_mma_kernel(const __grid
                 float4* const sums = red + ((mine - b0) * wpu + part) * 32u;
                 sums[lane] = make_float4(total[0], total[1], total[2], total[3]);
                 if (wide)   // uniform over the block
-                    k5_wide_unit<TYPE>(&tl, mA, mB, g * p.row_bytes + st0 * Step::kBytes, (GATEUP ? g : g + 8u) * p.row_bytes + st0 * Step::kBytes,
-                                       st0 * Step::kGroups * 32u, my_steps, count, reinterpret_cast<float*>(sums));
+                    k5_wide_unit<TYPE>(&tl, mA, mB, g * p.row_bytes, (GATEUP ? g : g + 8u) * p.row_bytes, part, wpu, steps, count, reinterpret_cast<float*>(sums));
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&empty[stage]);
                 stage += ngroups;
@@ -732,7 +732,7 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     const uint32_t dense_tiles = (tokens + p.tile_tokens - 1) / p.tile_tokens, rw = gateup ? 8u : 16u;
     const uint32_t km_groups = a->type == TSP_TYPE_Q5_K ? 8u : 4u;
     if (nc == 1 && a->rows % rw == 0 && groups % km_groups == 0 && a->cols <= 3328) {
-        for (p.wpu = 1; p.wpu < kKmParts && groups / km_groups % (2u * p.wpu) == 0;) p.wpu *= 2;
+        for (p.wpu = 1; p.wpu < kKmParts && groups / km_groups >= 2u * p.wpu;) p.wpu *= 2;
         const uint32_t lines = rw * p.row_bytes / 128u;   // whole: eight rows of 176 or 96 bytes a step
         p.copies = (lines + 255u) / 256u;                 // a box holds 256 lines at most; 16 rows are an even number of lines
         p.copy_lines = lines / p.copies;
@@ -741,10 +741,13 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
         const uint32_t budget = 225 * 1024;               // of the 227 KB, the static tile record and the alignment of the base taken off
         p.off_sx = 2048u + 16u * (a->cols * 2u + 64u);
         p.off_red = p.off_sx + groups * 32u;
-        for (p.slots = 128; p.slots > kKmParts && p.off_red + p.slots * 512u + 4u * p.stage_bytes > budget;) p.slots /= 2;   // four units in flight before long batches
+        for (p.slots = 128; p.slots > kKmParts && p.off_red + p.slots * 512u + (kKmWarps / p.wpu > 4u ? kKmWarps / p.wpu : 4u) * p.stage_bytes > budget;) p.slots /= 2;   // units in flight before long batches
         p.off_stage = (p.off_red + p.slots * 512u + 1023u) & ~1023u;
+        // The warps that share a unit take every unit_groups-th one. A whole number of such rounds in the ring: the unit that had a unit's stage before
+        // it was then read by the same warps, so that a wait is never a phase of the barrier too early.
+        const uint32_t unit_groups = kKmWarps / p.wpu;
         p.stages = (budget - p.off_stage) / p.stage_bytes;
-        if (p.stages > kKmStages) p.stages = kKmStages;
+        p.stages = (p.stages < kKmStages ? p.stages : kKmStages) / unit_groups * unit_groups;
         if (p.copies * p.copy_lines != lines || p.stages < 2) return fail(TSP_E_ARG, "five-bit projection: no room for the weight rows in shared memory");
         K5Maps maps;
         const uint32_t n_lo = p.split ? p.split : 1u, n_hi = p.experts > p.split ? p.experts - p.split : 1u;
