@@ -6,6 +6,7 @@
 #include <cstdio>
 
 #include "tsp_common.cuh"
+#include "tsp_q8_rows.cuh"
 
 namespace tsp {
 
@@ -43,7 +44,7 @@ int launch_permute(const uint32_t*, uint32_t, uint32_t, uint32_t, uint32_t, uint
 int launch_combine(const void*, uint64_t, uint32_t, const float*, const float*, uint64_t, const float*, const void*, uint64_t, uint32_t, float*,
                    uint32_t, uint32_t, uint32_t, float*, uint64_t, void*, uint64_t, uint32_t*, cudaStream_t);
 int launch_decode_prologue(const float*, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t, uint32_t*, float*, uint32_t*, uint32_t*,
-                           uint32_t*, const void*, uint64_t, float*, uint64_t, uint32_t, uint32_t*, cudaStream_t);
+                           uint32_t*, const void*, uint64_t, float*, uint64_t, uint32_t, DecodeDense*, uint32_t*, cudaStream_t);
 int launch_f16_to_f32(const void*, uint64_t, float*, uint64_t, uint32_t, uint32_t, cudaStream_t);
 int launch_dequant(uint32_t, uint32_t, const uint8_t*, uint64_t, float*, uint32_t*, cudaStream_t);
 int launch_gemv(const tsp_matrix_set*, const tsp_matrix_set*, bool, const float*, uint64_t, uint32_t, uint32_t,
@@ -468,22 +469,40 @@ int tsp_moe_layer_decode(const tsp_moe_weights* w, const tsp_moe_scratch* s, con
     uint64_t x32_stride = x_stride;
     if (x_dtype == 1) { x32 = s->d_x32; x32_stride = channels * 4ull; }
     const int exact = x_dtype == 1;
-    // small batches: route, permutation, tile table and the binary16 -> FP32 copy of the rows in ONE launch
+    // A dense Q8_0 shared expert that cannot ride in the routed launches (they take one of their own encoding, Q4_K) rides in the prologue's: all-Q8_0
+    // layer of five rows 83 -> 73 us, five-bit layer of 13 rows 157 -> 137 us. What its own launches would refuse goes to them.
+    DecodeDense dense{static_cast<const uint8_t*>(w->shared_gate.base), static_cast<const uint8_t*>(w->shared_up.base), static_cast<const uint8_t*>(w->shared_down.base),
+                      hidden, channels, d_x, x_stride, s->d_shared_hidden, s->d_shared_out, d_error};
+    const uint64_t x_bytes = tokens * x_stride, h_bytes = tokens * hidden * 4ull, o_bytes = tokens * channels * 4ull;
+    auto plain_q8 = [](const tsp_matrix_set& m) { return m.type == TSP_TYPE_Q8_0 && m.layout == TSP_LAYOUT_GGUF && m.experts == 1 && m.split >= 1; };
+    const bool dense_ok = plain_q8(w->shared_gate) && plain_q8(w->shared_up) && plain_q8(w->shared_down) && check_matrix(&w->shared_gate, "gate") == TSP_OK &&
+                          check_matrix(&w->shared_up, "up") == TSP_OK && check_matrix(&w->shared_down, "project") == TSP_OK && w->shared_up.rows == hidden &&
+                          w->shared_up.cols == channels && w->shared_gate.expert_stride == w->shared_up.expert_stride && w->shared_gate.split == w->shared_up.split &&
+                          channels % 16 == 0 && aligned16(s->d_shared_hidden) && aligned16(s->d_shared_out) && !overlap(d_x, x_bytes, s->d_shared_hidden, h_bytes) &&
+                          (!s->d_x32 || !overlap(s->d_x32, o_bytes, s->d_shared_hidden, h_bytes)) && !overlap(s->d_shared_hidden, h_bytes, s->d_shared_out, o_bytes);
+    // small batches: route, permutation, tile table and the binary16 -> FP32 copy of the rows in two launches
     int fused = launch_decode_prologue(d_logits, logits_stride, tokens, experts, selected, mode, normalize, TSP_GEMV_TILE, s->d_ids, s->d_weights,
                                        s->d_token_map, s->d_counts, s->d_tasks, x_dtype == 1 ? d_x : nullptr, x_stride, s->d_x32, channels * 4ull,
-                                       channels, d_error, st);
+                                       channels, dense_ok ? &dense : nullptr, d_error, st);
     if (fused < 0) return fused;
     if (fused == 1) {
         if (x_dtype == 1) { if (int rc = tsp_rows_f16_to_f32(d_x, x_stride, s->d_x32, channels * 4ull, tokens, channels, st)) return rc; }
         if (int rc = tsp_moe_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_error, st)) return rc;
         if (int rc = tsp_moe_permute(s->d_ids, tokens, experts, selected, TSP_GEMV_TILE, s->d_token_map, s->d_counts, s->d_tasks, d_error, st)) return rc;
     }
-    if (int rc = tsp_moe_gate_up_swiglu_shared(&w->gate, &w->up, &w->shared_gate, &w->shared_up, x32, x32_stride, x_dtype == 1 ? d_x : nullptr,
-                                               x_dtype == 1 ? x_stride : 0, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden,
-                                               hidden * 4ull, s->d_shared_hidden, hidden * 4ull, exact, d_error, stream)) return rc;
-    if (int rc = tsp_moe_project_shared(&w->down, &w->shared_down, s->d_hidden, hidden * 4ull, s->d_shared_hidden, hidden * 4ull, tokens, selected,
-                                        s->d_token_map, s->d_counts, s->d_tasks, s->d_routed, channels * 4ull, s->d_shared_out, channels * 4ull,
-                                        d_error, stream)) return rc;
+    if (dense.done) {
+        if (int rc = tsp_moe_gate_up_swiglu(&w->gate, &w->up, x32, x32_stride, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden, hidden * 4ull,
+                                            exact, d_error, stream)) return rc;
+        if (int rc = tsp_moe_project(&w->down, s->d_hidden, hidden * 4ull, 1, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_routed, channels * 4ull, 0,
+                                     d_error, stream)) return rc;
+    } else {
+        if (int rc = tsp_moe_gate_up_swiglu_shared(&w->gate, &w->up, &w->shared_gate, &w->shared_up, x32, x32_stride, x_dtype == 1 ? d_x : nullptr,
+                                                   x_dtype == 1 ? x_stride : 0, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden,
+                                                   hidden * 4ull, s->d_shared_hidden, hidden * 4ull, exact, d_error, stream)) return rc;
+        if (int rc = tsp_moe_project_shared(&w->down, &w->shared_down, s->d_hidden, hidden * 4ull, s->d_shared_hidden, hidden * 4ull, tokens, selected,
+                                            s->d_token_map, s->d_counts, s->d_tasks, s->d_routed, channels * 4ull, s->d_shared_out, channels * 4ull,
+                                            d_error, stream)) return rc;
+    }
     // binary16 output rows are written straight from the FP32 mixture; no FP32 copy of the output is kept
     return tsp_moe_combine(s->d_routed, channels * 4ull, 0, s->d_weights, s->d_shared_out, channels * 4ull, w->d_shared_router, x32,
                            x32_stride, 0, s->d_shared_logit, tokens, channels, selected,

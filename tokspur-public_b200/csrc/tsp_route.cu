@@ -2,6 +2,7 @@
 // All integer results (ids, token_map, counts, tasks) are deterministic and independent of
 // scheduling: no atomics decide an order anywhere.
 #include "tsp_common.cuh"
+#include "tsp_q8_rows.cuh"
 
 namespace tsp {
 
@@ -313,16 +314,24 @@ constexpr int kPrologueThreads = 1024;
 constexpr int kPrologueRouteWarps = 4;
 constexpr uint32_t kPrologueTokens = 1024, kPrologueExperts = 1024;
 
-__global__ void __launch_bounds__(kPrologueRouteWarps * 32)
+// DENSE: 0 no dense expert; 1, 2: blocks past the conversion blocks work on the gate / up pair of a dense Q8_0 expert, from FP32 / binary16 rows
+constexpr uint32_t kRouteDenseWarps = 8, kTablesDenseWarps = 16;
+
+template <int DENSE>
+__global__ void __launch_bounds__(DENSE ? kRouteDenseWarps * 32 : kPrologueRouteWarps * 32)
 decode_route_kernel(const float* logits, uint64_t logits_stride, uint32_t tokens, uint32_t experts, uint32_t selected,
-                    uint32_t mode, int normalize, uint32_t route_blocks, uint32_t* __restrict__ ids, float* __restrict__ weights,
+                    uint32_t mode, int normalize, uint32_t route_blocks, uint32_t nconv, uint32_t* __restrict__ ids, float* __restrict__ weights,
                     const __half* x16, uint64_t x16_stride, float* __restrict__ x32, uint64_t x32_stride, uint32_t channels,
-                    uint32_t* error) {
+                    const Q8Rows dense, uint32_t* error) {
     pdl_launch_dependents();
+    extern __shared__ __align__(16) float pro_smem[];          // [warps][experts] routing rows of the shared-memory form; the dense blocks' weights
     pdl_wait();
+    if (DENSE && blockIdx.x >= route_blocks + nconv) {
+        q8_rows_block<true, DENSE == 2, kRouteDenseWarps>(dense, blockIdx.x - route_blocks - nconv, reinterpret_cast<uint8_t*>(pro_smem));
+        return;
+    }
     if (blockIdx.x >= route_blocks) {   // the conversion blocks: binary16 rows -> FP32 rows (exact)
         const uint32_t per_row = channels / 4;   // four values per thread step
-        const uint32_t nconv = gridDim.x - route_blocks;
         for (uint32_t i = (blockIdx.x - route_blocks) * blockDim.x + threadIdx.x; i < tokens * per_row; i += nconv * blockDim.x) {
             const uint32_t row = i / per_row, c4 = i - row * per_row;
             const uint2 h = *reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(x16) + row * x16_stride + c4 * 8ull);
@@ -331,10 +340,9 @@ decode_route_kernel(const float* logits, uint64_t logits_stride, uint32_t tokens
         }
         return;
     }
-    extern __shared__ float pro_smem[];          // [warps][experts] routing rows of the shared-memory form
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t t = blockIdx.x * kPrologueRouteWarps + warp;
-    if (t >= tokens) return;
+    if ((DENSE && warp >= kPrologueRouteWarps) || t >= tokens) return;
     const float* row = reinterpret_cast<const float*>(reinterpret_cast<const char*>(logits) + t * logits_stride);
     if (experts <= 512 && normalize) route_row_regs(row, t, experts, selected, mode, ids, weights, error, lane);
     else route_row(pro_smem + warp * experts, row, t, experts, selected, mode, normalize, ids, weights, error, lane);
@@ -343,13 +351,20 @@ decode_route_kernel(const float* logits, uint64_t logits_stride, uint32_t tokens
 // Permutation + tile table of up to 1024 token rows in ONE block: a mask of the rows that name each expert (`words` 32-bit words per
 // expert in shared memory), positions = number of lower set bits. ids are global; this launch owns experts [first, first + experts);
 // with local_only, routes to other owners are skipped, without it they are an index error.
-__global__ void __launch_bounds__(kPrologueThreads)
+// DENSE: blocks 1 .. work on the down matrix of a dense Q8_0 expert (512 threads; up to 512 experts, one per thread).
+template <bool DENSE>
+__global__ void __launch_bounds__(DENSE ? kTablesDenseWarps * 32 : kPrologueThreads)
 tables_kernel(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
-              uint32_t words, uint32_t* __restrict__ token_map, uint32_t* __restrict__ counts, uint32_t* __restrict__ tasks, uint32_t* error) {
+              uint32_t words, uint32_t* __restrict__ token_map, uint32_t* __restrict__ counts, uint32_t* __restrict__ tasks, const Q8Rows dense, uint32_t* error) {
     pdl_launch_dependents();
     // [experts][stride] masks (an odd stride: lanes with different experts and one word index hit different banks), then [experts][stride]
     // running counts of the words before each word. (With a stride of 32 words and a walk over the words per route, 1003 rows took 100 us; 14 us now.)
-    extern __shared__ uint32_t tables_mask[];
+    extern __shared__ __align__(16) uint32_t tables_mask[];
+    if (DENSE && blockIdx.x > 0) {
+        pdl_wait();
+        q8_rows_block<false, false, kTablesDenseWarps>(dense, blockIdx.x - 1, reinterpret_cast<uint8_t*>(tables_mask));
+        return;
+    }
     const uint32_t stride = words | 1u;
     uint16_t* const before_word = reinterpret_cast<uint16_t*>(tables_mask + experts * stride);
     __shared__ uint32_t warp_tiles[32], warp_routes[32];
@@ -408,32 +423,73 @@ static bool tables_fit(uint32_t tokens, uint32_t experts) {
     return tokens >= 1 && tokens <= 1024 && experts <= static_cast<uint32_t>(kPrologueThreads) && static_cast<uint64_t>(experts) * ((tokens + 31) / 32) * 4 <= 96 * 1024;
 }
 static int launch_tables(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
-                         uint32_t* token_map, uint32_t* counts, uint32_t* tasks, uint32_t* error, cudaStream_t st) {
+                         uint32_t* token_map, uint32_t* counts, uint32_t* tasks, uint32_t* error, cudaStream_t st, const Q8Rows* dense = nullptr) {
     const uint32_t words = (tokens + 31) / 32;
-    const size_t smem = static_cast<size_t>(experts) * (words | 1u) * 6;
+    const size_t tables = static_cast<size_t>(experts) * (words | 1u) * 6;
+    if (dense) {
+        const size_t smem = tables > q8_rows_smem(kTablesDenseWarps) ? tables : q8_rows_smem(kTablesDenseWarps);
+        static thread_local SmemAttrCache configured;
+        TSP_CUDA(ensure_dynamic_smem(tables_kernel<true>, configured, smem));
+        TSP_CUDA(launch_pdl(tables_kernel<true>, dim3(1 + dense->blocks), dim3(kTablesDenseWarps * 32), smem, st, ids, tokens, experts, selected, tile, first, local_only,
+                            words, token_map, counts, tasks, *dense, error));
+        return TSP_OK;
+    }
     static thread_local SmemAttrCache configured;
-    TSP_CUDA(ensure_dynamic_smem(tables_kernel, configured, smem));
-    TSP_CUDA(launch_pdl(tables_kernel, dim3(1), dim3(kPrologueThreads), smem, st, ids, tokens, experts, selected, tile, first, local_only, words, token_map, counts,
-                        tasks, error));
+    TSP_CUDA(ensure_dynamic_smem(tables_kernel<false>, configured, tables));
+    TSP_CUDA(launch_pdl(tables_kernel<false>, dim3(1), dim3(kPrologueThreads), tables, st, ids, tokens, experts, selected, tile, first, local_only, words, token_map, counts,
+                        tasks, Q8Rows{}, error));
     return TSP_OK;
 }
 
-// Returns 1 when the batch does not fit the short prologue (the caller then issues the separate launches).
+// The dense Q8_0 expert of a decode batch in the prologue's launches (gate-up beside the routing, down beside the tables): its geometry, or false
+// where the launches do not serve it. The limits: 128 token rows (its matrices are read once per eight rows, in launches of its own once per sixteen:
+// Q8_0 layer of 64 / 128 / 192 / 256 rows 287 / 368 / 403 / 438 us, with launches of its own 307 / 376 / 407 / 437) and 512 experts (the tables' block has
+// 512 threads then).
+constexpr uint32_t kDenseTokens = 128;
+static bool plan_dense(DecodeDense& d, uint32_t tokens, uint32_t experts, bool x16) {
+    const bool ok = tokens <= kDenseTokens && experts <= kTablesDenseWarps * 32 && d.hidden % 256 == 0 && d.channels % 256 == 0 && aligned16(d.x) && d.x_stride % 16 == 0;
+    if (!ok) return false;
+    d.x16 = x16;
+    d.up = Q8Rows{d.gate_w, d.up_w, d.hidden, d.channels, d.channels / 32 * 34, d.x, d.x_stride, d.h, d.hidden * 4ull, tokens, 1, 0, d.error};
+    d.down = Q8Rows{d.down_w, nullptr, d.channels, d.hidden, d.hidden / 32 * 34, d.h, d.hidden * 4ull, d.out, d.channels * 4ull, tokens, 1, 0, d.error};
+    q8_rows_plan(d.up, true, kRouteDenseWarps);
+    q8_rows_plan(d.down, false, kTablesDenseWarps);
+    return true;
+}
+
+template <int DENSE>
+static int launch_decode_route(dim3 grid, size_t smem, cudaStream_t st, const float* logits, uint64_t logits_stride, uint32_t tokens, uint32_t experts, uint32_t selected,
+                               uint32_t mode, int normalize, uint32_t route_blocks, uint32_t conv, uint32_t* ids, float* weights, const void* x16, uint64_t x16_stride,
+                               float* x32, uint64_t x32_stride, uint32_t channels, const Q8Rows& dense, uint32_t* error) {
+    if (DENSE && smem < q8_rows_smem(kRouteDenseWarps)) smem = q8_rows_smem(kRouteDenseWarps);
+    static thread_local SmemAttrCache configured;   // per kernel instantiation, keyed by device
+    TSP_CUDA(ensure_dynamic_smem(decode_route_kernel<DENSE>, configured, smem));
+    TSP_CUDA(launch_pdl(decode_route_kernel<DENSE>, grid, dim3(DENSE ? kRouteDenseWarps * 32 : kPrologueRouteWarps * 32), smem, st, logits, logits_stride, tokens, experts,
+                        selected, mode, normalize, route_blocks, conv, ids, weights, static_cast<const __half*>(x16), x16_stride, x32, x32_stride, channels, dense, error));
+    return TSP_OK;
+}
+
+// Returns 1 when the batch does not fit the short prologue (the caller then issues the separate launches). dense: a Q8_0 shared expert for these
+// launches to work on; dense->done says whether they do.
 int launch_decode_prologue(const float* logits, uint64_t logits_stride, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t mode,
                            int normalize, uint32_t tile, uint32_t* ids, float* weights, uint32_t* token_map, uint32_t* counts, uint32_t* tasks,
-                           const void* x16, uint64_t x16_stride, float* x32, uint64_t x32_stride, uint32_t channels, uint32_t* error, cudaStream_t st) {
+                           const void* x16, uint64_t x16_stride, float* x32, uint64_t x32_stride, uint32_t channels, DecodeDense* dense, uint32_t* error, cudaStream_t st) {
     if (tokens > kPrologueTokens || experts > kPrologueExperts || !tables_fit(tokens, experts)) return 1;
     if (x16 && (channels % 4 || x16_stride % 8 || x32_stride % 16 || reinterpret_cast<uintptr_t>(x16) % 8 || reinterpret_cast<uintptr_t>(x32) % 16)) return 1;
     const size_t smem = (experts <= 512 && normalize) ? 0 : static_cast<size_t>(kPrologueRouteWarps) * experts * sizeof(float);
-    static thread_local SmemAttrCache configured;
-    TSP_CUDA(ensure_dynamic_smem(decode_route_kernel, configured, smem));
     const uint32_t route_blocks = (tokens + kPrologueRouteWarps - 1) / kPrologueRouteWarps;
     // conversion blocks: enough to cover the rows in two passes
     const uint32_t conv = x16 ? min(128u, (tokens * (channels / 4) + 2 * kPrologueRouteWarps * 32 - 1) / (2 * kPrologueRouteWarps * 32)) : 0u;
-    TSP_CUDA(launch_pdl(decode_route_kernel, dim3(route_blocks + conv), dim3(kPrologueRouteWarps * 32), smem, st, logits, logits_stride, tokens, experts,
-                        selected, mode, normalize, route_blocks, ids, weights, static_cast<const __half*>(x16), x16_stride, x32, x32_stride, channels, error));
-    if (int rc = launch_tables(ids, tokens, experts, selected, tile, 0, 0, token_map, counts, tasks, error, st)) return rc;
+    const int form = dense && plan_dense(*dense, tokens, experts, x16 != nullptr) ? (x16 ? 2 : 1) : 0;
+    const Q8Rows up = form ? dense->up : Q8Rows{};
+    const dim3 grid(route_blocks + conv + up.blocks);
+#define TSP_ROUTE(D) launch_decode_route<D>(grid, smem, st, logits, logits_stride, tokens, experts, selected, mode, normalize, route_blocks, conv, ids, weights, x16, \
+                                            x16_stride, x32, x32_stride, channels, up, error)
+    if (int rc = form == 2 ? TSP_ROUTE(2) : form == 1 ? TSP_ROUTE(1) : TSP_ROUTE(0)) return rc;
+#undef TSP_ROUTE
+    if (int rc = launch_tables(ids, tokens, experts, selected, tile, 0, 0, token_map, counts, tasks, error, st, form ? &dense->down : nullptr)) return rc;
     TSP_CUDA(cudaGetLastError());
+    if (dense) dense->done = form != 0;
     return TSP_OK;
 }
 
