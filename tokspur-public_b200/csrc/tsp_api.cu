@@ -371,17 +371,15 @@ int tsp_rows_f16_to_f32(const void* d_in, uint64_t in_stride, float* d_out, uint
     return launch_f16_to_f32(d_in, in_stride, d_out, out_stride, rows, cols, static_cast<cudaStream_t>(stream));
 }
 
-// Routed experts and the layer's dense shared expert in one launch when the shared expert looks like a routed one (same
-// shape, encoding and layout, Q4_K); otherwise the shared expert gets a launch of its own.
-int tsp_moe_gate_up_swiglu_shared_rows(const tsp_matrix_set* gate, const tsp_matrix_set* up, const tsp_matrix_set* shared_gate,
-                                       const tsp_matrix_set* shared_up, const float* d_x, uint64_t x_stride, const void* d_x16,
-                                       uint64_t x16_stride, uint32_t tokens, uint32_t selected, const uint32_t* d_token_map,
-                                       const uint32_t* d_counts, const uint32_t* d_tasks, float* d_h, uint64_t h_stride,
-                                       const float* d_shared_x, uint64_t shared_x_stride, uint32_t shared_tokens, float* d_shared_h,
-                                       uint64_t shared_h_stride, int x_is_f16_exact, uint32_t* d_error, void* stream) {
-    TSP_REQUIRE(gate && up && shared_gate && shared_up && d_token_map && d_counts && d_tasks && d_shared_h && d_shared_x && shared_tokens >= 1,
-                "gate-up with shared expert: null argument");
-    TSP_REQUIRE(!d_x16 || (d_shared_x == d_x && shared_tokens == tokens), "gate-up with shared expert: binary16 rows serve both row sets only when they are the same rows");
+}  // extern "C"
+
+// The routed experts and a dense expert of their shape, encoding and layout in one gate-up launch, which routes its own batch where `route` is given.
+// 1: not for this launch.
+static int gate_up_shared_launch(const tsp_matrix_set* gate, const tsp_matrix_set* up, const tsp_matrix_set* shared_gate, const tsp_matrix_set* shared_up,
+                                 const float* d_x, uint64_t x_stride, const void* d_x16, uint64_t x16_stride, uint32_t tokens, uint32_t selected,
+                                 const uint32_t* d_token_map, const uint32_t* d_counts, const uint32_t* d_tasks, float* d_h, uint64_t h_stride,
+                                 const float* d_shared_x, uint64_t shared_x_stride, uint32_t shared_tokens, float* d_shared_h, uint64_t shared_h_stride,
+                                 int x_is_f16_exact, uint32_t* d_error, void* stream, const GemvRoute* route) {
     const bool same_shape = shared_gate->type == gate->type && shared_gate->layout == gate->layout && shared_up->type == gate->type &&
                             shared_up->layout == gate->layout && shared_gate->rows == gate->rows && shared_gate->cols == gate->cols &&
                             shared_up->rows == gate->rows && shared_up->cols == gate->cols && shared_gate->experts == 1 && shared_up->experts == 1;
@@ -397,10 +395,29 @@ int tsp_moe_gate_up_swiglu_shared_rows(const tsp_matrix_set* gate, const tsp_mat
         GemvShared sh{shared_gate, shared_up, d_shared_x, shared_x_stride, d_shared_h, shared_h_stride};
         sh.tokens = shared_tokens;
         if (d_x16 && x_is_f16_exact) { sh.x16 = d_x16; sh.x16_stride_bytes = x16_stride; }   // the binary16 rows themselves: staged without conversion
-        const int rc = launch_gemv(gate, up, true, d_x, x_stride, selected, tokens, d_token_map, d_counts, d_tasks, d_h, h_stride,
-                                   x_is_f16_exact, 1, d_error, static_cast<cudaStream_t>(stream), &sh);
-        if (rc <= 0) return rc;
+        sh.route = route;
+        return launch_gemv(gate, up, true, d_x, x_stride, selected, tokens, d_token_map, d_counts, d_tasks, d_h, h_stride, x_is_f16_exact, 1, d_error,
+                           static_cast<cudaStream_t>(stream), &sh);
     }
+    return 1;
+}
+
+extern "C" {
+
+// Routed experts and the layer's dense shared expert in one launch when the shared expert looks like a routed one (same
+// shape, encoding and layout, Q4_K); otherwise the shared expert gets a launch of its own.
+int tsp_moe_gate_up_swiglu_shared_rows(const tsp_matrix_set* gate, const tsp_matrix_set* up, const tsp_matrix_set* shared_gate,
+                                       const tsp_matrix_set* shared_up, const float* d_x, uint64_t x_stride, const void* d_x16,
+                                       uint64_t x16_stride, uint32_t tokens, uint32_t selected, const uint32_t* d_token_map,
+                                       const uint32_t* d_counts, const uint32_t* d_tasks, float* d_h, uint64_t h_stride,
+                                       const float* d_shared_x, uint64_t shared_x_stride, uint32_t shared_tokens, float* d_shared_h,
+                                       uint64_t shared_h_stride, int x_is_f16_exact, uint32_t* d_error, void* stream) {
+    TSP_REQUIRE(gate && up && shared_gate && shared_up && d_token_map && d_counts && d_tasks && d_shared_h && d_shared_x && shared_tokens >= 1,
+                "gate-up with shared expert: null argument");
+    TSP_REQUIRE(!d_x16 || (d_shared_x == d_x && shared_tokens == tokens), "gate-up with shared expert: binary16 rows serve both row sets only when they are the same rows");
+    if (const int rc = gate_up_shared_launch(gate, up, shared_gate, shared_up, d_x, x_stride, d_x16, x16_stride, tokens, selected, d_token_map, d_counts, d_tasks, d_h,
+                                             h_stride, d_shared_x, shared_x_stride, shared_tokens, d_shared_h, shared_h_stride, x_is_f16_exact, d_error, stream, nullptr);
+        rc <= 0) return rc;
     if (int rc = tsp_moe_gate_up_swiglu(gate, up, d_x, x_stride, tokens, selected, d_token_map, d_counts, d_tasks, d_h, h_stride, x_is_f16_exact,
                                         d_error, stream)) return rc;
     return tsp_moe_gate_up_swiglu(shared_gate, shared_up, d_shared_x, shared_x_stride, shared_tokens, 1, nullptr, nullptr, nullptr, d_shared_h, shared_h_stride,
@@ -480,12 +497,23 @@ int tsp_moe_layer_decode(const tsp_moe_weights* w, const tsp_moe_scratch* s, con
                           w->shared_up.cols == channels && w->shared_gate.expert_stride == w->shared_up.expert_stride && w->shared_gate.split == w->shared_up.split &&
                           channels % 16 == 0 && aligned16(s->d_shared_hidden) && aligned16(s->d_shared_out) && !overlap(d_x, x_bytes, s->d_shared_hidden, h_bytes) &&
                           (!s->d_x32 || !overlap(s->d_x32, o_bytes, s->d_shared_hidden, h_bytes)) && !overlap(s->d_shared_hidden, h_bytes, s->d_shared_out, o_bytes);
+    // up to eight rows on Q4_K experts: the gate-up launch routes the batch itself (binary16 rows are then read as they are)
+    int fused = 1;
+    bool gated = false;
+    if (tokens <= TSP_GEMV_TILE && experts <= 512 && normalize && w->gate.type == TSP_TYPE_Q4_K) {
+        const GemvRoute route{d_logits, logits_stride, selected, mode, s->d_ids, s->d_weights, s->d_token_map, s->d_counts, s->d_tasks};
+        const int rc = gate_up_shared_launch(&w->gate, &w->up, &w->shared_gate, &w->shared_up, x_dtype == 1 ? s->d_x32 : x32, x32_stride, x_dtype == 1 ? d_x : nullptr,
+                                             x_dtype == 1 ? x_stride : 0, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden, hidden * 4ull,
+                                             x_dtype == 1 ? s->d_x32 : x32, x32_stride, tokens, s->d_shared_hidden, hidden * 4ull, exact, d_error, stream, &route);
+        if (rc < 0) return rc;
+        gated = rc == 0;
+    }
     // small batches: route, permutation, tile table and the binary16 -> FP32 copy of the rows in two launches
-    int fused = launch_decode_prologue(d_logits, logits_stride, tokens, experts, selected, mode, normalize, TSP_GEMV_TILE, s->d_ids, s->d_weights,
+    if (!gated) fused = launch_decode_prologue(d_logits, logits_stride, tokens, experts, selected, mode, normalize, TSP_GEMV_TILE, s->d_ids, s->d_weights,
                                        s->d_token_map, s->d_counts, s->d_tasks, x_dtype == 1 ? d_x : nullptr, x_stride, s->d_x32, channels * 4ull,
                                        channels, dense_ok ? &dense : nullptr, d_error, st);
     if (fused < 0) return fused;
-    if (fused == 1) {
+    if (!gated && fused == 1) {
         if (x_dtype == 1) { if (int rc = tsp_rows_f16_to_f32(d_x, x_stride, s->d_x32, channels * 4ull, tokens, channels, st)) return rc; }
         if (int rc = tsp_moe_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_error, st)) return rc;
         if (int rc = tsp_moe_permute(s->d_ids, tokens, experts, selected, TSP_GEMV_TILE, s->d_token_map, s->d_counts, s->d_tasks, d_error, st)) return rc;
@@ -496,16 +524,17 @@ int tsp_moe_layer_decode(const tsp_moe_weights* w, const tsp_moe_scratch* s, con
         if (int rc = tsp_moe_project(&w->down, s->d_hidden, hidden * 4ull, 1, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_routed, channels * 4ull, 0,
                                      d_error, stream)) return rc;
     } else {
-        if (int rc = tsp_moe_gate_up_swiglu_shared(&w->gate, &w->up, &w->shared_gate, &w->shared_up, x32, x32_stride, x_dtype == 1 ? d_x : nullptr,
-                                                   x_dtype == 1 ? x_stride : 0, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden,
-                                                   hidden * 4ull, s->d_shared_hidden, hidden * 4ull, exact, d_error, stream)) return rc;
+        if (!gated)
+            if (int rc = tsp_moe_gate_up_swiglu_shared(&w->gate, &w->up, &w->shared_gate, &w->shared_up, x32, x32_stride, x_dtype == 1 ? d_x : nullptr,
+                                                       x_dtype == 1 ? x_stride : 0, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden,
+                                                       hidden * 4ull, s->d_shared_hidden, hidden * 4ull, exact, d_error, stream)) return rc;
         if (int rc = tsp_moe_project_shared(&w->down, &w->shared_down, s->d_hidden, hidden * 4ull, s->d_shared_hidden, hidden * 4ull, tokens, selected,
                                             s->d_token_map, s->d_counts, s->d_tasks, s->d_routed, channels * 4ull, s->d_shared_out, channels * 4ull,
                                             d_error, stream)) return rc;
     }
     // binary16 output rows are written straight from the FP32 mixture; no FP32 copy of the output is kept
-    return tsp_moe_combine(s->d_routed, channels * 4ull, 0, s->d_weights, s->d_shared_out, channels * 4ull, w->d_shared_router, x32,
-                           x32_stride, 0, s->d_shared_logit, tokens, channels, selected,
+    return tsp_moe_combine(s->d_routed, channels * 4ull, 0, s->d_weights, s->d_shared_out, channels * 4ull, w->d_shared_router, gated ? d_x : x32,
+                           gated ? x_stride : x32_stride, gated ? x_dtype : 0, s->d_shared_logit, tokens, channels, selected,
                            out_dtype == 0 ? static_cast<float*>(d_out) : nullptr, out_dtype == 0 ? out_stride : 0,
                            out_dtype == 1 ? d_out : nullptr, out_dtype == 1 ? out_stride : 0, d_error, st);
 }

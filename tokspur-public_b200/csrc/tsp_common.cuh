@@ -31,6 +31,14 @@ static inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }
 
+// Routing of a small decode batch inside the gate-up launch itself (tsp_gemv_tma.cu): what tsp_moe_route and tsp_moe_permute would be given
+struct GemvRoute {
+    const float* logits; uint64_t logits_stride_bytes;
+    uint32_t selected, mode;
+    uint32_t* ids; float* weights;
+    uint32_t *token_map, *counts, *tasks;
+};
+
 // A dense expert (experts == 1 sets with the routed experts' shape, encoding and layout) that a routed projection launch
 // also processes, for every token row: input rows `x`, output rows `out`. b is used by gate-up launches only.
 struct GemvShared {
@@ -40,6 +48,7 @@ struct GemvShared {
     // optional: the token rows as binary16 (exactly the values of `x`); both the routed and the dense tiles then read these
     const void* x16 = nullptr; uint64_t x16_stride_bytes = 0;
     uint32_t tokens = 0;   // rows of the dense expert (0: as many as the routed launch has token rows)
+    const GemvRoute* route = nullptr;   // gate-up: the launch routes its own batch
 };
 
 // the layer's dense shared expert riding in a routed launch: one-expert matrix sets of the routed experts' shape, binary16

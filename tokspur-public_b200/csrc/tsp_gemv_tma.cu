@@ -27,6 +27,7 @@
 #include <cuda.h>
 
 #include "tsp_common.cuh"
+#include "tsp_route_row.cuh"
 
 namespace tsp {
 
@@ -75,7 +76,20 @@ struct Gemv3Params {
     const float* sh_x; uint64_t sh_x_stride_bytes;
     float* sh_out; uint64_t sh_out_stride_bytes;
     uint32_t sh_tiles, sh_tokens;
+    // gate-up of up to kRouteTokens3 rows: the launch routes the batch (logits != null). Every block but the last works; the last one publishes
+    uint32_t workers;
+    const float* logits; uint64_t logits_stride_bytes;
+    uint32_t selected, route_mode;
+    uint32_t* r_ids; float* r_weights; uint32_t *r_token_map, *r_counts, *r_tasks;
 };
+
+// Routing inside the gate-up launch. At these sizes a layer is a chain of short launches; routing and its tables were two of them, and a third of
+// the time up to the first weight (four layers of one row 138 -> 118 us, two of eight rows 133 -> 128). Every block selects the experts of all rows itself (a warp
+// per row), takes its own tiles from a mask of rows per expert in shared memory, and one block that takes no weights writes ids, mixture weights and
+// tables for the launches behind: the ones of the kernels in tsp_route.cu, bit for bit. Up to eight rows: an expert then has one tile
+// (TSP_GEMV_TILE rows), and one warp per row is there.
+constexpr uint32_t kRouteTokens3 = TSP_GEMV_TILE, kRouteExperts3 = 512;
+constexpr uint32_t kRouteScratch3 = kRouteExperts3 * 4 + 64 + kRouteTokens3 * 64 * 4;   // row masks, hit bits, ids
 
 __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, int c0, int c1, int c2, int c3, uint64_t* bar) {
     asm volatile(
@@ -120,11 +134,72 @@ __device__ __forceinline__ Tile3 tile3(const Gemv3Params& p, uint32_t tile, uint
     return t;
 }
 
+// ---- routing inside the launch (ROUTE). mask: [kRouteExperts3] rows that name an expert, 16 words of
+// experts hit, then the selected ids [row][selected]; zero on entry up to the ids.
+__device__ __forceinline__ uint32_t route3_select(const Gemv3Params& p, uint32_t* mask) {
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t *hit = mask + kRouteExperts3, *sel = hit + 16;
+    if (warp < p.tokens) {
+        const bool publish = blockIdx.x >= p.workers;
+        route_row_regs(reinterpret_cast<const float*>(reinterpret_cast<const char*>(p.logits) + warp * p.logits_stride_bytes), warp, p.experts, p.selected,
+                       p.route_mode, sel, publish ? p.r_weights : nullptr, publish ? p.error : nullptr, lane);
+        __syncwarp();
+        for (uint32_t r = lane; r < p.selected; r += 32) {
+            const uint32_t e = sel[warp * p.selected + r];
+            atomicOr(&mask[e], 1u << warp);
+            atomicOr(&hit[e >> 5], 1u << (e & 31u));
+        }
+    }
+    __syncthreads();
+    uint32_t tiles = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < 16; ++i) tiles += __popc(hit[i]);
+    return tiles;
+}
+__device__ __forceinline__ uint32_t route3_tile(const uint32_t* hit, uint32_t e) {   // tile of an expert: experts hit below it
+    uint32_t n = __popc(hit[e >> 5] & ((1u << (e & 31u)) - 1u));
+    for (uint32_t i = 0; i < (e >> 5); ++i) n += __popc(hit[i]);
+    return n;
+}
+__device__ __forceinline__ void route3_publish(const Gemv3Params& p, const uint32_t* mask, uint32_t tiles) {
+    const uint32_t *hit = mask + kRouteExperts3, *sel = hit + 16;
+    const uint32_t routes = p.tokens * p.selected, bound = routes / TSP_GEMV_TILE + p.experts;
+    for (uint32_t e = threadIdx.x; e < p.experts; e += blockDim.x) p.r_counts[e] = __popc(mask[e]);
+    for (uint32_t i = tiles + threadIdx.x; i < bound; i += blockDim.x) { p.r_tasks[2 + 2 * i] = 0xffffffffu; p.r_tasks[3 + 2 * i] = 0xffffffffu; }
+    for (uint32_t i = threadIdx.x; i < routes; i += blockDim.x) {
+        const uint32_t e = sel[i], t = i / p.selected, at = __popc(mask[e] & ((1u << t) - 1u));
+        p.r_ids[i] = e;
+        p.r_token_map[static_cast<uint64_t>(e) * p.tokens + at] = i;
+        if (at == 0) { const uint32_t tile = route3_tile(hit, e); p.r_tasks[2 + 2 * tile] = e; p.r_tasks[3 + 2 * tile] = 0u; }
+    }
+    if (threadIdx.x == 0) { p.r_tasks[0] = tiles; p.r_tasks[1] = routes; }
+}
+// The tile table of a block whose first tile is t0: up to 513 tiles over the blocks of a grid, never more than the table holds per block
+__device__ __forceinline__ void route3_table(const Gemv3Params& p, const uint32_t* mask, uint32_t routed_tiles, uint32_t t0, uint32_t* tt, uint32_t* trid, uint32_t* tin) {
+    const uint32_t *hit = mask + kRouteExperts3, *sel = hit + 16;
+    for (uint32_t i = threadIdx.x; i < p.tokens * p.selected; i += blockDim.x) {
+        const uint32_t e = sel[i], t = i / p.selected, rows = mask[e], slot = __popc(rows & ((1u << t) - 1u)), tl = route3_tile(hit, e) - t0;
+        if (tl < kTableTiles) {
+            trid[tl * 16 + slot] = i; tin[tl * 16 + slot] = t;
+            if (slot == 0) { tt[tl * 4] = e; tt[tl * 4 + 1] = 0u; tt[tl * 4 + 2] = __popc(rows); }
+        }
+    }
+    for (uint32_t i = threadIdx.x; i < p.sh_tiles * 8u; i += blockDim.x) {   // the dense expert's tiles
+        const uint32_t tl = routed_tiles + (i >> 3) - t0, slot = i & 7u;
+        if (tl < kTableTiles) {
+            trid[tl * 16 + slot] = i; tin[tl * 16 + slot] = i;
+            if (slot == 0) { tt[tl * 4] = p.experts; tt[tl * 4 + 1] = i; tt[tl * 4 + 2] = min(p.sh_tokens - i, 8u); }
+        }
+    }
+}
+
 // LAYOUT: TSP_LAYOUT_PLANAR (code lines + scale / (d, dmin) planes) or TSP_LAYOUT_GGUF (whole 144-byte blocks, unswizzled)
 // KB: super-blocks per unit. SPLIT: also run the low-half pass of the activations (needed unless every
 // activation is exactly a binary16 value).
 // W: consumer warps (pipelines) per CTA. Every launch uses eight (232 registers each); the parameter exists for experiments.
-template <uint32_t LAYOUT, bool GATEUP, int NC, int NT, int KB, bool SPLIT, int W = kW3>
+// ROUTE: the launch routes its own batch (an instantiation of its own: with the routing as a run-time choice the loop below it came out slower, 16 rows
+// 90 -> 93 us, of GGUF blocks 95 -> 104).
+template <uint32_t LAYOUT, bool GATEUP, int NC, int NT, int KB, bool SPLIT, bool ROUTE, int W = kW3>
 __global__ void __launch_bounds__((W + kProd3) * 32, 1) gemv3_kernel(const __grid_constant__ Gemv3Maps maps, const Gemv3Params p) {
     pdl_launch_dependents();
     extern __shared__ uint8_t smem3_raw[];
@@ -148,9 +223,20 @@ __global__ void __launch_bounds__((W + kProd3) * 32, 1) gemv3_kernel(const __gri
         for (uint32_t s = 0; s < S * W; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_fence_init();
     }
+    // routing scratch: the activation rows' place (staged later, behind barriers)
+    uint32_t* const r_mask = reinterpret_cast<uint32_t*>(smem3 + p.off_xhi);
+    uint32_t hit_tiles = 0;
+    if constexpr (ROUTE) {
+        for (uint32_t i = threadIdx.x; i < kRouteExperts3 + 16; i += blockDim.x) r_mask[i] = 0u;
+        __syncthreads();
+    }
     pdl_wait();   // everything above touched shared memory only
+    if constexpr (ROUTE) {
+        hit_tiles = route3_select(p, r_mask);
+        if (blockIdx.x >= p.workers) { route3_publish(p, r_mask, hit_tiles); return; }
+    }
 
-    const uint32_t routed_tiles = p.token_map ? p.tasks[0] : (p.tokens + 8u * NC - 1) / (8u * NC);
+    const uint32_t routed_tiles = ROUTE ? hit_tiles : p.token_map ? p.tasks[0] : (p.tokens + 8u * NC - 1) / (8u * NC);
     const uint32_t n_tiles = routed_tiles + p.sh_tiles;
     const uint64_t n_items = static_cast<uint64_t>(n_tiles) * p.groups;   // item = (tile, row group)
     // Static split by cost, not by item count: besides its items a token tile costs the staging of its activation rows, about
@@ -158,19 +244,21 @@ __global__ void __launch_bounds__((W + kProd3) * 32, 1) gemv3_kernel(const __gri
     // an even split the CTAs that get the dense expert's tiles (the last ones) finished 9-14 us after the rest of a 100 us launch.
     // Cost per item in 1/256 item units: 256 + rows of the tile * row cost / groups, piecewise constant over the two kinds of tile.
     const uint64_t row_cost = 200ull * p.cols / 2048u;
-    const uint64_t routes = p.token_map ? p.tasks[1] : p.tokens;
+    const uint64_t routes = ROUTE ? p.tokens * p.selected : p.token_map ? p.tasks[1] : p.tokens;
     const uint64_t ci_r = 256ull + (routed_tiles ? routes * row_cost / (static_cast<uint64_t>(routed_tiles) * p.groups) : 0ull);
     const uint64_t ci_s = 256ull + static_cast<uint64_t>(p.sh_tiles ? (p.sh_tokens + p.sh_tiles - 1) / p.sh_tiles : 0u) * row_cost / p.groups;
     const uint64_t n_r = static_cast<uint64_t>(routed_tiles) * p.groups, cost_r = n_r * ci_r, cost_all = cost_r + (n_items - n_r) * ci_s;
     auto boundary = [&](uint32_t b) -> uint32_t {
-        if (b >= gridDim.x) return static_cast<uint32_t>(n_items);
-        const uint64_t c = cost_all * b / gridDim.x;
+        if (b >= p.workers) return static_cast<uint32_t>(n_items);
+        const uint64_t c = cost_all * b / p.workers;
         return static_cast<uint32_t>(c < cost_r ? c / ci_r : n_r + (c - cost_r) / ci_s);
     };
     const uint32_t item0 = boundary(blockIdx.x), item1 = boundary(blockIdx.x + 1);
     // Tile table: the (expert, first route, route count), route ids and input rows of the first kTableTiles token tiles this
     // CTA touches, fetched once and in parallel, so that the dependent global loads behind them are not paid at every tile.
     const uint32_t t0 = item0 / p.groups;
+    if constexpr (ROUTE) route3_table(p, r_mask, routed_tiles, t0, tt, trid, tin);
+    else
     for (uint32_t i = threadIdx.x; i < kTableTiles * 16; i += blockDim.x) {
         const uint32_t tl = i >> 4, slot = i & 15u, tile = t0 + tl;
         if (tile < n_tiles && item0 < item1) {
@@ -614,9 +702,9 @@ __global__ void __launch_bounds__((W + kProd3) * 32, 1) gemv3_kernel(const __gri
 // ---------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------
-template <uint32_t LAYOUT, bool GATEUP, int NC, int NT, int KB, bool SPLIT, int W = kW3>
+template <uint32_t LAYOUT, bool GATEUP, int NC, int NT, int KB, bool SPLIT, bool ROUTE = false, int W = kW3>
 static int launch3(const Gemv3Maps& maps, const Gemv3Params& p, size_t smem, int grid, cudaStream_t st) {
-    auto kernel = gemv3_kernel<LAYOUT, GATEUP, NC, NT, KB, SPLIT, W>;
+    auto kernel = gemv3_kernel<LAYOUT, GATEUP, NC, NT, KB, SPLIT, ROUTE, W>;
     static thread_local int regs_ok = -1;   // the register hand-over between producer and consumer warps adds up for this build
     if (regs_ok < 0) {
         cudaFuncAttributes fa{};
@@ -788,6 +876,22 @@ int launch_gemv_q4k_tma(const tsp_matrix_set* a, const tsp_matrix_set* b, bool g
     }
     const int grid = sm_count();
     if (grid <= 0) return fail(TSP_E_CUDA, "no usable CUDA device");
+    p.workers = static_cast<uint32_t>(grid);
+    if (shared && shared->route) {
+        const GemvRoute& r = *shared->route;
+        // a block's tiles fit its table (513 tiles at most), the scratch fits the rows' place; anything else is routed by launches of its own
+        if (!gateup || nc != 1 || tokens > kRouteTokens3 || a->experts > kRouteExperts3 || grid < 32 || 8u * p.x_stride < kRouteScratch3 ||
+            (f16_exact && !p.x16)) return 1;
+        p.workers = static_cast<uint32_t>(grid) - 1u;
+        p.logits = r.logits; p.logits_stride_bytes = r.logits_stride_bytes; p.selected = r.selected; p.route_mode = r.mode;
+        p.r_ids = r.ids; p.r_weights = r.weights; p.r_token_map = r.token_map; p.r_counts = r.counts; p.r_tasks = r.tasks;
+    }
+#define TSP_R4(L, K)                                                               \
+    return split_lo ? launch3<L, true, 1, 1, K, true, true>(maps, p, smem, grid, st) : launch3<L, true, 1, 1, K, false, true>(maps, p, smem, grid, st)
+#define TSP_R3(L) do { if (kb == 4) { TSP_R4(L, 4); } else if (kb == 2) { TSP_R4(L, 2); } else { TSP_R4(L, 1); } } while (0)
+    if (p.logits) { if (planar) TSP_R3(TSP_LAYOUT_PLANAR); TSP_R3(TSP_LAYOUT_GGUF); }
+#undef TSP_R3
+#undef TSP_R4
 #define TSP_D4(L, G, NCV, NTV, K)                                                  \
     return split_lo ? launch3<L, G, NCV, NTV, K, true>(maps, p, smem, grid, st)    \
                     : launch3<L, G, NCV, NTV, K, false>(maps, p, smem, grid, st)
