@@ -236,38 +236,59 @@ __global__ void __launch_bounds__((W + kProd3) * 32, 1) gemv3_kernel(const __gri
         if (blockIdx.x >= p.workers) { route3_publish(p, r_mask, hit_tiles); return; }
     }
 
+    // The task table's first entries, on their way together with the tile count (a block's tiles are known only behind it); the table holds at
+    // least as many entries as there are experts. In the activation rows' place, like the routing's scratch.
+    uint2* const ahead_tasks = reinterpret_cast<uint2*>(r_mask);
+    const uint32_t ahead = !ROUTE && p.token_map ? min(min(p.experts, blockDim.x), static_cast<uint32_t>(8u * NC * p.x_stride / sizeof(uint2))) : 0u;
+    if (threadIdx.x < ahead) ahead_tasks[threadIdx.x] = make_uint2(p.tasks[2 + 2 * threadIdx.x], p.tasks[3 + 2 * threadIdx.x]);
     const uint32_t routed_tiles = ROUTE ? hit_tiles : p.token_map ? p.tasks[0] : (p.tokens + 8u * NC - 1) / (8u * NC);
     const uint32_t n_tiles = routed_tiles + p.sh_tiles;
-    const uint64_t n_items = static_cast<uint64_t>(n_tiles) * p.groups;   // item = (tile, row group)
+    const uint32_t n_items = n_tiles * p.groups;   // item = (tile, row group)
     // Static split by cost, not by item count: besides its items a token tile costs the staging of its activation rows, about
     // 0.8 items per row of 2048 columns. Routed tiles carry routes / tiles rows on average, the dense expert's tiles eight: with
     // an even split the CTAs that get the dense expert's tiles (the last ones) finished 9-14 us after the rest of a 100 us launch.
     // Cost per item in 1/256 item units: 256 + rows of the tile * row cost / groups, piecewise constant over the two kinds of tile.
-    const uint64_t row_cost = 200ull * p.cols / 2048u;
-    const uint64_t routes = ROUTE ? p.tokens * p.selected : p.token_map ? p.tasks[1] : p.tokens;
-    const uint64_t ci_r = 256ull + (routed_tiles ? routes * row_cost / (static_cast<uint64_t>(routed_tiles) * p.groups) : 0ull);
-    const uint64_t ci_s = 256ull + static_cast<uint64_t>(p.sh_tiles ? (p.sh_tokens + p.sh_tiles - 1) / p.sh_tiles : 0u) * row_cost / p.groups;
-    const uint64_t n_r = static_cast<uint64_t>(routed_tiles) * p.groups, cost_r = n_r * ci_r, cost_all = cost_r + (n_items - n_r) * ci_s;
+    // In FP32: every block computes a bound the same way and the bounds ascend, so that each item has one owner whatever the rounding; as 64-bit integer
+    // divisions the split took about a microsecond in front of every launch's first copy.
+    const float row_cost = 200.f * p.cols / 2048.f;
+    const float routes = static_cast<float>(ROUTE ? p.tokens * p.selected : p.token_map ? p.tasks[1] : p.tokens);
+    const float ci_r = 256.f + (routed_tiles ? __fdividef(routes * row_cost, static_cast<float>(routed_tiles) * p.groups) : 0.f);
+    const float ci_s = 256.f + (p.sh_tiles ? __fdividef(static_cast<float>((p.sh_tokens + p.sh_tiles - 1) / p.sh_tiles) * row_cost, static_cast<float>(p.groups)) : 0.f);
+    const uint32_t n_r = routed_tiles * p.groups;
+    const float cost_r = n_r * ci_r, cost_all = cost_r + (n_items - n_r) * ci_s, inv_r = __fdividef(1.f, ci_r), inv_s = __fdividef(1.f, ci_s);
+    const float per_worker = __fdividef(cost_all, static_cast<float>(p.workers));
     auto boundary = [&](uint32_t b) -> uint32_t {
-        if (b >= p.workers) return static_cast<uint32_t>(n_items);
-        const uint64_t c = cost_all * b / p.workers;
-        return static_cast<uint32_t>(c < cost_r ? c / ci_r : n_r + (c - cost_r) / ci_s);
+        if (b >= p.workers) return n_items;
+        const float c = __fmul_rn(per_worker, static_cast<float>(b));   // no contraction: the same value wherever this is inlined
+        return c < cost_r ? min(n_r, static_cast<uint32_t>(__fmul_rn(c, inv_r))) : min(n_items, n_r + static_cast<uint32_t>(__fmul_rn(__fsub_rn(c, cost_r), inv_s)));
     };
     const uint32_t item0 = boundary(blockIdx.x), item1 = boundary(blockIdx.x + 1);
     // Tile table: the (expert, first route, route count), route ids and input rows of the first kTableTiles token tiles this
     // CTA touches, fetched once and in parallel, so that the dependent global loads behind them are not paid at every tile.
     const uint32_t t0 = item0 / p.groups;
+    if constexpr (!ROUTE) __syncthreads();
     if constexpr (ROUTE) route3_table(p, r_mask, routed_tiles, t0, tt, trid, tin);
     else
     for (uint32_t i = threadIdx.x; i < kTableTiles * 16; i += blockDim.x) {
         const uint32_t tl = i >> 4, slot = i & 15u, tile = t0 + tl;
         if (tile < n_tiles && item0 < item1) {
-            const Tile3 ti = tile3<NC>(p, tile, routed_tiles);
-            if (slot == 0) { tt[tl * 4] = ti.expert; tt[tl * 4 + 1] = ti.start; tt[tl * 4 + 2] = ti.count; }
-            uint32_t rid = 0;
-            if (slot < ti.count) rid = (p.token_map && ti.expert < p.experts) ? p.token_map[static_cast<uint64_t>(ti.expert) * p.tokens + ti.start + slot] : ti.start + slot;
-            trid[i] = rid;
-            tin[i] = ti.expert < p.experts ? rid / p.in_div : rid;
+            if (p.token_map && tile < routed_tiles) {
+                // count and route id side by side, each one load behind the task entry (which came with the tile count, where it is one of the first)
+                const uint2 task = tile < ahead ? ahead_tasks[tile] : make_uint2(p.tasks[2 + 2 * tile], p.tasks[3 + 2 * tile]);
+                const bool valid = task.x < p.experts;
+                const uint32_t expert = valid ? task.x : 0u, at = valid ? task.y + slot : p.tokens;
+                const uint32_t c = valid ? p.counts[expert] : 0u, rid = at < p.tokens ? p.token_map[static_cast<uint64_t>(expert) * p.tokens + at] : 0u;
+                const uint32_t count = c > task.y ? min(c - task.y, 8u * NC) : 0u;
+                if (slot == 0) { tt[tl * 4] = expert; tt[tl * 4 + 1] = valid ? task.y : 0u; tt[tl * 4 + 2] = count; }
+                trid[i] = slot < count ? rid : 0u;
+                tin[i] = slot < count ? rid / p.in_div : 0u;
+            } else {
+                const Tile3 ti = tile3<NC>(p, tile, routed_tiles);
+                if (slot == 0) { tt[tl * 4] = ti.expert; tt[tl * 4 + 1] = ti.start; tt[tl * 4 + 2] = ti.count; }
+                const uint32_t rid = slot < ti.count ? ti.start + slot : 0u;
+                trid[i] = rid;
+                tin[i] = ti.expert < p.experts ? rid / p.in_div : rid;
+            }
         }
     }
     __syncthreads();
