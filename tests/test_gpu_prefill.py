@@ -124,3 +124,47 @@ def test_overflowing_hidden_row_is_reported_and_stays_alone(oracle):
     others = np.arange(T) != 77
     assert np.array_equal(outs[0][others], outs[1][others]) and np.array_equal(outs[0][others], outs[2][others])
     assert np.isfinite(outs[1]).all() and not np.isfinite(outs[2][77]).all()
+
+
+# The cluster that builds the tables of more than 256 rows: an eighth of the rows per block in words of 32 (blocks without rows at 257), one word
+# per block and several, the largest batch whose masks fit and the first that takes a block per pair of experts, an owner's slice of the experts
+@pytest.mark.parametrize("tokens,experts,selected,first,local", [(257, 512, 10, 0, 512), (512, 512, 1, 0, 512), (1003, 1000, 8, 0, 1000), (2049, 16, 16, 0, 16), (4096, 512, 10, 128, 64),
+                                                                 (16640, 512, 2, 0, 512), (16641, 512, 2, 0, 512), (300, 1024, 64, 0, 1024)])
+def test_tables_of_large_batches(oracle, tokens, experts, selected, first, local):
+    rng = np.random.default_rng(tokens)
+    ids = np.argsort(rng.random((tokens, experts), dtype=np.float32) - (np.arange(experts) < experts // 8) * 0.5, axis=1)[:, :selected].astype(np.uint32)
+    dids = torch.from_numpy(ids.view(np.int32)).cuda()
+    tmap, counts = torch.full((local * tokens,), -7, dtype=torch.int32, device="cuda"), torch.empty(local, dtype=torch.int32, device="cuda")
+    words = int(capi.lib().tsp_moe_tasks_words(tokens, local, selected, 32))
+    tasks, e = torch.full((words,), -7, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    if local == experts:
+        capi.call("tsp_moe_permute", dids.data_ptr(), tokens, experts, selected, 32, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(), e.data_ptr(), L.stream_ptr())
+    else:
+        capi.call("tsp_moe_permute_local", dids.data_ptr(), tokens, first, local, selected, 32, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(), e.data_ptr(), L.stream_ptr())
+    torch.cuda.synchronize()
+    assert int(e.item()) == 0
+    want_counts = np.bincount(ids.reshape(-1), minlength=experts)[first:first + local]
+    assert np.array_equal(counts.cpu().numpy(), want_counts)
+    order = np.argsort(ids.reshape(-1), kind="stable")   # routes by expert, ascending
+    starts = np.concatenate([[0], np.cumsum(np.bincount(ids.reshape(-1), minlength=experts))])
+    got = tmap.cpu().numpy().reshape(local, tokens)
+    for i in range(local):
+        n = want_counts[i]
+        assert np.array_equal(got[i, :n], order[starts[first + i]:starts[first + i] + n]) and (got[i, n:] == -7).all()
+    pairs = [(i, t) for i in range(local) for t in range(0, want_counts[i], 32)]
+    want_tasks = np.full(words, 0xffffffff, dtype=np.uint32)
+    want_tasks[:2 + 2 * len(pairs)] = np.array([len(pairs), want_counts.sum()] + [v for p in pairs for v in p], dtype=np.uint32)
+    assert np.array_equal(tasks.cpu().numpy().view(np.uint32), want_tasks)
+
+
+@pytest.mark.parametrize("bad", ["twice", "range"])
+def test_tables_of_large_batches_report_bad_ids(bad):
+    tokens, experts, selected = 700, 64, 4
+    ids = np.tile(np.arange(selected, dtype=np.int32), (tokens, 1))
+    ids[650, 2] = ids[650, 1] if bad == "twice" else experts
+    dids, e = torch.from_numpy(ids).cuda(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    tmap, counts = torch.empty(experts * tokens, dtype=torch.int32, device="cuda"), torch.empty(experts, dtype=torch.int32, device="cuda")
+    tasks = torch.empty(int(capi.lib().tsp_moe_tasks_words(tokens, experts, selected, 8)), dtype=torch.int32, device="cuda")
+    capi.call("tsp_moe_permute", dids.data_ptr(), tokens, experts, selected, 8, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(), e.data_ptr(), L.stream_ptr())
+    torch.cuda.synchronize()
+    assert int(e.item()) & capi.ERR_INDEX

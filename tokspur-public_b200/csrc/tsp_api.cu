@@ -40,7 +40,7 @@ int sm_count() {
 
 // launchers implemented in the kernel files
 int launch_route(const float*, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t*, float*, uint32_t*, cudaStream_t, float* = nullptr);
-int launch_permute(const uint32_t*, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t*, uint32_t*, uint32_t*, uint32_t*, cudaStream_t);
+int launch_permute(const uint32_t*, uint32_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t*, uint32_t*, uint32_t*, uint32_t*, cudaStream_t, uint32_t* = nullptr);
 int launch_combine(const void*, uint64_t, uint32_t, const float*, const float*, uint64_t, const float*, const void*, uint64_t, uint32_t, float*,
                    uint32_t, uint32_t, uint32_t, float*, uint64_t, void*, uint64_t, uint32_t*, cudaStream_t);
 int launch_decode_prologue(const float*, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t, uint32_t*, float*, uint32_t*, uint32_t*,
@@ -226,15 +226,24 @@ uint64_t tsp_moe_tasks_words(uint32_t tokens, uint32_t experts, uint32_t selecte
     return 2 + 2 * ((static_cast<uint64_t>(tokens) * selected) / tile + experts);
 }
 
-int tsp_moe_permute(const uint32_t* d_ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile,
-                    uint32_t* d_token_map, uint32_t* d_counts, uint32_t* d_tasks, uint32_t* d_error, void* stream) {
+}  // extern "C"
+
+static int permute(const uint32_t* d_ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t* d_token_map, uint32_t* d_counts,
+                   uint32_t* d_tasks, uint32_t* d_offsets, uint32_t* d_error, void* stream) {
     TSP_REQUIRE(d_ids && d_token_map && d_counts && d_tasks, "permute: null buffer");
     TSP_REQUIRE(tokens >= 1 && experts >= 1 && experts <= 4096 && selected >= 1 && selected <= 64 && selected <= experts,
                 "permute: invalid shape");
     TSP_REQUIRE(tile >= 1 && tile <= 1024, "permute: tile out of range");
     TSP_REQUIRE(static_cast<uint64_t>(tokens) * selected < (1ull << 31), "permute: too many routes");
     return launch_permute(d_ids, tokens, experts, selected, tile, 0, 0, d_token_map, d_counts, d_tasks, d_error,
-                          static_cast<cudaStream_t>(stream));
+                          static_cast<cudaStream_t>(stream), d_offsets);
+}
+
+extern "C" {
+
+int tsp_moe_permute(const uint32_t* d_ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile,
+                    uint32_t* d_token_map, uint32_t* d_counts, uint32_t* d_tasks, uint32_t* d_error, void* stream) {
+    return permute(d_ids, tokens, experts, selected, tile, d_token_map, d_counts, d_tasks, nullptr, d_error, stream);
 }
 
 int tsp_moe_permute_local(const uint32_t* d_ids, uint32_t tokens, uint32_t first_expert, uint32_t local_experts, uint32_t selected,
@@ -755,8 +764,7 @@ int tsp_moe_layer_prefill(const tsp_moe_weights* w, const tsp_moe_prefill_scratc
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int rc = tsp_moe_rows_f16k(d_x, x_stride, x_dtype, tokens, channels, ps->d_xk, channels * 2ull, d_error, st)) return rc;
     if (int rc = tsp_moe_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_error, st)) return rc;
-    if (int rc = tsp_moe_permute(s->d_ids, tokens, experts, selected, TSP_GROUPED_TILE, s->d_token_map, s->d_counts, s->d_tasks, d_error, st)) return rc;
-    if (int rc = tsp_moe_route_offsets(s->d_counts, experts, ps->d_offsets, st)) return rc;
+    if (int rc = permute(s->d_ids, tokens, experts, selected, TSP_GROUPED_TILE, s->d_token_map, s->d_counts, s->d_tasks, ps->d_offsets, d_error, st)) return rc;
     if (int rc = tsp_moe_gather_rows16(ps->d_xk, channels * 2ull, s->d_token_map, ps->d_offsets, experts, tokens, selected, channels, ps->d_xp,
                                        channels * 2ull, st)) return rc;
     // the dense shared expert rides in both launches when it has the routed experts' encoding and layout; in another form (the

@@ -339,6 +339,134 @@ tables_kernel(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t s
     }
 }
 
+// The same tables of larger batches by ONE cluster of eight blocks, each with the masks of an eighth of the rows (whole words): a block counts its
+// experts, reads the other blocks' counts through distributed shared memory, and so knows every expert's total, its own first position in each and
+// the scan over experts. offsets (optional): first permuted position of every expert, their total, four zeroed counters (tsp_moe_route_offsets).
+// Latency of a few round trips whatever the batch. A block per pair of experts that reads all routes took 45 us for 4096 rows of ten (512
+// experts) of Zipf loads and 35 us of even ones, the one-block form 14 us for 1003, the scans behind them 6 and 2 us more; 15 and 6.5 us now. Up to 256 rows
+// the one block is as fast (257 rows 5.8 / 5.2 us).
+constexpr uint32_t kTablesCluster = 8;
+__device__ __forceinline__ uint32_t dsmem_u32(const uint32_t* own, uint32_t rank) {   // the word at the same place in another block's shared memory
+    uint32_t addr, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(own)), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kPrologueThreads)
+tables_cluster_kernel(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
+                      uint32_t words, uint32_t* __restrict__ token_map, uint32_t* __restrict__ counts, uint32_t* __restrict__ tasks, uint32_t* __restrict__ offsets,
+                      uint32_t* error) {
+    pdl_launch_dependents();
+    // [experts] counts of this block, [experts][stride] masks, [experts][stride] running counts of the words before each word, then first positions
+    extern __shared__ __align__(16) uint32_t tables_mask[];
+    const uint32_t stride = words | 1u;
+    uint32_t* const own = tables_mask;
+    uint32_t* const mask = own + experts;
+    uint32_t* const base = mask + experts * stride;
+    uint16_t* const before_word = reinterpret_cast<uint16_t*>(base + experts);
+    __shared__ uint32_t warp_tiles[32], warp_routes[32];
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5, rank = blockIdx.x;
+    for (uint32_t i = tid; i < experts * stride; i += blockDim.x) mask[i] = 0u;
+    const uint32_t t0 = rank * words * 32u, t1 = min(tokens, t0 + words * 32u);   // this block's rows
+    const uint32_t r0 = t0 * selected, r1 = max(t0, t1) * selected;
+    const uint32_t routes = tokens * selected, bound = routes / tile + experts;
+    pdl_wait();   // the ids come from the previous launch; everything above touched shared memory only
+    __syncthreads();
+    for (uint32_t i = r0 + tid; i < r1; i += blockDim.x) {
+        const uint32_t t = i / selected - t0, e = ids[i] - first;
+        if (e >= experts) { if (!local_only) raise_error(error, TSP_ERR_INDEX); continue; }
+        const uint32_t bit = 1u << (t & 31u);
+        if (atomicOr(&mask[e * stride + (t >> 5)], bit) & bit) raise_error(error, TSP_ERR_INDEX);   // an expert named twice by one token
+    }
+    for (uint32_t i = rank * blockDim.x + tid; i < bound; i += kTablesCluster * blockDim.x) { tasks[2 + 2 * i] = 0xffffffffu; tasks[3 + 2 * i] = 0xffffffffu; }
+    __syncthreads();
+    if (tid < experts) {
+        uint32_t c = 0;
+        for (uint32_t w = 0; w < words; ++w) { before_word[tid * stride + w] = static_cast<uint16_t>(c); c += __popc(mask[tid * stride + w]); }
+        own[tid] = c;
+    }
+    cluster_sync();   // counts of every block; the padding of the tile table is ordered before the entries below as well
+    uint32_t c = 0, n = 0;
+    if (tid < experts) {
+        uint32_t at = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kTablesCluster; ++q) {
+            const uint32_t v = dsmem_u32(own + tid, q);
+            if (q < rank) at += v;
+            c += v;
+        }
+        base[tid] = at;
+        n = (c + tile - 1) / tile;
+    }
+    uint32_t incl_n = n, incl_c = c;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t tn = __shfl_up_sync(0xffffffffu, incl_n, o), tc = __shfl_up_sync(0xffffffffu, incl_c, o);
+        if (lane >= static_cast<uint32_t>(o)) { incl_n += tn; incl_c += tc; }
+    }
+    if (lane == 31) { warp_tiles[warp] = incl_n; warp_routes[warp] = incl_c; }
+    __syncthreads();
+    for (uint32_t i = r0 + tid; i < r1; i += blockDim.x) {
+        const uint32_t t = i / selected - t0, e = ids[i] - first;
+        if (e >= experts) continue;
+        const uint32_t at = e * stride + (t >> 5);
+        token_map[static_cast<uint64_t>(e) * tokens + base[e] + before_word[at] + __popc(mask[at] & ((1u << (t & 31u)) - 1u))] = i;
+    }
+    if (rank == 0) {
+        uint32_t before_n = 0, total_n = 0, before_c = 0, total_c = 0;
+        for (uint32_t i = 0; i < nwarps; ++i) {
+            if (i < warp) { before_n += warp_tiles[i]; before_c += warp_routes[i]; }
+            total_n += warp_tiles[i]; total_c += warp_routes[i];
+        }
+        if (tid == 0) {
+            tasks[0] = min(total_n, bound);
+            tasks[1] = total_c;
+            if (total_n > bound || (!local_only && total_c != routes) || total_c > routes) raise_error(error, TSP_ERR_INDEX);
+            if (offsets) {
+                offsets[experts] = total_c;
+                for (uint32_t i = 1; i <= 4; ++i) offsets[experts + i] = 0;
+            }
+        }
+        if (tid < experts) {
+            counts[tid] = c;
+            if (offsets) offsets[tid] = before_c + incl_c - c;
+            const uint32_t at0 = before_n + incl_n - n;
+            for (uint32_t i = 0; i < n; ++i) {
+                const uint32_t at = at0 + i;
+                if (at < bound) { tasks[2 + 2 * at] = tid; tasks[3 + 2 * at] = i * tile; }
+            }
+        }
+    }
+    cluster_sync();   // no block leaves while another reads its counts
+}
+
+static uint32_t cluster_words(uint32_t tokens) { return ((tokens + kTablesCluster - 1) / kTablesCluster + 31) / 32; }
+static size_t cluster_smem(uint32_t tokens, uint32_t experts) { return static_cast<size_t>(experts) * (8u + (cluster_words(tokens) | 1u) * 6u); }
+static bool cluster_fits(uint32_t tokens, uint32_t experts) {
+    return tokens > 256 && experts <= static_cast<uint32_t>(kPrologueThreads) && cluster_smem(tokens, experts) <= 200 * 1024;
+}
+static int launch_tables_cluster(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
+                                 uint32_t* token_map, uint32_t* counts, uint32_t* tasks, uint32_t* offsets, uint32_t* error, cudaStream_t st) {
+    const size_t smem = cluster_smem(tokens, experts);
+    static thread_local SmemAttrCache configured;
+    TSP_CUDA(ensure_dynamic_smem(tables_cluster_kernel, configured, smem));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kTablesCluster); cfg.blockDim = dim3(kPrologueThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = kTablesCluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 2;
+    TSP_CUDA(cudaLaunchKernelEx(&cfg, tables_cluster_kernel, ids, tokens, experts, selected, tile, first, local_only, cluster_words(tokens), token_map, counts, tasks,
+                                offsets, error));
+    return TSP_OK;
+}
+
 // The one-block form covers up to 1024 rows and experts whose masks fit 96 KB of shared memory.
 static bool tables_fit(uint32_t tokens, uint32_t experts) {
     return tokens >= 1 && tokens <= 1024 && experts <= static_cast<uint32_t>(kPrologueThreads) && static_cast<uint64_t>(experts) * ((tokens + 31) / 32) * 4 <= 96 * 1024;
@@ -679,15 +807,23 @@ int launch_route(const float* logits, uint64_t stride, uint32_t tokens, uint32_t
     return TSP_OK;
 }
 
+int launch_route_offsets(const uint32_t*, uint32_t, uint32_t*, cudaStream_t);
+
+// offsets (optional): the first permuted position of every expert and the grouped launches' counters, as launch_route_offsets writes them
 int launch_permute(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
-                   uint32_t* token_map, uint32_t* counts, uint32_t* tasks, uint32_t* error, cudaStream_t st) {
-    if (tables_fit(tokens, experts)) return launch_tables(ids, tokens, experts, selected, tile, first, local_only, token_map, counts, tasks, error, st);
+                   uint32_t* token_map, uint32_t* counts, uint32_t* tasks, uint32_t* error, cudaStream_t st, uint32_t* offsets) {
+    if (cluster_fits(tokens, experts))
+        return launch_tables_cluster(ids, tokens, experts, selected, tile, first, local_only, token_map, counts, tasks, offsets, error, st);
+    if (tables_fit(tokens, experts)) {
+        if (int rc = launch_tables(ids, tokens, experts, selected, tile, first, local_only, token_map, counts, tasks, error, st)) return rc;
+        return offsets ? launch_route_offsets(counts, experts, offsets, st) : TSP_OK;
+    }
     TSP_CUDA(launch_pdl(grouped_routes_kernel, dim3((experts + kPermuteExperts - 1) / kPermuteExperts), dim3(kPermuteThreads), 0, st, ids, tokens, experts, selected, first, local_only, token_map, counts, error));
     TSP_CUDA(cudaGetLastError());
     const uint32_t bound = static_cast<uint32_t>((static_cast<uint64_t>(tokens) * selected) / tile + experts);
     TSP_CUDA(launch_pdl(grouped_tasks_kernel, dim3(1), dim3(256), (experts + 1) * sizeof(uint32_t), st, counts, tokens, experts, selected, tile, bound, local_only, tasks, error));
     TSP_CUDA(cudaGetLastError());
-    return TSP_OK;
+    return offsets ? launch_route_offsets(counts, experts, offsets, st) : TSP_OK;
 }
 
 int launch_combine(const void* routed, uint64_t routed_stride, uint32_t routed_f16, const float* weights, const float* shared,
