@@ -45,6 +45,8 @@ int launch_combine(const void*, uint64_t, uint32_t, const float*, const float*, 
                    uint32_t, uint32_t, uint32_t, float*, uint64_t, void*, uint64_t, uint32_t*, cudaStream_t);
 int launch_decode_prologue(const float*, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t, uint32_t*, float*, uint32_t*, uint32_t*,
                            uint32_t*, const void*, uint64_t, float*, uint64_t, uint32_t, DecodeDense*, uint32_t*, cudaStream_t);
+int launch_prefill_route(const float*, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t*, float*, const void*, uint64_t, uint32_t, uint32_t, void*,
+                         uint64_t, uint32_t*, cudaStream_t);
 int launch_f16_to_f32(const void*, uint64_t, float*, uint64_t, uint32_t, uint32_t, cudaStream_t);
 int launch_dequant(uint32_t, uint32_t, const uint8_t*, uint64_t, float*, uint32_t*, cudaStream_t);
 int launch_gemv(const tsp_matrix_set*, const tsp_matrix_set*, bool, const float*, uint64_t, uint32_t, uint32_t,
@@ -593,12 +595,28 @@ int tsp_moe_route_offsets(const uint32_t* d_counts, uint32_t experts, uint32_t* 
     return launch_route_offsets(d_counts, experts, d_offsets, static_cast<cudaStream_t>(stream));
 }
 
-int tsp_moe_rows_f16k(const void* d_x, uint64_t x_stride, uint32_t x_dtype, uint32_t rows, uint32_t cols, void* d_xk, uint64_t xk_stride,
-                      uint32_t* d_error, void* stream) {
+}  // extern "C"
+
+static int check_rows_f16k(const void* d_x, uint64_t x_stride, uint32_t x_dtype, uint32_t rows, uint32_t cols, void* d_xk, uint64_t xk_stride) {
     TSP_REQUIRE(x_dtype <= 1 && rows >= 1 && cols >= 8 && cols % 8 == 0, "K-ordered rows: invalid shape or dtype");
     if (int rc = check_rows(d_x, x_stride, cols, x_dtype ? 2 : 4, "K-ordered rows input")) return rc;
     if (int rc = check_rows(d_xk, xk_stride, cols, 2, "K-ordered rows output")) return rc;
     TSP_REQUIRE(!overlap(d_x, rows * x_stride, d_xk, rows * xk_stride), "K-ordered rows: input and output overlap");
+    return TSP_OK;
+}
+static int check_route(const void* d_logits, uint64_t stride, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t mode, const void* d_ids, const void* d_weights) {
+    TSP_REQUIRE(d_logits && d_ids && d_weights, "route: null buffer");
+    TSP_REQUIRE(tokens >= 1, "route: no token rows");
+    TSP_REQUIRE(experts >= 1 && experts <= 4096 && selected >= 1 && selected <= 64 && selected <= experts && mode <= 1, "route: invalid router shape/mode");
+    TSP_REQUIRE(stride >= static_cast<uint64_t>(experts) * 4 && stride % 4 == 0, "route: logits stride too small");
+    return TSP_OK;
+}
+
+extern "C" {
+
+int tsp_moe_rows_f16k(const void* d_x, uint64_t x_stride, uint32_t x_dtype, uint32_t rows, uint32_t cols, void* d_xk, uint64_t xk_stride,
+                      uint32_t* d_error, void* stream) {
+    if (int rc = check_rows_f16k(d_x, x_stride, x_dtype, rows, cols, d_xk, xk_stride)) return rc;
     return launch_rows_f16k(d_x, x_stride, x_dtype, rows, cols, d_xk, xk_stride, d_error, static_cast<cudaStream_t>(stream));
 }
 
@@ -762,8 +780,15 @@ int tsp_moe_layer_prefill(const tsp_moe_weights* w, const tsp_moe_prefill_scratc
     TSP_REQUIRE(s->d_ids && s->d_weights && s->d_routed && s->d_shared_out && s->d_token_map && s->d_counts && s->d_tasks && ps->d_xk &&
                 ps->d_xp && ps->d_hp && ps->d_offsets && ps->d_s_hp, "prefill layer: incomplete scratch");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (int rc = tsp_moe_rows_f16k(d_x, x_stride, x_dtype, tokens, channels, ps->d_xk, channels * 2ull, d_error, st)) return rc;
-    if (int rc = tsp_moe_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_error, st)) return rc;
+    if (int rc = check_rows_f16k(d_x, x_stride, x_dtype, tokens, channels, ps->d_xk, channels * 2ull)) return rc;
+    if (int rc = check_route(d_logits, logits_stride, tokens, experts, selected, mode, s->d_ids, s->d_weights)) return rc;
+    const int routed = launch_prefill_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_x, x_stride, x_dtype, channels,
+                                            ps->d_xk, channels * 2ull, d_error, st);
+    if (routed < 0) return routed;
+    if (routed) {
+        if (int rc = launch_rows_f16k(d_x, x_stride, x_dtype, tokens, channels, ps->d_xk, channels * 2ull, d_error, st)) return rc;
+        if (int rc = launch_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_error, st)) return rc;
+    }
     if (int rc = permute(s->d_ids, tokens, experts, selected, TSP_GROUPED_TILE, s->d_token_map, s->d_counts, s->d_tasks, ps->d_offsets, d_error, st)) return rc;
     if (int rc = tsp_moe_gather_rows16(ps->d_xk, channels * 2ull, s->d_token_map, ps->d_offsets, experts, tokens, selected, channels, ps->d_xp,
                                        channels * 2ull, st)) return rc;
