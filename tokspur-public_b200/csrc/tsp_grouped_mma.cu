@@ -236,17 +236,22 @@ __device__ __forceinline__ ChunkScale chunk_scale(float d, float dmin, uint32_t 
 // binary16 pairs without byte shuffles.
 __device__ __forceinline__ void dequant8(uint32_t a, uint32_t b, const ChunkScale& cs, uint4& lo, uint4& hi) {
     const __half2 k1032 = __float2half2_rn(1032.f), k72 = __float2half2_rn(72.f);
-    const uint32_t src[4] = {a, a >> 8, b, b >> 8};
+    // byte pairs (0, 2) and (1, 3) under 0x64 / 0x54: the integer pipe takes two cycles an instruction and is what dequantising is bound by; a mask
+    // and an or of two constants came out as two instructions a pair
     uint32_t l[4], h[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t lw = (src[i] & 0x000f000fu) | 0x64006400u;     // 1024 + q
-        const uint32_t hw = (src[i] & 0x00f000f0u) | 0x54005400u;     //   64 + q
-        const __half2 ql = __hsub2(*reinterpret_cast<const __half2*>(&lw), k1032);   // q - 8, exact
-        const __half2 qh = __hsub2(*reinterpret_cast<const __half2*>(&hw), k72);
-        const __half2 wl = __hfma2(ql, cs.s_lo, cs.c_lo), wh = __hfma2(qh, cs.s_hi, cs.c_hi);
-        l[i] = *reinterpret_cast<const uint32_t*>(&wl);
-        h[i] = *reinterpret_cast<const uint32_t*>(&wh);
+    for (int i = 0; i < 2; ++i) {
+        const uint32_t src = i ? b : a, t = src & 0x0f0f0f0fu, u = src & 0xf0f0f0f0u;
+        const uint32_t lw[2] = {__byte_perm(t, 0x64646464u, 0x4240), __byte_perm(t, 0x64646464u, 0x4341)};   // 1024 + q
+        const uint32_t hw[2] = {__byte_perm(u, 0x54545454u, 0x4240), __byte_perm(u, 0x54545454u, 0x4341)};   //   64 + q
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const __half2 ql = __hsub2(*reinterpret_cast<const __half2*>(&lw[j]), k1032);   // q - 8, exact
+            const __half2 qh = __hsub2(*reinterpret_cast<const __half2*>(&hw[j]), k72);
+            const __half2 wl = __hfma2(ql, cs.s_lo, cs.c_lo), wh = __hfma2(qh, cs.s_hi, cs.c_hi);
+            l[2 * i + j] = *reinterpret_cast<const uint32_t*>(&wl);
+            h[2 * i + j] = *reinterpret_cast<const uint32_t*>(&wh);
+        }
     }
     lo = make_uint4(l[0], l[1], l[2], l[3]);
     hi = make_uint4(h[0], h[1], h[2], h[3]);
@@ -615,6 +620,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                 }
             }
             ok = gwait(&acc_full[ab], accph);
+            bool held = true;   // this warp still has to hand the accumulator back
             if (ok) {
                 tc_fence_after();
                 char* const obase = reinterpret_cast<char*>(shared ? p.sh_out : p.out);
@@ -631,6 +637,12 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                         uint32_t v[32];
                         tmem_ld32(taddr + j0, v);
                         tmem_ld_wait();
+                        if (b == 1 || j0 + 64 >= cnt) {   // the warp's last batch is in its registers: the accumulator is free
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&acc_empty[ab]);
+                            held = false;
+                        }
                         // Results leave through a per-warp transposition tile in shared memory: the accumulators arrive with a lane per
                         // weight row and a register per token column, the output rows want a lane per token and a run of weight rows
                         // (16-byte stores instead of one 2-byte store per value).
@@ -711,7 +723,7 @@ __global__ void __launch_bounds__(kGWarps * 32, 1) grouped_mma_kernel(const __gr
                 tc_fence_before();
             }
             __syncwarp();
-            if (lane == 0 && ok) mbar_arrive(&acc_empty[ab]);
+            if (lane == 0 && ok && held) mbar_arrive(&acc_empty[ab]);
             if (++ab == 2) { ab = 0; accph ^= 1u; }
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
