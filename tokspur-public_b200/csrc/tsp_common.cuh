@@ -176,6 +176,14 @@ __device__ __forceinline__ void mma_f16_16816_zero(float (&d)[4], uint32_t a0, u
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// Dot product of two FP32 rows by one warp: FMAs by lane, then a butterfly (every lane returns the sum)
+__device__ __forceinline__ float f32_dot_row(const float* w, const float* x, uint32_t cols, uint32_t lane) {
+    float acc = 0.f;
+    for (uint32_t c = lane; c < cols; c += 32) acc = fmaf(w[c], x[c], acc);
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    return acc;
+}
+
 // Branch-stable sigmoid / SiLU in FP32 (operators.cpp:28-36 restated for float).
 __device__ __forceinline__ float stable_sigmoid(float v) {
     if (v >= 0.f) return 1.f / (1.f + expf(-v));

@@ -724,29 +724,28 @@ combine_kernel(const void* routed, uint64_t routed_stride, const float* weights,
 }
 
 // ---------------------------------------------------------------------------------------------
-// F32 matrix-vector product for the router projections: one warp per (matrix row, token), FP32 FMA + tree sum.
+// F32 matrix-vector product for the router projections: one warp per (matrix row, token), FP32 FMA + tree sum (f32_dot_row). `extra`
+// (optional): one more matrix row with an output array of its own, the last row of every token.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-gemv_f32_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, uint64_t x_stride, uint32_t tokens,
-                float* __restrict__ out, uint64_t out_stride, uint32_t* error) {
+gemv_f32_kernel(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x, uint64_t x_stride, uint32_t tokens,
+                float* __restrict__ out, uint64_t out_stride, float* __restrict__ extra_out, uint32_t* error) {
     pdl_launch_dependents();
     pdl_wait();
 
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= rows * tokens) return;
-    const uint32_t token = warp / rows, row = warp % rows;
-    const float* wr = w + static_cast<uint64_t>(row) * cols;
-    const float* xr = reinterpret_cast<const float*>(reinterpret_cast<const char*>(x) + token * x_stride);
-    float acc = 0.f;
-    for (uint32_t c = lane; c < cols; c += 32) acc = fmaf(wr[c], xr[c], acc);
-    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, all = rows + (extra ? 1u : 0u);
+    if (warp >= all * tokens) return;
+    const uint32_t token = warp / all, row = warp % all;
+    const float acc = f32_dot_row(row < rows ? w + static_cast<uint64_t>(row) * cols : extra,
+                                  reinterpret_cast<const float*>(reinterpret_cast<const char*>(x) + token * x_stride), cols, lane);
     if (lane == 0) {
         if (!finite_f32(acc)) raise_error(error, TSP_ERR_NONFINITE);
-        reinterpret_cast<float*>(reinterpret_cast<char*>(out) + token * out_stride)[row] = acc;
+        if (row < rows) reinterpret_cast<float*>(reinterpret_cast<char*>(out) + token * out_stride)[row] = acc;
+        else extra_out[token] = acc;
     }
 }
 
-int launch_router_mma(const float*, uint32_t, uint32_t, const float*, uint64_t, uint32_t, float*, uint64_t, uint32_t*, cudaStream_t);
+int launch_router_mma(const float*, uint32_t, uint32_t, const float*, const float*, uint64_t, uint32_t, float*, uint64_t, float*, uint32_t*, cudaStream_t);
 // Fewest token rows for the tensor-core product, from 512 matrix rows: its one wave of blocks takes 18 us at 1024 columns and 28 us at 2048
 // whatever the batch; one warp per output takes 15 us at 63 rows of 1024 columns, 20 us at 64 and 28 us at 95 rows of 2048. The warp form scales
 // with matrix rows x token rows (64 matrix rows: 8 us at 95 token rows of 2048 columns), the other does not (28 us at 96), so a matrix of fewer
@@ -755,15 +754,10 @@ constexpr uint32_t kRouterMmaTokens = 96;
 
 int launch_gemv_f32(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x, uint64_t x_stride, uint32_t tokens, float* out,
                     uint64_t out_stride, float* extra_out, uint32_t* error, cudaStream_t st) {
-    if (tokens >= kRouterMmaTokens) {
-        // the extra row (one dot product per token) takes its own small launch
-        if (int rc = launch_router_mma(w, rows, cols, x, x_stride, tokens, out, out_stride, error, st)) return rc;
-        if (extra) TSP_CUDA(launch_pdl(gemv_f32_kernel, dim3(static_cast<unsigned>((tokens + 7) / 8)), dim3(256), 0, st, extra, 1u, cols, x, x_stride, tokens, extra_out, sizeof(float), error));
-        return TSP_OK;
-    }
-    const uint64_t warps = static_cast<uint64_t>(rows) * tokens;
-    TSP_CUDA(launch_pdl(gemv_f32_kernel, dim3(static_cast<unsigned>((warps + 7) / 8)), dim3(256), 0, st, w, rows, cols, x, x_stride, tokens, out, out_stride, error));
-    if (extra) TSP_CUDA(launch_pdl(gemv_f32_kernel, dim3(static_cast<unsigned>((tokens + 7) / 8)), dim3(256), 0, st, extra, 1u, cols, x, x_stride, tokens, extra_out, sizeof(float), error));
+    if (tokens >= kRouterMmaTokens) return launch_router_mma(w, rows, cols, extra, x, x_stride, tokens, out, out_stride, extra_out, error, st);
+    const uint64_t warps = (static_cast<uint64_t>(rows) + (extra ? 1u : 0u)) * tokens;
+    TSP_CUDA(launch_pdl(gemv_f32_kernel, dim3(static_cast<unsigned>((warps + 7) / 8)), dim3(256), 0, st, w, rows, cols, extra, x, x_stride, tokens, out, out_stride, extra_out,
+                        error));
     return TSP_OK;
 }
 

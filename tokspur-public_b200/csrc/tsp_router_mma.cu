@@ -82,9 +82,23 @@ __device__ __forceinline__ float4 rm_load4(const float* row, uint32_t k, uint32_
 
 template <bool V>
 __global__ void __launch_bounds__(kRmThreads, 1)
-router_mma_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, uint64_t x_stride, uint32_t tokens, float* __restrict__ out,
-                  uint64_t out_stride, uint32_t* error) {
+router_mma_kernel(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x, uint64_t x_stride, uint32_t tokens, float* __restrict__ out,
+                  uint64_t out_stride, float* __restrict__ extra_out, uint32_t* error) {
     pdl_launch_dependents();
+    // The extra row (the shared expert's gate, one dot product per token): the blocks past the matrix's columns of blocks, a warp per token in turn,
+    // with the sums of gemv_f32_kernel. A launch of its own behind this one took 6 to 8 us; one wave of this launch leaves SMs idle.
+    if (blockIdx.x * kRmN >= rows) {
+        pdl_wait();
+        const uint32_t end = min(tokens, (blockIdx.y + 1) * kRmM);
+        for (uint32_t t = blockIdx.y * kRmM + (threadIdx.x >> 5); t < end; t += kRmThreads / 32) {
+            const float acc = f32_dot_row(extra, reinterpret_cast<const float*>(reinterpret_cast<const char*>(x) + static_cast<uint64_t>(t) * x_stride), cols, threadIdx.x & 31u);
+            if ((threadIdx.x & 31u) == 0) {
+                if (!finite_f32(acc)) raise_error(error, TSP_ERR_NONFINITE);
+                extra_out[t] = acc;
+            }
+        }
+        return;
+    }
     extern __shared__ uint8_t rm_raw[];
     uint8_t* sm = rm_raw + ((1024u - (smem_u32(rm_raw) & 1023u)) & 1023u);
     uint64_t *full = reinterpret_cast<uint64_t*>(sm), *empty = full + kRmStages, *main_full = empty + kRmStages, *main_empty = main_full + 2;
@@ -261,20 +275,20 @@ router_mma_kernel(const float* w, uint32_t rows, uint32_t cols, const float* x, 
 }
 
 template <bool V>
-static int launch_router_mma_t(const float* w, uint32_t rows, uint32_t cols, const float* x, uint64_t x_stride, uint32_t tokens, float* out,
-                               uint64_t out_stride, uint32_t* error, cudaStream_t st) {
+static int launch_router_mma_t(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x, uint64_t x_stride, uint32_t tokens, float* out,
+                               uint64_t out_stride, float* extra_out, uint32_t* error, cudaStream_t st) {
     static thread_local SmemAttrCache configured;   // per kernel instantiation, keyed by device
     TSP_CUDA(ensure_dynamic_smem(router_mma_kernel<V>, configured, kRmSmem));
-    const dim3 grid((rows + kRmN - 1) / kRmN, (tokens + kRmM - 1) / kRmM);
-    TSP_CUDA(launch_pdl(router_mma_kernel<V>, grid, dim3(kRmThreads), kRmSmem, st, w, rows, cols, x, x_stride, tokens, out, out_stride, error));
+    const dim3 grid((rows + kRmN - 1) / kRmN + (extra ? 1u : 0u), (tokens + kRmM - 1) / kRmM);
+    TSP_CUDA(launch_pdl(router_mma_kernel<V>, grid, dim3(kRmThreads), kRmSmem, st, w, rows, cols, extra, x, x_stride, tokens, out, out_stride, extra_out, error));
     return TSP_OK;
 }
 
-int launch_router_mma(const float* w, uint32_t rows, uint32_t cols, const float* x, uint64_t x_stride, uint32_t tokens, float* out,
-                      uint64_t out_stride, uint32_t* error, cudaStream_t st) {
+int launch_router_mma(const float* w, uint32_t rows, uint32_t cols, const float* extra, const float* x, uint64_t x_stride, uint32_t tokens, float* out,
+                      uint64_t out_stride, float* extra_out, uint32_t* error, cudaStream_t st) {
     const bool v4 = cols % 4 == 0 && (reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x) | x_stride) % 16 == 0;
-    if (v4) return launch_router_mma_t<true>(w, rows, cols, x, x_stride, tokens, out, out_stride, error, st);
-    return launch_router_mma_t<false>(w, rows, cols, x, x_stride, tokens, out, out_stride, error, st);
+    if (v4) return launch_router_mma_t<true>(w, rows, cols, extra, x, x_stride, tokens, out, out_stride, extra_out, error, st);
+    return launch_router_mma_t<false>(w, rows, cols, extra, x, x_stride, tokens, out, out_stride, extra_out, error, st);
 }
 
 }  // namespace tsp
