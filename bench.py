@@ -241,9 +241,9 @@ def decode_record(args, dev, T, layers, etype, layout, full: bool):
            "timed_repeats": repeats, "unique_experts": U, "layer_algorithmic_bytes": layer_bytes,
            "layer_hbm_gbs": layer_bytes / (ms * 1e-3) / 1e9, "layer_hbm_frac": layer_bytes / (ms * 1e-3) / 1e9 / hbm_peak,
            "layer_tflops": T * (SELECTED + 1) * FLOPS_PER_ROUTE / (ms * 1e-3) / 1e12,
-           # routing, tables, gate-up, down, mixture; experts that cannot take the shared expert into their launches (Q8_0, Q5_K) run it
-           # in a launch of its own beside each projection
-           "launches_per_step": 5 if etype == formats.Q4_K else 7}
+           # routing, tables, gate-up, down, mixture (a dense Q8_0 shared expert beside Q8_0 or Q5_K experts works in the first two); up to eight rows
+           # on Q4_K experts are routed by the gate-up launch
+           "launches_per_step": 3 if etype == formats.Q4_K and T <= 8 else 5}
     if not full:
         return rec, None
     # ---- the dominant launch alone, back to back over the rotating layers (tables of batch 0; the weights change every launch)
@@ -386,7 +386,7 @@ def prefill_record(args, dev, layers, T):
            "timed_repeats": repeats, "layer_tflops": layer_flops / (ms * 1e-3) / 1e12, "layer_frac_of_bf16_peak": layer_flops / (ms * 1e-3) / 1e12 / tf_peak,
            "gate_up_launch_tflops": gu_flops / (stages["gate_up_ms"] * 1e-3) / 1e12,
            "gate_up_launch_frac_of_bf16_peak": gu_flops / (stages["gate_up_ms"] * 1e-3) / 1e12 / tf_peak, "peak_tflops": tf_peak, "peak_kind": peak_kind,
-           "stage_ms": stages, "launches_per_step": 9 + 2 * int(layers[0].shared_type != layers[0].type), "router": "N(0,1) + Zipf(1.1) per-expert bias",
+           "stage_ms": stages, "launches_per_step": 6 + 2 * int(layers[0].shared_type != layers[0].type), "router": "N(0,1) + Zipf(1.1) per-expert bias",
            "h2d_bytes_per_step": T * CHANNELS * 2 + T * EXPERTS * 4, "d2h_bytes_per_step": T * CHANNELS * 2}
     cpu = None
     if args.cpu_tokens != 0:
@@ -618,7 +618,7 @@ def run_ours(args):
                              "f16 operands, f32 accumulate", {"router": rec["router"], "l2_policy": "inputs larger than L2: 0.93 GB of weights and 0.4 GB of intermediates per step"})
             line.update({"e2e": {"value": rec["e2e_tokens_per_s"], "unit": "tokens/s", "ms_per_step": rec["e2e_ms_per_step"],
                                  "h2d_bytes_per_step": rec["h2d_bytes_per_step"], "d2h_bytes_per_step": rec["d2h_bytes_per_step"]},
-                         "gpu_launches": 9 * max(4, args.steps // 4),
+                         "gpu_launches": rec["launches_per_step"] * max(4, args.steps // 4),
                          "roofline": {"bound": "tensor", "kernel": "grouped_mma_kernel<gate-up> (routed experts + shared expert, tcgen05)", "achieved": rec["gate_up_launch_tflops"],
                                       "peak": tf_peak, "unit": "TFLOP/s", "frac": rec["gate_up_launch_frac_of_bf16_peak"], "peak_kind": peak_kind, "traffic": 471.3e6 if Tp == 4096 and p_layout == formats.PLANAR and sh_type is None else None,
                                       "traffic_source": "profiles/grouped_mma_prefill_T4096.md (ncu: DRAM bytes read and written by the gate-up launch)",

@@ -381,7 +381,7 @@ int tsp_moe_staged_f16(const tsp_matrix_set* m, uint32_t expert, void* d_out, vo
  * path (graph.mm:9293-9420). Weights: Q4_K, Pack v3 planar or plain GGUF super-blocks, hidden a multiple of 64 and channels
  * of 256. A shared expert in the routed experts' form rides in the routed launches; in another form (dense Q8_0 GGUF blocks
  * beside Q4_K experts, as the reference's model has it) it is computed by tsp_dense_mm_swiglu / tsp_dense_mm in launches of
- * its own (11 launches instead of 9). Arguments as tsp_moe_layer_decode; `tokens` <= s->base.capacity.
+ * its own (8 launches instead of 6). Arguments as tsp_moe_layer_decode; `tokens` <= s->base.capacity.
  * Caller-owned scratch, all device memory, nothing has to start at zero:
  *   base: as for the decode layer, except d_tasks sized tsp_moe_tasks_words(capacity, experts, selected, TSP_GROUPED_TILE);
  *         d_routed is used as binary16 rows [capacity*selected x channels]; d_hidden, d_shared_hidden and d_x32 are not

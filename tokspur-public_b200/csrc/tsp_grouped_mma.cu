@@ -19,7 +19,8 @@
 //     about 100 cycles each (operands moved to uniform registers under a loop over the lanes the compiler cannot rule out): with
 //     the rest in place, 470 k of the 731 k cycles of the 4096-row gate-up launch; 485 k in all without it.
 //   * Measured (layer with 512 experts of 512 x 2048, ten per token, Zipf loads, whole layer): 4096 rows 761 -> 650 us, 160 rows
-//     179 -> 112 us, 1003 rows (dense Q8_0 shared expert; 85 us of it in the routing tables) 437 -> 262 us.
+//     179 -> 112 us, 1003 rows (dense Q8_0 shared expert; 85 us of it in the routing tables) 437 -> 262 us. Since then (codes by permutes, accumulators handed back
+//     when loaded, tables by a cluster, routing beside the row copy) 605, 103 and 244 us.
 //   * Gate-up items hold 64 hidden units as 128 A rows: inside every group of 32 rows (one tensor-memory lane quarter)
 //     rows 0..15 are gate rows and rows 16..31 the up rows of the same 16 units, so SwiGLU is a lane exchange inside one
 //     warp and one accumulator serves both matrices.
