@@ -157,6 +157,26 @@ def test_tables_of_large_batches(oracle, tokens, experts, selected, first, local
     assert np.array_equal(tasks.cpu().numpy().view(np.uint32), want_tasks)
 
 
+# Few experts: slices of up to 65536 rows per block of the cluster, all of one expert's (the running counts are 16 bits), and the first batch beyond
+@pytest.mark.parametrize("tokens", [524288, 524289, 600000])
+@pytest.mark.parametrize("experts", [1, 16])
+def test_tables_of_very_large_batches(tokens, experts):
+    selected = 1 if experts == 1 else 2
+    ids = np.zeros((tokens, selected), dtype=np.int32)   # every row names expert 0
+    ids[:, 1:] = 1 + np.random.default_rng(tokens).integers(0, max(experts - 1, 1), (tokens, selected - 1))
+    dids, e = torch.from_numpy(ids).cuda(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    tmap, counts = torch.full((experts * tokens,), -7, dtype=torch.int32, device="cuda"), torch.empty(experts, dtype=torch.int32, device="cuda")
+    tasks = torch.empty(int(capi.lib().tsp_moe_tasks_words(tokens, experts, selected, 256)), dtype=torch.int32, device="cuda")
+    capi.call("tsp_moe_permute", dids.data_ptr(), tokens, experts, selected, 256, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(), e.data_ptr(), L.stream_ptr())
+    torch.cuda.synchronize()
+    assert int(e.item()) == 0
+    want_counts = np.bincount(ids.reshape(-1), minlength=experts)
+    assert np.array_equal(counts.cpu().numpy(), want_counts)
+    got = tmap.cpu().numpy().reshape(experts, tokens)
+    for i in range(experts):
+        assert np.array_equal(got[i, :want_counts[i]], np.flatnonzero(ids.reshape(-1) == i)) and (got[i, want_counts[i]:] == -7).all()
+
+
 @pytest.mark.parametrize("bad", ["twice", "range"])
 def test_tables_of_large_batches_report_bad_ids(bad):
     tokens, experts, selected = 700, 64, 4

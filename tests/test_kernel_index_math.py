@@ -3,6 +3,7 @@ tests do not reach (group counts that are not powers of two: the reference model
 (row, group) pair of a block's rows is visited by exactly one lane, the lanes that share a row form one aligned run whose
 width the shuffle reduction covers, and the staged activation index stays inside the shared-memory extent the host sizes."""
 import os
+import re
 
 import numpy as np
 import pytest
@@ -172,3 +173,28 @@ def test_topk_merge_candidates_pass_a_tight_bound(vocab):
         bound = np.sort(lanes, axis=1)[:, -8].min()                           # the smallest of the warps' eighth-largest
         passed = int((key >= max(bound, np.finfo(np.float32).min)).sum())
         assert min(64, vocab) <= passed <= limit
+
+
+def cluster_admits(tokens, experts):
+    """csrc/tsp_route.cu, cluster_fits: the batches whose tables one cluster of eight blocks builds, and a block's mask words per expert."""
+    src = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "tokspur-public_b200", "csrc", "tsp_route.cu")).read()
+    limit = re.search(r"constexpr uint32_t kClusterWords = (\d+);", src)
+    words = ((tokens + 7) // 8 + 31) // 32
+    return tokens > 256 and experts <= 1024 and (limit is None or words <= int(limit.group(1))) and experts * (8 + (words | 1) * 6) <= 200 * 1024, words
+
+
+@pytest.mark.parametrize("experts", [1, 2, 4, 8, 16, 17, 64, 512, 1024])
+def test_running_counts_of_the_routing_tables_fit_16_bits(experts):
+    """Rows before each mask word of a block, one expert named by every row: what the kernel stores in 16 bits, at the largest batch that takes it."""
+    lo, hi = 257, 1 << 24
+    if not cluster_admits(lo, experts)[0]:
+        return
+    while hi - lo > 1:   # words grow with the batch: the rule changes over once
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if cluster_admits(mid, experts)[0] else (lo, mid)
+    words = cluster_admits(lo, experts)[1]
+    rows = min(words * 32, lo)   # of the first block
+    mask = np.ones(words * 32, dtype=np.int64)
+    mask[rows:] = 0
+    before = np.concatenate([[0], np.cumsum(mask.reshape(words, 32).sum(1))[:-1]])
+    assert np.array_equal(before.astype(np.uint16), before)

@@ -447,8 +447,11 @@ tables_cluster_kernel(const uint32_t* ids, uint32_t tokens, uint32_t experts, ui
 
 static uint32_t cluster_words(uint32_t tokens) { return ((tokens + kTablesCluster - 1) / kTablesCluster + 31) / 32; }
 static size_t cluster_smem(uint32_t tokens, uint32_t experts) { return static_cast<size_t>(experts) * (8u + (cluster_words(tokens) | 1u) * 6u); }
+// The running counts are 16 bits: before a block's last word lie at most 32 * (words - 1) rows, so 2048 words at most (few experts leave shared memory for more)
+constexpr uint32_t kClusterWords = 2048;
+static_assert(32u * (kClusterWords - 1u) <= 0xffffu, "running counts of the cluster's tables");
 static bool cluster_fits(uint32_t tokens, uint32_t experts) {
-    return tokens > 256 && experts <= static_cast<uint32_t>(kPrologueThreads) && cluster_smem(tokens, experts) <= 200 * 1024;
+    return tokens > 256 && experts <= static_cast<uint32_t>(kPrologueThreads) && cluster_words(tokens) <= kClusterWords && cluster_smem(tokens, experts) <= 200 * 1024;
 }
 static int launch_tables_cluster(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
                                  uint32_t* token_map, uint32_t* counts, uint32_t* tasks, uint32_t* offsets, uint32_t* error, cudaStream_t st) {
