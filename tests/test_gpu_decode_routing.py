@@ -91,3 +91,60 @@ def test_nonfinite_logits_are_reported(tokens):
         outs.append(out.cpu().numpy())
     assert np.array_equal(outs[0][:tokens - 1], outs[1][:tokens - 1])
     assert not s.weights.cpu().numpy()[(tokens - 1) * selected:tokens * selected].any()
+
+
+def layer_rows(dl, shape, tokens, x, logits, out, share=None):
+    """Output rows of one call; share(scratch): gives some of the scratch's pointers other buffers' memory."""
+    s = L.Scratch(*shape, tokens, DEV)
+    if share:
+        share(s)
+    L.moe_layer_decode(dl, s, x, logits, out)
+    torch.cuda.synchronize()
+    assert s.error_word() == 0
+    return out.clone()
+
+
+# Up to eight rows the mixture reads the caller's binary16 rows, in slices of a row; nine rows take the FP32 copy. `beside`: output rows between
+# the input rows of one buffer
+@pytest.mark.parametrize("tokens", [1, 8, 9])
+@pytest.mark.parametrize("place", ["same", "shifted", "beside"])
+def test_output_in_the_input_rows(tokens, place):
+    shape = channels, hidden, experts, selected = 2048, 256, 16, 4
+    dl = L.SynthDeviceLayer(9, channels, hidden, experts, formats.Q4_K, formats.PLANAR, DEV)
+    rows = torch.from_numpy(synth.normal(36, (tokens, channels), 1.0)).to(DEV).half()
+    logits = torch.from_numpy(synth.router_logits(37, tokens, experts)).to(DEV)
+    want = layer_rows(dl, shape, tokens, rows, logits, torch.empty_like(rows))
+    for _ in range(20):
+        buf = torch.empty(tokens * 2 * channels + channels, dtype=torch.float16, device=DEV)
+        if place == "beside":
+            both = buf[:tokens * 2 * channels].view(tokens, 2 * channels)
+            x, out = both[:, :channels], both[:, channels:]
+        else:
+            at = 8 if place == "shifted" else 0
+            x, out = (buf[o:o + tokens * channels].view(tokens, channels) for o in (0, at))
+        x.copy_(rows)
+        assert torch.equal(layer_rows(dl, shape, tokens, x, logits, out), want)
+
+
+# What one launch does now was done in turn by several: buffers that those did not need at the same time may be the same memory
+@pytest.mark.parametrize("tokens", [3, 8])
+@pytest.mark.parametrize("shared", ["rows in routed", "rows in shared_out", "ids in hidden", "logits in hidden", "logits in shared_hidden"])
+def test_buffers_that_share_memory(tokens, shared):
+    shape = channels, hidden, experts, selected = 1024, 256, 512, 10
+    dl = L.SynthDeviceLayer(9, channels, hidden, experts, formats.Q4_K, formats.PLANAR, DEV)
+    x = torch.from_numpy(synth.normal(38, (tokens, channels), 1.0)).to(DEV).half()
+    logits = torch.from_numpy(synth.router_logits(39, tokens, experts)).to(DEV)
+    want = layer_rows(dl, shape, tokens, x, logits, torch.empty_like(x))
+    own, other = shared.split(" in ")
+    room = torch.zeros(max(tokens * selected * channels, tokens * experts), device=DEV)
+    if own == "rows":
+        x = room.view(torch.float16)[:x.numel()].view_as(x).copy_(x)
+    elif own == "logits":
+        logits = room[:logits.numel()].view_as(logits).copy_(logits)
+
+    def share(s):
+        setattr(s.c, "d_" + other, room.data_ptr())
+        if own == "ids":
+            s.c.d_ids = room.data_ptr()
+
+    assert torch.equal(layer_rows(dl, shape, tokens, x, logits, torch.empty_like(x), share), want)

@@ -98,6 +98,19 @@ static bool overlap(const void* a, uint64_t abytes, const void* b, uint64_t bbyt
     const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
     return x < y + bbytes && y < x + abytes;
 }
+// Strided rows: rows of one buffer may lie between those of the other
+static bool rows_overlap(const void* a, uint64_t a_stride, uint64_t a_row, const void* b, uint64_t b_stride, uint64_t b_row, uint64_t rows) {
+    if (!overlap(a, (rows - 1) * a_stride + a_row, b, (rows - 1) * b_stride + b_row)) return false;
+    if (a_stride != b_stride) return true;
+    const uint64_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b), d = y >= x ? (y - x) % a_stride : (a_stride - (x - y) % a_stride) % a_stride;
+    return d < a_row || d + b_row > a_stride;
+}
+struct Span { const void* p; uint64_t bytes; };
+template <size_t N>
+static bool apart(const void* p, uint64_t bytes, const Span (&from)[N]) {
+    for (const Span& s : from) if (overlap(p, bytes, s.p, s.bytes)) return false;
+    return true;
+}
 
 }  // namespace tsp
 
@@ -508,10 +521,25 @@ int tsp_moe_layer_decode(const tsp_moe_weights* w, const tsp_moe_scratch* s, con
                           w->shared_up.cols == channels && w->shared_gate.expert_stride == w->shared_up.expert_stride && w->shared_gate.split == w->shared_up.split &&
                           channels % 16 == 0 && aligned16(s->d_shared_hidden) && aligned16(s->d_shared_out) && !overlap(d_x, x_bytes, s->d_shared_hidden, h_bytes) &&
                           (!s->d_x32 || !overlap(s->d_x32, o_bytes, s->d_shared_hidden, h_bytes)) && !overlap(s->d_shared_hidden, h_bytes, s->d_shared_out, o_bytes);
-    // up to eight rows on Q4_K experts: the gate-up launch routes the batch itself (binary16 rows are then read as they are)
+    // up to eight rows on Q4_K experts: the gate-up launch routes the batch itself (binary16 rows are then read as they are). It reads logits and rows while
+    // it writes what separate launches write later, and the mixture, a block per slice of a row, reads binary16 rows where it read their FP32 copy: a caller
+    // whose buffers share memory (output rows in the input rows, say) gets the separate launches.
+    const uint64_t routes = static_cast<uint64_t>(tokens) * selected, x_elem = x_dtype == 1 ? 2 : 4, out_elem = out_dtype == 1 ? 2 : 4;
+    const Span x_span{d_x, (tokens - 1) * x_stride + channels * x_elem}, logits_span{d_logits, (tokens - 1) * logits_stride + experts * 4ull};
+    const Span written[] = {{s->d_ids, routes * 4}, {s->d_weights, routes * 4}, {s->d_token_map, static_cast<uint64_t>(experts) * tokens * 4}, {s->d_counts, experts * 4ull},
+                            {s->d_tasks, tsp_moe_tasks_words(tokens, experts, selected, TSP_GEMV_TILE) * 4}, {s->d_hidden, routes * hidden * 4}, {s->d_shared_hidden, h_bytes}};
+    const Span later[] = {{s->d_routed, routes * channels * 4}, {s->d_shared_out, o_bytes}, {s->d_shared_logit, s->d_shared_logit ? tokens * 4ull : 0}};
+    auto own_memory = [&] {
+        for (const Span* a = written; a != written + sizeof written / sizeof *written; ++a) {
+            if (overlap(a->p, a->bytes, x_span.p, x_span.bytes) || overlap(a->p, a->bytes, logits_span.p, logits_span.bytes)) return false;
+            for (const Span* b = written; b != a; ++b) if (overlap(a->p, a->bytes, b->p, b->bytes)) return false;
+        }
+        return x_dtype == 0 || !w->d_shared_router ||
+               (apart(x_span.p, x_span.bytes, later) && !rows_overlap(d_x, x_stride, channels * x_elem, d_out, out_stride, channels * out_elem, tokens));
+    };
     int fused = 1;
     bool gated = false;
-    if (tokens <= TSP_GEMV_TILE && experts <= 512 && normalize && w->gate.type == TSP_TYPE_Q4_K) {
+    if (tokens <= TSP_GEMV_TILE && experts <= 512 && normalize && w->gate.type == TSP_TYPE_Q4_K && own_memory()) {
         const GemvRoute route{d_logits, logits_stride, selected, mode, s->d_ids, s->d_weights, s->d_token_map, s->d_counts, s->d_tasks};
         const int rc = gate_up_shared_launch(&w->gate, &w->up, &w->shared_gate, &w->shared_up, x_dtype == 1 ? s->d_x32 : x32, x32_stride, x_dtype == 1 ? d_x : nullptr,
                                              x_dtype == 1 ? x_stride : 0, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden, hidden * 4ull,
