@@ -510,36 +510,36 @@ int tsp_moe_layer_decode(const tsp_moe_weights* w, const tsp_moe_scratch* s, con
     uint64_t x32_stride = x_stride;
     if (x_dtype == 1) { x32 = s->d_x32; x32_stride = channels * 4ull; }
     const int exact = x_dtype == 1;
+    const uint64_t x_bytes = tokens * x_stride, h_bytes = tokens * hidden * 4ull, o_bytes = tokens * channels * 4ull, routes = static_cast<uint64_t>(tokens) * selected;
+    const uint64_t x_elem = x_dtype == 1 ? 2 : 4, out_elem = out_dtype == 1 ? 2 : 4;
+    // Two forms below do in one launch, or in another order, what a launch each did in turn: they write all of `written` while logits and rows are read. A caller
+    // whose buffers share memory that launches in turn do not need at the same time gets those.
+    const Span x_span{d_x, (tokens - 1) * x_stride + channels * x_elem}, logits_span{d_logits, (tokens - 1) * logits_stride + experts * 4ull};
+    const Span written[] = {{s->d_ids, routes * 4}, {s->d_weights, routes * 4}, {s->d_token_map, static_cast<uint64_t>(experts) * tokens * 4}, {s->d_counts, experts * 4ull},
+                            {s->d_tasks, tsp_moe_tasks_words(tokens, experts, selected, TSP_GEMV_TILE) * 4}, {s->d_hidden, routes * hidden * 4}, {s->d_shared_hidden, h_bytes}};
+    bool own_memory = apart(x_span.p, x_span.bytes, written) && apart(logits_span.p, logits_span.bytes, written);
+    for (const Span& a : written)
+        for (const Span* b = written; b != &a; ++b) own_memory &= !overlap(a.p, a.bytes, b->p, b->bytes);
     // A dense Q8_0 shared expert that cannot ride in the routed launches (they take one of their own encoding, Q4_K) rides in the prologue's: all-Q8_0
-    // layer of five rows 83 -> 73 us, five-bit layer of 13 rows 157 -> 137 us. What its own launches would refuse goes to them.
+    // layer of five rows 83 -> 75 us, two five-bit layers of 13 rows 314 -> 269 us. What its own launches would refuse goes to them. Its output rows are written
+    // before the routed experts read theirs.
     DecodeDense dense{static_cast<const uint8_t*>(w->shared_gate.base), static_cast<const uint8_t*>(w->shared_up.base), static_cast<const uint8_t*>(w->shared_down.base),
                       hidden, channels, d_x, x_stride, s->d_shared_hidden, s->d_shared_out, d_error};
-    const uint64_t x_bytes = tokens * x_stride, h_bytes = tokens * hidden * 4ull, o_bytes = tokens * channels * 4ull;
     auto plain_q8 = [](const tsp_matrix_set& m) { return m.type == TSP_TYPE_Q8_0 && m.layout == TSP_LAYOUT_GGUF && m.experts == 1 && m.split >= 1; };
     const bool dense_ok = plain_q8(w->shared_gate) && plain_q8(w->shared_up) && plain_q8(w->shared_down) && check_matrix(&w->shared_gate, "gate") == TSP_OK &&
                           check_matrix(&w->shared_up, "up") == TSP_OK && check_matrix(&w->shared_down, "project") == TSP_OK && w->shared_up.rows == hidden &&
                           w->shared_up.cols == channels && w->shared_gate.expert_stride == w->shared_up.expert_stride && w->shared_gate.split == w->shared_up.split &&
                           channels % 16 == 0 && aligned16(s->d_shared_hidden) && aligned16(s->d_shared_out) && !overlap(d_x, x_bytes, s->d_shared_hidden, h_bytes) &&
-                          (!s->d_x32 || !overlap(s->d_x32, o_bytes, s->d_shared_hidden, h_bytes)) && !overlap(s->d_shared_hidden, h_bytes, s->d_shared_out, o_bytes);
-    // up to eight rows on Q4_K experts: the gate-up launch routes the batch itself (binary16 rows are then read as they are). It reads logits and rows while
-    // it writes what separate launches write later, and the mixture, a block per slice of a row, reads binary16 rows where it read their FP32 copy: a caller
-    // whose buffers share memory (output rows in the input rows, say) gets the separate launches.
-    const uint64_t routes = static_cast<uint64_t>(tokens) * selected, x_elem = x_dtype == 1 ? 2 : 4, out_elem = out_dtype == 1 ? 2 : 4;
-    const Span x_span{d_x, (tokens - 1) * x_stride + channels * x_elem}, logits_span{d_logits, (tokens - 1) * logits_stride + experts * 4ull};
-    const Span written[] = {{s->d_ids, routes * 4}, {s->d_weights, routes * 4}, {s->d_token_map, static_cast<uint64_t>(experts) * tokens * 4}, {s->d_counts, experts * 4ull},
-                            {s->d_tasks, tsp_moe_tasks_words(tokens, experts, selected, TSP_GEMV_TILE) * 4}, {s->d_hidden, routes * hidden * 4}, {s->d_shared_hidden, h_bytes}};
+                          (!s->d_x32 || !overlap(s->d_x32, o_bytes, s->d_shared_hidden, h_bytes)) && own_memory && apart(s->d_shared_out, o_bytes, written) &&
+                          !overlap(s->d_shared_out, o_bytes, x32, (tokens - 1) * x32_stride + channels * 4ull);
+    // up to eight rows on Q4_K experts: the gate-up launch routes the batch itself (binary16 rows are then read as they are). The mixture, a block per slice
+    // of a row, then reads binary16 rows where it read their FP32 copy: not where something writes them meanwhile (output rows in the input rows, say).
     const Span later[] = {{s->d_routed, routes * channels * 4}, {s->d_shared_out, o_bytes}, {s->d_shared_logit, s->d_shared_logit ? tokens * 4ull : 0}};
-    auto own_memory = [&] {
-        for (const Span* a = written; a != written + sizeof written / sizeof *written; ++a) {
-            if (overlap(a->p, a->bytes, x_span.p, x_span.bytes) || overlap(a->p, a->bytes, logits_span.p, logits_span.bytes)) return false;
-            for (const Span* b = written; b != a; ++b) if (overlap(a->p, a->bytes, b->p, b->bytes)) return false;
-        }
-        return x_dtype == 0 || !w->d_shared_router ||
-               (apart(x_span.p, x_span.bytes, later) && !rows_overlap(d_x, x_stride, channels * x_elem, d_out, out_stride, channels * out_elem, tokens));
-    };
+    const bool rows_last = x_dtype == 0 || !w->d_shared_router ||
+                           (apart(x_span.p, x_span.bytes, later) && !rows_overlap(d_x, x_stride, channels * x_elem, d_out, out_stride, channels * out_elem, tokens));
     int fused = 1;
     bool gated = false;
-    if (tokens <= TSP_GEMV_TILE && experts <= 512 && normalize && w->gate.type == TSP_TYPE_Q4_K && own_memory()) {
+    if (tokens <= TSP_GEMV_TILE && experts <= 512 && normalize && w->gate.type == TSP_TYPE_Q4_K && own_memory && rows_last) {
         const GemvRoute route{d_logits, logits_stride, selected, mode, s->d_ids, s->d_weights, s->d_token_map, s->d_counts, s->d_tasks};
         const int rc = gate_up_shared_launch(&w->gate, &w->up, &w->shared_gate, &w->shared_up, x_dtype == 1 ? s->d_x32 : x32, x32_stride, x_dtype == 1 ? d_x : nullptr,
                                              x_dtype == 1 ? x_stride : 0, tokens, selected, s->d_token_map, s->d_counts, s->d_tasks, s->d_hidden, hidden * 4ull,
