@@ -188,3 +188,33 @@ def test_tables_of_large_batches_report_bad_ids(bad):
     capi.call("tsp_moe_permute", dids.data_ptr(), tokens, experts, selected, 8, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(), e.data_ptr(), L.stream_ptr())
     torch.cuda.synchronize()
     assert int(e.item()) & capi.ERR_INDEX
+
+
+# Without a shared router nothing reads the input rows after their K-ordered copy, and nothing the ids after the route tables. Rows: the last ones, of more
+# blocks than run at a time
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("tokens,own,other", [(8192, "ids", "rows"), (8192, "weights", "rows"), (300, "ids", "offsets"), (1100, "ids", "offsets"), (1100, "ids", "tasks")])
+def test_layer_buffers_that_share_memory(dtype, tokens, own, other):
+    channels, hidden, experts, selected = 256, 256, 8, 2
+    dl = L.SynthDeviceLayer(13, channels, hidden, experts, formats.Q4_K, formats.PLANAR, "cuda")
+    dl.weights.d_shared_router = None
+    x = torch.from_numpy(synth.activations_f16(14, tokens, channels)).cuda().to(dtype)
+    logits = torch.from_numpy(synth.router_logits(15, tokens, experts)).cuda()
+    outs = []
+    for share in (False, True):
+        ps, out = L.PrefillScratch(channels, hidden, experts, selected, tokens, "cuda"), torch.empty((tokens, channels), device="cuda")
+        rows = x.clone()
+        if share:
+            room = torch.zeros(tokens * channels, device="cuda")
+            setattr(ps.c.base, "d_" + own, room.data_ptr() + (x.numel() * x.element_size() - tokens * selected * 4 if other == "rows" else 0))
+            if other == "rows":
+                rows = room.view(dtype)[:x.numel()].view_as(x).copy_(x)
+            elif other == "tasks":
+                ps.c.base.d_tasks = room.data_ptr()
+            else:
+                ps.c.d_offsets = room.data_ptr()
+        L.moe_layer_prefill(dl, ps, rows, logits, out)
+        torch.cuda.synchronize()
+        assert ps.base.error_word() == 0
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])

@@ -94,17 +94,6 @@ static int check_rows(const void* p, uint64_t stride, uint32_t cols, uint32_t el
     return TSP_OK;
 }
 
-static bool overlap(const void* a, uint64_t abytes, const void* b, uint64_t bbytes) {
-    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-    return x < y + bbytes && y < x + abytes;
-}
-// Strided rows: rows of one buffer may lie between those of the other
-static bool rows_overlap(const void* a, uint64_t a_stride, uint64_t a_row, const void* b, uint64_t b_stride, uint64_t b_row, uint64_t rows) {
-    if (!overlap(a, (rows - 1) * a_stride + a_row, b, (rows - 1) * b_stride + b_row)) return false;
-    if (a_stride != b_stride) return true;
-    const uint64_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b), d = y >= x ? (y - x) % a_stride : (a_stride - (x - y) % a_stride) % a_stride;
-    return d < a_row || d + b_row > a_stride;
-}
 struct Span { const void* p; uint64_t bytes; };
 template <size_t N>
 static bool apart(const void* p, uint64_t bytes, const Span (&from)[N]) {
@@ -810,7 +799,10 @@ int tsp_moe_layer_prefill(const tsp_moe_weights* w, const tsp_moe_prefill_scratc
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (int rc = check_rows_f16k(d_x, x_stride, x_dtype, tokens, channels, ps->d_xk, channels * 2ull)) return rc;
     if (int rc = check_route(d_logits, logits_stride, tokens, experts, selected, mode, s->d_ids, s->d_weights)) return rc;
-    const int routed = launch_prefill_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_x, x_stride, x_dtype, channels,
+    // one launch for the routing and the copy of the rows, unless ids or weights are written into the rows (the copy came first: nothing else may read them)
+    const uint64_t x_bytes = (tokens - 1) * x_stride + channels * (x_dtype ? 2ull : 4ull), route_bytes = static_cast<uint64_t>(tokens) * selected * 4;
+    const int routed = overlap(d_x, x_bytes, s->d_ids, route_bytes) || overlap(d_x, x_bytes, s->d_weights, route_bytes) ? 1 :
+                       launch_prefill_route(d_logits, logits_stride, tokens, experts, selected, mode, normalize, s->d_ids, s->d_weights, d_x, x_stride, x_dtype, channels,
                                             ps->d_xk, channels * 2ull, d_error, st);
     if (routed < 0) return routed;
     if (routed) {

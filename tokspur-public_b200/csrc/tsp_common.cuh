@@ -19,6 +19,18 @@ int cuda_fail(cudaError_t e, const char* what);
 #define TSP_CUDA(expr) do { cudaError_t e_ = (expr); if (e_ != cudaSuccess) return ::tsp::cuda_fail(e_, #expr); } while (0)
 int sm_count();  // SM count of the current device (cached), 0 when no device is usable
 
+static inline bool overlap(const void* a, uint64_t abytes, const void* b, uint64_t bbytes) {
+    const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+    return x < y + bbytes && y < x + abytes;
+}
+// Strided rows: rows of one buffer may lie between those of the other
+static inline bool rows_overlap(const void* a, uint64_t a_stride, uint64_t a_row, const void* b, uint64_t b_stride, uint64_t b_row, uint64_t rows) {
+    if (!overlap(a, (rows - 1) * a_stride + a_row, b, (rows - 1) * b_stride + b_row)) return false;
+    if (a_stride != b_stride) return true;
+    const uint64_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b), d = y >= x ? (y - x) % a_stride : (a_stride - (x - y) % a_stride) % a_stride;
+    return d < a_row || d + b_row > a_stride;
+}
+
 // kernel<<<grid, block, smem, stream>>>(args...) with programmatic stream serialisation allowed (see pdl_wait below)
 template <typename... Params, typename... Args>
 static inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {

@@ -847,7 +847,11 @@ int launch_route_offsets(const uint32_t*, uint32_t, uint32_t*, cudaStream_t);
 // offsets (optional): the first permuted position of every expert and the grouped launches' counters, as launch_route_offsets writes them
 int launch_permute(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t tile, uint32_t first, int local_only,
                    uint32_t* token_map, uint32_t* counts, uint32_t* tasks, uint32_t* error, cudaStream_t st, uint32_t* offsets) {
-    if (cluster_fits(tokens, experts))
+    const uint32_t bound = static_cast<uint32_t>((static_cast<uint64_t>(tokens) * selected) / tile + experts);
+    // the cluster reads the ids until its last writes; the launches below have read them before they write tile table and offsets
+    const uint64_t id_bytes = static_cast<uint64_t>(tokens) * selected * 4;
+    const bool ids_apart = !overlap(ids, id_bytes, tasks, 8 + bound * 8ull) && !(offsets && overlap(ids, id_bytes, offsets, (experts + 5) * 4ull));
+    if (ids_apart && cluster_fits(tokens, experts))
         return launch_tables_cluster(ids, tokens, experts, selected, tile, first, local_only, token_map, counts, tasks, offsets, error, st);
     if (tables_fit(tokens, experts)) {
         if (int rc = launch_tables(ids, tokens, experts, selected, tile, first, local_only, token_map, counts, tasks, error, st)) return rc;
@@ -855,7 +859,6 @@ int launch_permute(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint3
     }
     TSP_CUDA(launch_pdl(grouped_routes_kernel, dim3((experts + kPermuteExperts - 1) / kPermuteExperts), dim3(kPermuteThreads), 0, st, ids, tokens, experts, selected, first, local_only, token_map, counts, error));
     TSP_CUDA(cudaGetLastError());
-    const uint32_t bound = static_cast<uint32_t>((static_cast<uint64_t>(tokens) * selected) / tile + experts);
     TSP_CUDA(launch_pdl(grouped_tasks_kernel, dim3(1), dim3(256), (experts + 1) * sizeof(uint32_t), st, counts, tokens, experts, selected, tile, bound, local_only, tasks, error));
     TSP_CUDA(cudaGetLastError());
     return offsets ? launch_route_offsets(counts, experts, offsets, st) : TSP_OK;
