@@ -303,7 +303,8 @@ typedef struct tsp_moe_weights {
  * route -> permute -> gate-up+SwiGLU -> down -> shared expert -> gated combine.
  * Replaces `encode_moe` after its router GEMV (moe.cpp:37-83) and `encode_verify_nax_moe`
  * (verify_nax.cpp:436-575) for small batches. x_dtype/out_dtype: 0 = FP32 rows, 1 = binary16 rows.
- * When d_shared_router is NULL the shared expert is added ungated (gate = 1). */
+ * When d_shared_router is NULL the shared expert is added ungated (gate = 1). Output rows may be the input rows (the same address
+ * and stride). */
 int tsp_moe_layer_decode(const tsp_moe_weights* w, const tsp_moe_scratch* s,
                          const void* d_x, uint64_t x_stride_bytes, uint32_t x_dtype,
                          const float* d_logits, uint64_t logits_stride_bytes,

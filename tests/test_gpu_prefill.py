@@ -218,3 +218,22 @@ def test_layer_buffers_that_share_memory(dtype, tokens, own, other):
         assert ps.base.error_word() == 0
         outs.append(out)
     assert torch.equal(outs[0], outs[1])
+
+
+# In place: every block of the mixture that works on a part of a row reads the whole input row for the shared router
+@pytest.mark.parametrize("path", ["decode", "prefill"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+@pytest.mark.parametrize("tokens", [5, 64, 591, 592])
+def test_layer_in_place(path, dtype, tokens):
+    channels, hidden, experts, selected = 2048, 256, 8, 2
+    dl = L.SynthDeviceLayer(13, channels, hidden, experts, formats.Q4_K, formats.PLANAR, "cuda")
+    x = torch.from_numpy(synth.activations_f16(14, tokens, channels)).cuda().to(dtype)
+    logits = torch.from_numpy(synth.router_logits(15, tokens, experts)).cuda()
+    s = (L.Scratch if path == "decode" else L.PrefillScratch)(channels, hidden, experts, selected, tokens, "cuda")
+    call = L.moe_layer_decode if path == "decode" else L.moe_layer_prefill
+    want = torch.empty_like(x)
+    call(dl, s, x, logits, want)
+    for _ in range(20):
+        rows = x.clone()
+        call(dl, s, rows, logits, rows)
+        assert torch.equal(rows, want)

@@ -872,6 +872,10 @@ int launch_combine(const void* routed, uint64_t routed_stride, uint32_t routed_f
     uint32_t slices = (channels + kCombineThreads - 1) / kCombineThreads;
     const uint32_t want = (4u * 148u + tokens - 1) / tokens;
     if (slices > want) slices = want;
+    // output rows in the input rows (each its own): a block reads the whole row for the shared router before it writes, so one block per row
+    const uint64_t x_row = channels * (x_f16 ? 2ull : 4ull);
+    if (shared_router && ((out && rows_overlap(x, x_stride, x_row, out, out_stride, channels * 4ull, tokens)) ||
+                          (out16 && rows_overlap(x, x_stride, x_row, out16, out16_stride, channels * 2ull, tokens)))) slices = 1;
     auto a16 = [](const void* p, uint64_t stride) { return (reinterpret_cast<uintptr_t>(p) | stride) % 16 == 0; };
     const int vec4 = (routed_f16 ? (reinterpret_cast<uintptr_t>(routed) | routed_stride) % 8 == 0 : a16(routed, routed_stride)) && (!shared || a16(shared, shared_stride)) &&
                      (!out || a16(out, out_stride)) && (!out16 || (reinterpret_cast<uintptr_t>(out16) | out16_stride) % 8 == 0);
