@@ -160,3 +160,17 @@ def test_nonfinite_router_inputs(T, bad):
         got = out.cpu().numpy()
         assert int(err.item()) & capi.ERR_NONFINITE
         assert np.array_equal(got[keep], clean[keep]) and not np.isfinite(got[~keep]).any()
+
+
+def test_extra_row_of_the_largest_matrix_by_warps():
+    """A warp per output: one row more than 2^27 outputs, numbered beyond what 32 bits of threads count."""
+    rows, tokens = 1 << 21, 64
+    w, x = torch.randn(rows, device="cuda"), torch.randn(tokens, device="cuda")
+    extra = torch.tensor([1.5], device="cuda")
+    out, extra_out, e = torch.full((tokens, rows), float("nan"), device="cuda"), torch.full((tokens,), float("nan"), device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    capi.call("tsp_router_project", w.data_ptr(), rows, 1, extra.data_ptr(), x.data_ptr(), 4, tokens, out.data_ptr(), rows * 4, extra_out.data_ptr(), e.data_ptr(), L.stream_ptr())
+    torch.cuda.synchronize()
+    assert int(e.item()) == 0
+    assert torch.equal(extra_out, x * 1.5)
+    for t in (0, 1, tokens - 1):
+        assert torch.equal(out[t], w * x[t])

@@ -736,7 +736,7 @@ gemv_f32_kernel(const float* w, uint32_t rows, uint32_t cols, const float* extra
     pdl_launch_dependents();
     pdl_wait();
 
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, all = rows + (extra ? 1u : 0u);
+    const uint32_t warp = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31, all = rows + (extra ? 1u : 0u);   // threads exceed 32 bits from 2^27 outputs on
     if (warp >= all * tokens) return;
     const uint32_t token = warp / all, row = warp % all;
     const float acc = f32_dot_row(row < rows ? w + static_cast<uint64_t>(row) * cols : extra,
