@@ -174,6 +174,14 @@ def timed(fn, steps, warmup):
     return e0.elapsed_time(e1) / steps
 
 
+def launches_of(fn):
+    """This library's kernel launches in one call."""
+    from tokspur_public_b200 import capi
+    before = capi.lib().tsp_launch_count()
+    fn(0)
+    return int(capi.lib().tsp_launch_count() - before)
+
+
 def timed_median(fn, steps, warmup, min_seconds=0.5, max_repeats=400):
     """Repeats the timed loop of exactly `steps` calls until the timed regions add up to `min_seconds`; returns the median ms per
     call and the number of repeats."""
@@ -241,9 +249,7 @@ def decode_record(args, dev, T, layers, etype, layout, full: bool):
            "timed_repeats": repeats, "unique_experts": U, "layer_algorithmic_bytes": layer_bytes,
            "layer_hbm_gbs": layer_bytes / (ms * 1e-3) / 1e9, "layer_hbm_frac": layer_bytes / (ms * 1e-3) / 1e9 / hbm_peak,
            "layer_tflops": T * (SELECTED + 1) * FLOPS_PER_ROUTE / (ms * 1e-3) / 1e12,
-           # routing, tables, gate-up, down, mixture (a dense Q8_0 shared expert beside Q8_0 or Q5_K experts works in the first two); up to eight rows
-           # on Q4_K experts are routed by the gate-up launch
-           "launches_per_step": 3 if etype == formats.Q4_K and T <= 8 else 5}
+           "launches_per_step": launches_of(step_resident)}
     if not full:
         return rec, None
     # ---- the dominant launch alone, back to back over the rotating layers (tables of batch 0; the weights change every launch)
@@ -339,7 +345,8 @@ def prefill_record(args, dev, layers, T):
     ms_e2e, _ = timed_median(e2e, steps, args.warmup, args.min_seconds / 2)
 
     def stage_pass(n):
-        """CUDA-event time of each launch of the layer, issued exactly as tsp_moe_layer_prefill issues them."""
+        """CUDA-event time of each stage of the layer in a launch of its own (tsp_moe_layer_prefill issues the row copy with the routing, and from 257
+        rows on the offsets with the tables)."""
         s, st = ps.base, L.stream_ptr()
         mixed = layers[0].shared_type != layers[0].type   # a shared expert in another encoding: launches of its own
         names = ["rows_f16k", "route", "permute", "offsets", "gather", "gate_up"] + (["shared_gate_up"] if mixed else []) + ["down"] + \
@@ -386,7 +393,7 @@ def prefill_record(args, dev, layers, T):
            "timed_repeats": repeats, "layer_tflops": layer_flops / (ms * 1e-3) / 1e12, "layer_frac_of_bf16_peak": layer_flops / (ms * 1e-3) / 1e12 / tf_peak,
            "gate_up_launch_tflops": gu_flops / (stages["gate_up_ms"] * 1e-3) / 1e12,
            "gate_up_launch_frac_of_bf16_peak": gu_flops / (stages["gate_up_ms"] * 1e-3) / 1e12 / tf_peak, "peak_tflops": tf_peak, "peak_kind": peak_kind,
-           "stage_ms": stages, "launches_per_step": 6 + 2 * int(layers[0].shared_type != layers[0].type), "router": "N(0,1) + Zipf(1.1) per-expert bias",
+           "stage_ms": stages, "launches_per_step": launches_of(resident), "router": "N(0,1) + Zipf(1.1) per-expert bias",
            "h2d_bytes_per_step": T * CHANNELS * 2 + T * EXPERTS * 4, "d2h_bytes_per_step": T * CHANNELS * 2}
     cpu = None
     if args.cpu_tokens != 0:

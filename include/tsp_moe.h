@@ -264,7 +264,7 @@ int tsp_pack_planar(uint32_t type, uint32_t rows, uint32_t cols, uint32_t expert
 int tsp_gemv_f32(const float* d_w, uint32_t rows, uint32_t cols, const float* d_x, uint64_t x_stride_bytes, uint32_t tokens,
                  float* d_out, uint64_t out_stride_bytes, uint32_t* d_error, void* stream);
 /* Replaces `moe_router_f32_window` + `moe_shared_router_rows` (graph.mm:5812, 5884): the router projection of a batch and that
- * of the shared-router vector as a launch of its own, d_extra_out[t] = sum_c d_extra_row[c] x[t][c] (both NULL: none).
+ * of the shared-router vector in one launch, d_extra_out[t] = sum_c d_extra_row[c] x[t][c] (both NULL: none).
  * The ids chosen from these logits have to follow the reference's double-precision logits, so the error is that of FP32 sums or
  * less: up to 95 token rows one FP32 FMA chain per lane, from 96 on tensor-core products of the three bfloat16 parts that each
  * FP32 value splits into exactly (a term's error stays within 2^-24 of it, 2.4e-7 for 2048 columns in the relative 2-norm, one FP32
@@ -382,7 +382,7 @@ int tsp_moe_staged_f16(const tsp_matrix_set* m, uint32_t expert, void* d_out, vo
  * path (graph.mm:9293-9420). Weights: Q4_K, Pack v3 planar or plain GGUF super-blocks, hidden a multiple of 64 and channels
  * of 256. A shared expert in the routed experts' form rides in the routed launches; in another form (dense Q8_0 GGUF blocks
  * beside Q4_K experts, as the reference's model has it) it is computed by tsp_dense_mm_swiglu / tsp_dense_mm in launches of
- * its own (8 launches instead of 6). Arguments as tsp_moe_layer_decode; `tokens` <= s->base.capacity.
+ * its own. Arguments as tsp_moe_layer_decode; `tokens` <= s->base.capacity.
  * Caller-owned scratch, all device memory, nothing has to start at zero:
  *   base: as for the decode layer, except d_tasks sized tsp_moe_tasks_words(capacity, experts, selected, TSP_GROUPED_TILE);
  *         d_routed is used as binary16 rows [capacity*selected x channels]; d_hidden, d_shared_hidden and d_x32 are not
@@ -402,6 +402,16 @@ int tsp_moe_layer_prefill(const tsp_moe_weights* w, const tsp_moe_prefill_scratc
                           uint32_t x_dtype, const float* d_logits, uint64_t logits_stride_bytes, uint32_t tokens,
                           uint32_t channels, uint32_t hidden, uint32_t experts, uint32_t selected, uint32_t mode,
                           int normalize, void* d_out, uint64_t out_stride_bytes, uint32_t out_dtype, uint32_t* d_error, void* stream);
+
+/* What the reference counts as dispatches (graph.hpp BatchResult, moe_mm_many_dispatches): kernel launches the calling thread has made through
+ * the operators so far, and those of one layer call with these weights whose buffers share no memory. decode asks the layer itself, which
+ * launches nothing then (x_dtype as there; 0: the layer would refuse, tsp_last_error says why). A prefill call has six launches with more than 256
+ * rows, seven below; two more for a shared expert in another form, and others for many experts, for weights that are not renormalised, and from
+ * half a million rows on. */
+uint64_t tsp_launch_count(void);
+uint32_t tsp_moe_layer_decode_launches(const tsp_moe_weights* w, uint32_t x_dtype, uint32_t tokens, uint32_t channels, uint32_t hidden,
+                                       uint32_t experts, uint32_t selected, uint32_t mode, int normalize_selected);
+uint32_t tsp_moe_layer_prefill_launches(const tsp_moe_weights* w, uint32_t tokens, uint32_t experts, int normalize_selected);
 
 /* No counterpart in the reference (its graph always works out of caller-allocated buffers).
  *

@@ -90,6 +90,9 @@ SIGNATURES = {
                                   _u32, _u32, _u32, _i, _vp, _u64, _u32, _vp, _vp]),
     "tsp_moe_layer_prefill": (_i, [C.POINTER(MoeWeights), C.POINTER(MoePrefillScratch), _vp, _u64, _u32, _vp, _u64, _u32, _u32, _u32,
                                    _u32, _u32, _u32, _i, _vp, _u64, _u32, _vp, _vp]),
+    "tsp_launch_count": (_u64, []),
+    "tsp_moe_layer_decode_launches": (_u32, [C.POINTER(MoeWeights), _u32, _u32, _u32, _u32, _u32, _u32, _u32, _i]),
+    "tsp_moe_layer_prefill_launches": (_u32, [C.POINTER(MoeWeights), _u32, _u32, _i]),
     "tsp_moe_route_offsets": (_i, [_vp, _u32, _vp, _vp]),
     "tsp_moe_rows_f16k": (_i, [_vp, _u64, _u32, _u32, _u32, _vp, _u64, _vp, _vp]),
     "tsp_moe_gather_rows16": (_i, [_vp, _u64, _vp, _vp, _u32, _u32, _u32, _u32, _vp, _u64, _vp]),

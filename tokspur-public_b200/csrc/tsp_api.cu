@@ -4,6 +4,7 @@
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
+#include <type_traits>
 
 #include "tsp_common.cuh"
 #include "tsp_q8_rows.cuh"
@@ -23,6 +24,11 @@ int fail(int code, const char* fmt, ...) {
 int cuda_fail(cudaError_t e, const char* what) {
     snprintf(g_message, sizeof g_message, "CUDA error %d (%s) at %s", static_cast<int>(e), cudaGetErrorString(e), what);
     return TSP_E_CUDA;
+}
+
+LaunchCount& launch_count() {
+    static thread_local LaunchCount count;
+    return count;
 }
 
 int sm_count() {
@@ -45,6 +51,8 @@ int launch_combine(const void*, uint64_t, uint32_t, const float*, const float*, 
                    uint32_t, uint32_t, uint32_t, float*, uint64_t, void*, uint64_t, uint32_t*, cudaStream_t);
 int launch_decode_prologue(const float*, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t, uint32_t*, float*, uint32_t*, uint32_t*,
                            uint32_t*, const void*, uint64_t, float*, uint64_t, uint32_t, DecodeDense*, uint32_t*, cudaStream_t);
+bool prefill_route_fits(uint32_t, int);
+uint32_t permute_launches(uint32_t, uint32_t);
 int launch_prefill_route(const float*, uint64_t, uint32_t, uint32_t, uint32_t, uint32_t, int, uint32_t*, float*, const void*, uint64_t, uint32_t, uint32_t, void*,
                          uint64_t, uint32_t*, cudaStream_t);
 int launch_f16_to_f32(const void*, uint64_t, float*, uint64_t, uint32_t, uint32_t, cudaStream_t);
@@ -629,6 +637,10 @@ static int check_route(const void* d_logits, uint64_t stride, uint32_t tokens, u
     return TSP_OK;
 }
 
+static bool same_form(const tsp_matrix_set& a, const tsp_matrix_set& b) { return a.type == b.type && a.layout == b.layout; }
+static bool rides_up(const tsp_moe_weights& w) { return same_form(w.shared_gate, w.gate) && same_form(w.shared_up, w.gate); }
+static bool rides_down(const tsp_moe_weights& w) { return same_form(w.shared_down, w.down); }
+
 extern "C" {
 
 int tsp_moe_rows_f16k(const void* d_x, uint64_t x_stride, uint32_t x_dtype, uint32_t rows, uint32_t cols, void* d_xk, uint64_t xk_stride,
@@ -815,9 +827,7 @@ int tsp_moe_layer_prefill(const tsp_moe_weights* w, const tsp_moe_prefill_scratc
     // the dense shared expert rides in both launches when it has the routed experts' encoding and layout; in another form (the
     // reference's dense Q8_0 shared expert beside Q4_K experts) it gets the same kernel in launches of its own.
     // The route rows are kept as binary16 (half the traffic of the mixture)
-    auto same_form = [](const tsp_matrix_set& a, const tsp_matrix_set& b) { return a.type == b.type && a.layout == b.layout; };
-    const bool ride_up = same_form(w->shared_gate, w->gate) && same_form(w->shared_up, w->gate);
-    const bool ride_down = same_form(w->shared_down, w->down);
+    const bool ride_up = rides_up(*w), ride_down = rides_down(*w);
     if (int rc = tsp_moe_grouped_gate_up(&w->gate, &w->up, ride_up ? &w->shared_gate : nullptr, ride_up ? &w->shared_up : nullptr, ps->d_xp, channels * 2ull,
                                          ps->d_xk, channels * 2ull, tokens, tokens, selected, s->d_token_map,
                                          s->d_counts, s->d_tasks, ps->d_offsets, ps->d_hp, hidden * 2ull, ps->d_s_hp, hidden * 2ull, d_error, st)) return rc;
@@ -833,6 +843,36 @@ int tsp_moe_layer_prefill(const tsp_moe_weights* w, const tsp_moe_prefill_scratc
     return tsp_moe_combine(s->d_routed, channels * 2ull, 1, s->d_weights, s->d_shared_out, channels * 4ull, w->d_shared_router, d_x, x_stride, x_dtype,
                            s->d_shared_logit, tokens, channels, selected, out_dtype == 0 ? static_cast<float*>(d_out) : nullptr,
                            out_dtype == 0 ? out_stride : 0, out_dtype == 1 ? d_out : nullptr, out_dtype == 1 ? out_stride : 0, d_error, st);
+}
+
+uint64_t tsp_launch_count(void) { return launch_count().launches; }
+
+// Addresses for the buffers that no weight lies in: aligned, a tebibyte each, never read
+uint32_t tsp_moe_layer_decode_launches(const tsp_moe_weights* w, uint32_t x_dtype, uint32_t tokens, uint32_t channels, uint32_t hidden, uint32_t experts, uint32_t selected,
+                                       uint32_t mode, int normalize) {
+    uintptr_t next = 1ull << 48;
+    auto take = [&](auto*& p) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(next); next += 1ull << 40; };
+    tsp_moe_scratch s{};
+    take(s.d_ids); take(s.d_weights); take(s.d_hidden); take(s.d_routed); take(s.d_shared_hidden); take(s.d_shared_out); take(s.d_shared_logit); take(s.d_x32);
+    take(s.d_token_map); take(s.d_counts); take(s.d_tasks);
+    s.capacity = tokens;
+    float *x, *logits, *out;
+    uint32_t* error;
+    take(x); take(logits); take(out); take(error);
+    LaunchCount& count = launch_count();
+    const LaunchCount before = count;
+    count.dry = true;
+    const int rc = tsp_moe_layer_decode(w, &s, x, channels * (x_dtype ? 2ull : 4ull), x_dtype, logits, experts * 4ull, tokens, channels, hidden, experts, selected, mode,
+                                        normalize, out, channels * 4ull, 0, error, nullptr);
+    const uint64_t n = count.launches - before.launches;
+    count = before;
+    return rc == TSP_OK ? static_cast<uint32_t>(n) : 0u;
+}
+
+uint32_t tsp_moe_layer_prefill_launches(const tsp_moe_weights* w, uint32_t tokens, uint32_t experts, int normalize) {
+    if (!w || !tokens || !experts || experts > 4096) return 0;
+    const uint32_t dense = (rides_up(*w) ? 0u : 1u) + (rides_down(*w) ? 0u : 1u);
+    return (prefill_route_fits(experts, normalize) ? 1u : 2u) + permute_launches(tokens, experts) + 4u + dense;   // routed copy, gate-up, down, mixture
 }
 
 uint64_t tsp_moe_layer_decode_static_bytes(uint32_t tokens, uint32_t channels, uint32_t hidden, uint32_t experts, uint32_t selected) {

@@ -31,9 +31,16 @@ static inline bool rows_overlap(const void* a, uint64_t a_stride, uint64_t a_row
     return d < a_row || d + b_row > a_stride;
 }
 
+// Kernel launches of this thread, and whether they are only counted (tsp_moe_layer_decode_launches asks the layer itself what it would launch)
+struct LaunchCount { uint64_t launches = 0; bool dry = false; };
+LaunchCount& launch_count();
+
 // kernel<<<grid, block, smem, stream>>>(args...) with programmatic stream serialisation allowed (see pdl_wait below)
 template <typename... Params, typename... Args>
 static inline cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    LaunchCount& count = launch_count();
+    ++count.launches;
+    if (count.dry) return cudaSuccess;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
     cudaLaunchAttribute attr;

@@ -750,7 +750,7 @@ int launch_gemv(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup, c
     // A dense plain projection in K parts (the vocabulary head): 1187 items of 128 rows over 148 CTAs leave three CTAs a ninth item
     // while the rest idle. Splitting the (item, K part) sequence evenly instead costs one pass of zeros over the output rows.
     p.balance = (p.kparts > 1 && !gateup && !token_map && a->experts == 1 && p.items_per_matrix >= static_cast<uint32_t>(grid)) ? 1 : 0;
-    if (p.balance) TSP_CUDA(cudaMemset2DAsync(out, out_stride_bytes, 0, static_cast<size_t>(a->rows) * 4, tokens, st));
+    if (p.balance && !launch_count().dry) TSP_CUDA(cudaMemset2DAsync(out, out_stride_bytes, 0, static_cast<size_t>(a->rows) * 4, tokens, st));
     GemvPartMaps map{};
     if (p.kparts > 1) {   // [row bytes][rows][experts] as 32-bit elements: a box of one K part (272 or 544 bytes) of the item's rows
         if (p.expert_stride % 16 != 0 && a->experts > 1) return fail(TSP_E_ARG, "project: expert stride must be a multiple of 16 bytes");

@@ -458,6 +458,9 @@ static int launch_tables_cluster(const uint32_t* ids, uint32_t tokens, uint32_t 
     const size_t smem = cluster_smem(tokens, experts);
     static thread_local SmemAttrCache configured;
     TSP_CUDA(ensure_dynamic_smem(tables_cluster_kernel, configured, smem));
+    LaunchCount& count = launch_count();
+    ++count.launches;
+    if (count.dry) return TSP_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kTablesCluster); cfg.blockDim = dim3(kPrologueThreads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
     cudaLaunchAttribute attr[2];
@@ -526,6 +529,7 @@ static int launch_decode_route(dim3 grid, size_t smem, cudaStream_t st, const fl
 // 25 us of a 4096-row layer, 13 and 5 of 1003 and 160 rows; 11, 8 and 4 now): the first blocks route, a warp per row, the others copy. Register form of the routing only (up to 512 experts,
 // renormalised weights); returns 1 for anything else.
 constexpr uint32_t kPrefillRouteWarps = 8;
+bool prefill_route_fits(uint32_t experts, int normalize) { return experts <= 512 && normalize; }
 
 template <bool IN16>
 __global__ void __launch_bounds__(256)
@@ -547,7 +551,7 @@ prefill_route_kernel(const float* logits, uint64_t logits_stride, uint32_t token
 int launch_prefill_route(const float* logits, uint64_t logits_stride, uint32_t tokens, uint32_t experts, uint32_t selected, uint32_t mode, int normalize,
                          uint32_t* ids, float* weights, const void* x, uint64_t x_stride, uint32_t x_dtype, uint32_t cols, void* xk, uint64_t xk_stride,
                          uint32_t* error, cudaStream_t st) {
-    if (experts > 512 || !normalize) return 1;
+    if (!prefill_route_fits(experts, normalize)) return 1;
     const uint32_t route_blocks = (tokens + kPrefillRouteWarps - 1) / kPrefillRouteWarps, row_blocks = (tokens + 3) / 4;
     const dim3 grid(route_blocks + row_blocks);
     if (x_dtype == 1)
@@ -863,6 +867,9 @@ int launch_permute(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint3
     TSP_CUDA(cudaGetLastError());
     return offsets ? launch_route_offsets(counts, experts, offsets, st) : TSP_OK;
 }
+
+// launches of launch_permute with offsets, the ids in memory of their own
+uint32_t permute_launches(uint32_t tokens, uint32_t experts) { return cluster_fits(tokens, experts) ? 1u : tables_fit(tokens, experts) ? 2u : 3u; }
 
 int launch_combine(const void* routed, uint64_t routed_stride, uint32_t routed_f16, const float* weights, const float* shared,
                    uint64_t shared_stride, const float* shared_router, const void* x, uint64_t x_stride, uint32_t x_f16,

@@ -188,7 +188,7 @@ def _timed(fn, steps, warmup, dev):
 
 def _phase(ctx, args, rank, world, dev, prefill: bool, T: int, layers_n: int, nb: int, replicate: int, scratch=None):
     """One workload (decode batch or prefill batch per rank) through the expert-parallel layer: resident and end-to-end timing."""
-    from . import synth
+    from . import capi, synth
     from bench import CHANNELS, HIDDEN, EXPERTS, SELECTED
     bias = synth.zipf_bias(5, EXPERTS) if prefill else None
     # the replicated set comes from a calibration batch every rank can generate for itself (same seed everywhere)
@@ -215,13 +215,15 @@ def _phase(ctx, args, rank, world, dev, prefill: bool, T: int, layers_n: int, nb
         stream.synchronize()
 
     steps, warmup = (max(3, args.steps // 4), max(3, args.warmup)) if prefill else (args.steps, max(3, args.warmup))
+    before = capi.lib().tsp_launch_count()
     ms = _timed(resident, steps, warmup, dev)
+    launches = (capi.lib().tsp_launch_count() - before) // (steps + warmup) + 4   # and the exchange's own: plan, pack, unpack, finish
     ms_e2e = _timed(e2e, steps, warmup, dev)
     err = torch.tensor([sum(l.error_word() for l in layers)], device=dev)
     dist.all_reduce(err, op=dist.ReduceOp.MAX)
     assert int(err.item()) == 0, "device error word set during the benchmark"
     # parity of this rank's rows of batch 0 against the CPU oracle needs the whole layer's weights: done at N = 1 only
-    return {"ms": ms, "ms_e2e": ms_e2e, "tokens_per_rank": T, "replicated_experts": len(rep), "layers": layers, "steps": steps}
+    return {"ms": ms, "ms_e2e": ms_e2e, "tokens_per_rank": T, "replicated_experts": len(rep), "layers": layers, "steps": steps, "launches": int(launches)}
 
 
 def run_bench(args, rank: int, world: int, local: int) -> None:
@@ -265,7 +267,7 @@ def run_bench(args, rank: int, world: int, local: int) -> None:
                            "l2_policy": "layers rotate; per step each GPU streams its hit experts once"},
                 "e2e": {"value": total / (dec["ms_e2e"] * 1e-3), "unit": "tokens/s", "ms_per_step": dec["ms_e2e"],
                         "h2d_bytes_per_step": world * (T * CHANNELS * 2 + T * EXPERTS * 4), "d2h_bytes_per_step": world * T * CHANNELS * 2},
-                "gpu_launches": 17 * args.steps, "clocks": clocks.summary(),
+                "gpu_launches": dec["launches"] * args.steps, "clocks": clocks.summary(),
                 "roofline": {"bound": "hbm", "kernel": "whole expert-parallel decode step on the busiest GPU (its hit experts + the shared expert, gate-up and down)",
                              "achieved": step_bytes / (dec["ms"] * 1e-3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                              "frac": step_bytes / (dec["ms"] * 1e-3) / 1e9 / hbm_peak, "peak_kind": peak_kind, "traffic": None,

@@ -57,7 +57,7 @@ void release_moe_many_scratch(CudaGraph& graph, const MoeManyScratch& scratch);
 // moe_many.hpp:16). Kernels here need no pipeline objects, so nothing else is prepared.
 void prepare_moe_many(CudaGraph& graph, const MoeWeights& weights, MoeShape shape);
 // Launches one encode_moe_many of `steps` rows issues (the figure CommandBatch::dispatches grows by)
-uint64_t moe_many_dispatches(const CudaGraph& graph, const MoeWeights& weights, MoeShape shape, uint32_t steps);
+uint64_t moe_many_dispatches(const CudaGraph& graph, const MoeWeights& weights, MoeShape shape, uint32_t steps, bool normalize_selected = true);
 void encode_moe_many(CudaGraph& graph, const MoeWeights& weights, const MoeManyScratch& scratch, GpuView input, GpuView output, MoeShape shape,
                      RouterMode mode, bool normalize_selected, uint32_t steps);
 

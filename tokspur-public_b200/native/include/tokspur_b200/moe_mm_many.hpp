@@ -53,6 +53,6 @@ void prepare_moe_mm_many(CudaGraph& graph, const MoeWeights& weights, MoeShape s
 // Launches one encode_moe_mm_many of `rows` rows issues with a scratch of `capacity` rows (moe_mm_many_dispatches, moe_mm_many.hpp:60;
 // the reference's chunk is fixed, here it is the scratch capacity).
 uint64_t moe_mm_many_dispatches(const CudaGraph& graph, const MoeWeights& weights, MoeShape shape, uint32_t rows, uint32_t capacity,
-                                MoeMmLayouts layouts = {});
+                                MoeMmLayouts layouts = {}, bool normalize_selected = true);
 
 }  // namespace tokspur_b200

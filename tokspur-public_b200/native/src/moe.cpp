@@ -67,6 +67,29 @@ bool is_planar_moe(const CudaGraph& g, const MoeWeights& w, MoeShape s) {
 namespace {
 void encode_rows(CudaGraph& g, const MoeWeights& w, const MoeScratch& s, GpuView input, GpuView output, MoeShape shape, RouterMode mode,
                  bool normalize_selected, uint32_t rows);
+
+// the weights as the C ABI's layer takes them
+tsp_moe_weights layer_weights(const CudaGraph& g, const MoeWeights& w, MoeShape shape) {
+    if (w.router.encoding != 0 || w.shared_router.encoding != 0) throw FormatError("router projections must be F32");
+    tsp_moe_weights tw{};
+    if (is_planar_gate_up(g, w, shape)) {
+        // co-located pairs: the "gate" tensor holds experts [0, E/2) as [gate_e, up_e], the "up" tensor experts [E/2, E)
+        const uint64_t pb = tsp_expert_bytes(w.gate.encoding, TSP_LAYOUT_PLANAR, shape.hidden, shape.channels);
+        const auto lo = static_cast<const char*>(g.device_pointer(w.gate.view)), hi = static_cast<const char*>(g.device_pointer(w.up.view));
+        tw.gate = {lo, hi, 2 * pb, shape.experts / 2, shape.experts, shape.hidden, shape.channels, w.gate.encoding, TSP_LAYOUT_PLANAR};
+        tw.up = {lo + pb, hi + pb, 2 * pb, shape.experts / 2, shape.experts, shape.hidden, shape.channels, w.up.encoding, TSP_LAYOUT_PLANAR};
+    } else {
+        tw.gate = matrix_set(g, w.gate, shape.hidden, shape.channels, shape.experts);
+        tw.up = matrix_set(g, w.up, shape.hidden, shape.channels, shape.experts);
+    }
+    tw.down = matrix_set(g, w.down, shape.channels, shape.hidden, shape.experts);
+    tw.shared_gate = matrix_set(g, w.shared_gate, shape.hidden, shape.channels, 1);
+    tw.shared_up = matrix_set(g, w.shared_up, shape.hidden, shape.channels, 1);
+    tw.shared_down = matrix_set(g, w.shared_down, shape.channels, shape.hidden, 1);
+    tw.d_shared_router = static_cast<const float*>(g.device_pointer(w.shared_router.view));
+    if (w.shared_router.view.bytes != uint64_t(shape.channels) * 4) throw FormatError("shared router shape mismatch");
+    return tw;
+}
 }
 
 void encode_moe(CudaGraph& g, const MoeWeights& w, const MoeScratch& s, GpuView input, GpuView output, MoeShape shape,
@@ -95,10 +118,13 @@ void prepare_moe_many(CudaGraph& g, const MoeWeights& w, MoeShape shape) {
     (void)matrix_set(g, w.shared_down, shape.channels, shape.hidden, 1);
 }
 
-uint64_t moe_many_dispatches(const CudaGraph&, const MoeWeights&, MoeShape shape, uint32_t steps) {
+uint64_t moe_many_dispatches(const CudaGraph& g, const MoeWeights& w, MoeShape shape, uint32_t steps, bool normalize_selected) {
     shape_check(shape);
     if (!steps || steps > 64) throw FormatError("invalid row count for the mixture");
-    return 6;   // router GEMV, routing (+ row conversion), permutation + tile table, gate-up, down, mixture
+    const tsp_moe_weights tw = layer_weights(g, w, shape);
+    const uint32_t layer = tsp_moe_layer_decode_launches(&tw, 0, steps, shape.channels, shape.hidden, shape.experts, shape.selected, 0, normalize_selected);
+    if (!layer) throw FormatError(tsp_last_error());
+    return 1u + layer;   // the router GEMV first
 }
 
 void encode_moe_many(CudaGraph& g, const MoeWeights& w, const MoeManyScratch& s, GpuView input, GpuView output, MoeShape shape, RouterMode mode,
@@ -118,24 +144,7 @@ void encode_rows(CudaGraph& g, const MoeWeights& w, const MoeScratch& s, GpuView
                  bool normalize_selected, uint32_t rows) {
     shape_check(shape);
     if (input.bytes != uint64_t(shape.channels) * 4 * rows || output.bytes != uint64_t(shape.channels) * 4 * rows) throw FormatError("mixture shape mismatch");
-    if (w.router.encoding != 0 || w.shared_router.encoding != 0) throw FormatError("router projections must be F32");
-    tsp_moe_weights tw{};
-    if (is_planar_gate_up(g, w, shape)) {
-        // co-located pairs: the "gate" tensor holds experts [0, E/2) as [gate_e, up_e], the "up" tensor experts [E/2, E)
-        const uint64_t pb = tsp_expert_bytes(w.gate.encoding, TSP_LAYOUT_PLANAR, shape.hidden, shape.channels);
-        const auto lo = static_cast<const char*>(g.device_pointer(w.gate.view)), hi = static_cast<const char*>(g.device_pointer(w.up.view));
-        tw.gate = {lo, hi, 2 * pb, shape.experts / 2, shape.experts, shape.hidden, shape.channels, w.gate.encoding, TSP_LAYOUT_PLANAR};
-        tw.up = {lo + pb, hi + pb, 2 * pb, shape.experts / 2, shape.experts, shape.hidden, shape.channels, w.up.encoding, TSP_LAYOUT_PLANAR};
-    } else {
-        tw.gate = matrix_set(g, w.gate, shape.hidden, shape.channels, shape.experts);
-        tw.up = matrix_set(g, w.up, shape.hidden, shape.channels, shape.experts);
-    }
-    tw.down = matrix_set(g, w.down, shape.channels, shape.hidden, shape.experts);
-    tw.shared_gate = matrix_set(g, w.shared_gate, shape.hidden, shape.channels, 1);
-    tw.shared_up = matrix_set(g, w.shared_up, shape.hidden, shape.channels, 1);
-    tw.shared_down = matrix_set(g, w.shared_down, shape.channels, shape.hidden, 1);
-    tw.d_shared_router = static_cast<const float*>(g.device_pointer(w.shared_router.view));
-    if (w.shared_router.view.bytes != uint64_t(shape.channels) * 4) throw FormatError("shared router shape mismatch");
+    const tsp_moe_weights tw = layer_weights(g, w, shape);
 
     tsp_moe_scratch ts{};
     ts.d_ids = static_cast<uint32_t*>(g.device_pointer(s.indices, true));
@@ -158,12 +167,13 @@ void encode_rows(CudaGraph& g, const MoeWeights& w, const MoeScratch& s, GpuView
         throw FormatError("mixture scratch too small");
 
     g.gemv_f32_rows(w.router.view, input, uint64_t(shape.channels) * 4, rows, s.logits, uint64_t(shape.experts) * 4, shape.channels, shape.experts);
+    const uint64_t launched = tsp_launch_count();
     const int rc = tsp_moe_layer_decode(&tw, &ts, g.device_pointer(input), uint64_t(shape.channels) * 4, 0,
                                         static_cast<const float*>(g.device_pointer(s.logits)), uint64_t(shape.experts) * 4, rows, shape.channels,
                                         shape.hidden, shape.experts, shape.selected, uint32_t(mode), normalize_selected,
                                         g.device_pointer(output, true), uint64_t(shape.channels) * 4, 0, g.error_word(), g.stream());
     if (rc != TSP_OK) throw FormatError(tsp_last_error());
-    g.count_dispatches(5);   // routing (+ row conversion), permutation + tile table, gate-up, down, combine (the shared expert rides in the routed launches)
+    g.count_dispatches(tsp_launch_count() - launched);
 }
 }  // namespace
 

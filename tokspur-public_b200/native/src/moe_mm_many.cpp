@@ -45,12 +45,6 @@ void release_moe_mm_many_scratch(CudaGraph& graph, const MoeMmManyScratch& scrat
 }
 
 namespace {
-constexpr uint64_t kLaunchesPerChunk = 10;   // router GEMM, K-ordered rows, route, routes, tasks, offsets, routed copy, gate-up, down, mixture
-// a shared expert that cannot ride in the routed launches adds one launch per projection
-uint64_t extra_launches(const tsp_moe_weights& tw) {
-    auto same = [](const tsp_matrix_set& a, const tsp_matrix_set& b) { return a.type == b.type && a.layout == b.layout; };
-    return (same(tw.shared_gate, tw.gate) && same(tw.shared_up, tw.gate) ? 0u : 1u) + (same(tw.shared_down, tw.down) ? 0u : 1u);
-}
 tsp_moe_weights checked_weights(const CudaGraph& g, const MoeWeights& w, MoeShape shape, MoeMmLayouts l) {
     // gate and up go through one launch: one identity for the pair (routed, and shared). A shared expert whose encoding or
     // identity differs from the routed experts' gets launches of its own
@@ -102,11 +96,13 @@ void prepare_moe_mm_many(CudaGraph& g, const MoeWeights& w, MoeShape shape, MoeM
     (void)checked_weights(g, w, shape, layouts);
 }
 
-uint64_t moe_mm_many_dispatches(const CudaGraph& g, const MoeWeights& w, MoeShape shape, uint32_t rows, uint32_t capacity, MoeMmLayouts layouts) {
+uint64_t moe_mm_many_dispatches(const CudaGraph& g, const MoeWeights& w, MoeShape shape, uint32_t rows, uint32_t capacity, MoeMmLayouts layouts,
+                                bool normalize_selected) {
     (void)moe_mm_many_bytes(shape, capacity);
     need(rows > 0, "tiled MoE active rows");
     const tsp_moe_weights tw = checked_weights(g, w, shape, layouts);
-    return (kLaunchesPerChunk + extra_launches(tw)) * ((uint64_t(rows) + capacity - 1) / capacity);
+    auto chunk = [&](uint32_t n) { return 1ull + tsp_moe_layer_prefill_launches(&tw, n, shape.experts, normalize_selected); };   // the router projection first
+    return rows / capacity * chunk(capacity) + (rows % capacity ? chunk(rows % capacity) : 0ull);
 }
 
 void encode_moe_mm_many(CudaGraph& g, const MoeWeights& w, const MoeMmManyScratch& s, GpuRowsF32 input, GpuRowsF32 output, MoeShape shape,
@@ -143,11 +139,12 @@ void encode_moe_mm_many(CudaGraph& g, const MoeWeights& w, const MoeMmManyScratc
 
     const uint32_t n = input.rows;
     g.gemv_f32_rows(w.router.view, input.view, input.stride_bytes, n, s.logits, uint64_t(shape.experts) * 4, shape.channels, shape.experts);
+    const uint64_t launched = tsp_launch_count();   // the router projection has counted itself
     const int rc = tsp_moe_layer_prefill(&tw, &ps, g.device_pointer(input.view), input.stride_bytes, 0, static_cast<const float*>(g.device_pointer(s.logits)),
                                          uint64_t(shape.experts) * 4, n, shape.channels, shape.hidden, shape.experts, shape.selected, uint32_t(mode),
                                          normalize_selected, g.device_pointer(output.view, true), output.stride_bytes, 0, g.error_word(), g.stream());
     if (rc != TSP_OK) throw FormatError(tsp_last_error());
-    g.count_dispatches(kLaunchesPerChunk - 1 + extra_launches(tw));   // the router GEMM counted itself
+    g.count_dispatches(tsp_launch_count() - launched);
 }
 
 }  // namespace tokspur_b200

@@ -130,7 +130,7 @@ void layer(CudaGraph& g, uint32_t type, bool use_planar, MoeShape shape, uint32_
             g.begin();
             encode_moe(g, w, scratch, input, output, shape, RouterMode::softmax, true);
             const auto batch = g.submit();
-            require(batch.dispatches >= 5 && g.allocations() == allocations, "dispatch / allocation invariant");
+            require(batch.dispatches == moe_many_dispatches(g, w, shape, 1) && g.allocations() == allocations, "dispatch / allocation invariant");
             require(read<uint32_t>(g, scratch.indices) == eids, "route ids differ");
             close(read<float>(g, scratch.weights), ew.data(), K);
             close(read<float>(g, scratch.gate), act.data(), act.size());
@@ -314,7 +314,8 @@ void many(CudaGraph& g, MoeShape shape, uint32_t rows, uint32_t capacity, uint32
         encode_moe_mm_many(g, m, scratch, {input, rows, C, in_stride}, {output, rows, C, out_stride}, shape, RouterMode::softmax, true, mixed);
         const auto batch = g.submit();
         const uint64_t chunks = (uint64_t(rows) + capacity - 1) / capacity;
-        require(batch.dispatches == moe_mm_many_dispatches(g, m, shape, rows, capacity, mixed) && batch.dispatches == 12 * chunks && g.allocations() == before,
+        require(batch.dispatches == moe_mm_many_dispatches(g, m, shape, rows, capacity, mixed) &&
+                batch.dispatches == moe_mm_many_dispatches(g, w, shape, rows, capacity) + 2 * chunks && g.allocations() == before,
                 "dispatch / allocation invariant (Q8_0 shared)");
         const auto got = g.read(output);
         double num = 0, den = 0;
