@@ -287,7 +287,7 @@ def test_unit_geometry(oracle, type_, rows, cols, gate_up):
     assert int(e.item()) == 0
 
 
-@pytest.mark.parametrize("tokens,experts,selected", [(1500, 512, 8), (2048, 4096, 32)])
+@pytest.mark.parametrize("tokens,experts,selected", [(1500, 512, 32), (2048, 4096, 32)])
 def test_many_tiles_per_block(oracle, tokens, experts, selected):
     """Blocks that walk more tiles than their routing table holds (32), with the experts in two address ranges."""
     rows, cols = 16, 128
@@ -307,7 +307,9 @@ def test_many_tiles_per_block(oracle, tokens, experts, selected):
     capi.call("tsp_moe_project", C.byref(ms), dx.data_ptr(), cols * 4, selected, tokens, selected, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(),
               out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
     torch.cuda.synchronize()
-    assert int(e.item()) == 0 and int(tasks[0]) > 32 * 16
+    assert int(e.item()) == 0
+    # a unit of 16 rows per tile, spread evenly: every block has more tiles than its table
+    assert int(tasks[0]) > 33 * torch.cuda.get_device_properties(0).multi_processor_count
     w64 = oracle.dequantize(formats.Q5_1, w.reshape(-1), experts * rows * cols).astype(np.float64).reshape(experts, rows, cols)
     want = np.einsum("tkrc,tc->tkr", w64[ids[::16]], x[::16].astype(np.float64))
     got = out.cpu().numpy().reshape(tokens, selected, rows)[::16]
