@@ -25,7 +25,7 @@ def logits_of(kind, rows, experts, seed):
 
 
 @pytest.mark.parametrize("kind", ["normal", "ties", "zeros", "lane"])
-@pytest.mark.parametrize("experts,selected", [(8, 8), (33, 10), (512, 1), (512, 10), (512, 32), (512, 33), (500, 64)])
+@pytest.mark.parametrize("experts,selected", [(8, 8), (33, 10), (512, 1), (512, 8), (512, 9), (512, 10), (512, 32), (512, 33), (500, 64)])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_selection_against_oracle(oracle, kind, experts, selected, mode):
     rows = 5
