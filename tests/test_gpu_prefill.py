@@ -129,7 +129,8 @@ def test_overflowing_hidden_row_is_reported_and_stays_alone(oracle):
 # The cluster that builds the tables of more than 256 rows: an eighth of the rows per block in words of 32 (blocks without rows at 257), one word
 # per block and several, the largest batch whose masks fit and the first that takes a block per pair of experts, an owner's slice of the experts
 @pytest.mark.parametrize("tokens,experts,selected,first,local", [(257, 512, 10, 0, 512), (512, 512, 1, 0, 512), (1003, 1000, 8, 0, 1000), (2049, 16, 16, 0, 16), (4096, 512, 10, 128, 64),
-                                                                 (16640, 512, 2, 0, 512), (16641, 512, 2, 0, 512), (300, 1024, 64, 0, 1024)])
+                                                                 (16640, 512, 2, 0, 512), (16641, 512, 2, 0, 512), (300, 1024, 64, 0, 1024),
+                                                                 (300, 8, 3, 0, 8), (549, 8, 2, 0, 8), (550, 8, 2, 0, 8), (639, 8, 1, 0, 8), (640, 8, 1, 0, 8)])   # few routes: one block
 def test_tables_of_large_batches(oracle, tokens, experts, selected, first, local):
     rng = np.random.default_rng(tokens)
     ids = np.argsort(rng.random((tokens, experts), dtype=np.float32) - (np.arange(experts) < experts // 8) * 0.5, axis=1)[:, :selected].astype(np.uint32)

@@ -855,7 +855,10 @@ int launch_permute(const uint32_t* ids, uint32_t tokens, uint32_t experts, uint3
     // the cluster reads the ids until its last writes; the launches below have read them before they write tile table and offsets
     const uint64_t id_bytes = static_cast<uint64_t>(tokens) * selected * 4;
     const bool ids_apart = !overlap(ids, id_bytes, tasks, 8 + bound * 8ull) && !(offsets && overlap(ids, id_bytes, offsets, (experts + 5) * 4ull));
-    if (ids_apart && cluster_fits(tokens, experts))
+    // Tables of few routes alone: the one block is level up to about 1100 routes, or 640 rows of one expert each (300 rows, two of 8 experts: 3.5 us, cluster
+    // 4.3; 300 rows, four of 64: 4.4 and 4.3; 512 rows, two of 8: 4.0 and 4.4; 1003 rows of one expert: 6.8 and 6.2). With offsets the cluster saves a launch.
+    const bool cluster = offsets || tokens >= 640 || static_cast<uint64_t>(tokens) * selected >= 1100;
+    if (cluster && ids_apart && cluster_fits(tokens, experts))
         return launch_tables_cluster(ids, tokens, experts, selected, tile, first, local_only, token_map, counts, tasks, offsets, error, st);
     if (tables_fit(tokens, experts)) {
         if (int rc = launch_tables(ids, tokens, experts, selected, tile, first, local_only, token_map, counts, tasks, error, st)) return rc;
