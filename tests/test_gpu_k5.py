@@ -315,3 +315,38 @@ def test_many_tiles_per_block(oracle, tokens, experts, selected):
     got = out.cpu().numpy().reshape(tokens, selected, rows)[::16]
     bound = (cols + 8) * 2.0 ** -24 * 4 * np.abs(w64).max() * np.abs(x[::16].astype(np.float64)).sum(axis=1)[:, None, None]
     assert np.isfinite(out.cpu().numpy()).all() and np.all(np.abs(got - want) <= bound)
+
+
+# Short rows: whole blocks per tile where the tiles are fewer than the blocks (one block of several units, several blocks per tile and blocks without work
+# at the end), an even split beyond; each row the bits it has alone
+@pytest.mark.parametrize("tokens,experts,selected", [(8, 3, 1), (40, 16, 2), (64, 64, 4), (300, 100, 8), (8, 200, 40)])
+@pytest.mark.parametrize("type_,rows,cols", [(formats.Q5_K, 256, 512), (formats.Q5_1, 272, 128), (formats.Q5_1, 64, 1024)])
+@pytest.mark.parametrize("gate_up", [False, True])
+def test_whole_blocks_per_tile(oracle, type_, rows, cols, gate_up, tokens, experts, selected):
+    rng = np.random.default_rng(tokens + experts)
+    w = np.concatenate([formats.quantize(type_, synth.normal(200 + i % 7, (rows, cols), 0.02)).reshape(-1) for i in range(experts)])
+    t = dev(w)
+    ms = L.matrix_set(t, type_, formats.GGUF, rows, cols, experts)
+    ids = np.argsort(rng.random((tokens, experts)), axis=1)[:, :selected].astype(np.int32)
+    dx, e = dev(synth.normal(104, (tokens, cols), 1.0)), torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(x, which):
+        n = len(which)
+        dids = dev(which)
+        tmap, counts = torch.empty(experts * n, dtype=torch.int32, device=DEV), torch.empty(experts, dtype=torch.int32, device=DEV)
+        tasks = torch.empty(capi.lib().tsp_moe_tasks_words(n, experts, selected, 8), dtype=torch.int32, device=DEV)
+        out = torch.full((n * selected, rows), np.nan, dtype=torch.float32, device=DEV)
+        capi.call("tsp_moe_permute", dids.data_ptr(), n, experts, selected, 8, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(), e.data_ptr(), L.stream_ptr())
+        if gate_up:
+            capi.call("tsp_moe_gate_up_swiglu", C.byref(ms), C.byref(ms), x.data_ptr(), cols * 4, n, selected, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(),
+                      out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        else:
+            capi.call("tsp_moe_project", C.byref(ms), x.data_ptr(), cols * 4, selected, n, selected, tmap.data_ptr(), counts.data_ptr(), tasks.data_ptr(),
+                      out.data_ptr(), rows * 4, 0, e.data_ptr(), L.stream_ptr())
+        torch.cuda.synchronize()
+        return out.view(n, selected, rows)
+
+    got = run(dx, ids)
+    assert int(e.item()) == 0 and bool(torch.isfinite(got).all())
+    for at in range(0, tokens, max(1, tokens // 8)):   # one row: an even split
+        assert torch.equal(run(dx[at:at + 1], ids[at:at + 1])[0], got[at])

@@ -39,6 +39,7 @@ struct K5Params {
     uint32_t lanes_per_row;   // lanes that share one weight row: the largest power of two <= min(32, groups)
     float* out; uint64_t out_stride_bytes;
     uint32_t* error;
+    uint32_t staging;         // what staging the rows of a tile costs, in units
 };
 
 // byte k of `q` as a float: 0x4B0000bb is 2^23 + bb, the subtraction is exact (no integer-to-float conversion instruction)
@@ -388,7 +389,20 @@ __device__ __noinline__ void k5_wide_unit(const KmTile* tile, const uint8_t* mA,
 
 // Shared memory (from a multiple of 1024): barriers, tile table, high halves [8][x_stride], low halves [8][x_stride], group sums [group][8] (of the
 // scaled values), partial sums [unit of a batch][K part][lane][4], stages [matrix][lines].
-template <uint32_t TYPE, bool GATEUP>
+// WHOLE: where whole blocks per tile come out shorter than an even split, each tile gets as many blocks as there are for all. An even split has blocks
+// that straddle tiles and stage the rows of both, a chain of loads and barriers worth p.staging units (about 2.5 us): a few units of short rows
+// take no longer than that. 256 x 512 of 16 experts, 72 tiles 16 -> 11 us, 12 tiles 9 -> 7.
+__device__ __forceinline__ uint2 km_whole(uint32_t n_tiles, uint32_t tile_units, uint32_t staging) {   // first unit and number of units of this block
+    const uint32_t n_units = n_tiles * tile_units, share = n_units / gridDim.x, rest = n_units - share * gridDim.x;
+    const uint32_t per_tile = n_tiles ? gridDim.x / n_tiles : 0u;   // 0: more tiles than blocks
+    if (per_tile && share >= 2u && (tile_units + per_tile - 1u) / per_tile < share + staging) {   // uniform over the grid
+        const uint32_t tile = blockIdx.x / per_tile, sub = blockIdx.x - tile * per_tile, from = tile_units * sub / per_tile;
+        return tile < n_tiles ? make_uint2(tile * tile_units + from, tile_units * (sub + 1u) / per_tile - from) : make_uint2(0u, 0u);
+    }
+    const uint32_t more = rest * blockIdx.x / gridDim.x;   // the remainder spread over the blocks
+    return make_uint2(share * blockIdx.x + more, share + rest * (blockIdx.x + 1u) / gridDim.x - more);
+}
+template <uint32_t TYPE, bool GATEUP, bool WHOLE>
 __global__ void __launch_bounds__(kKmThreads, 1) gemv_k5_mma_kernel(const __grid_constant__ K5Maps maps, const K5Params p) {
     pdl_launch_dependents();
     extern __shared__ uint8_t km_raw[];
@@ -415,9 +429,10 @@ __global__ void __launch_bounds__(kKmThreads, 1) gemv_k5_mma_kernel(const __grid
     const uint32_t n_tiles = p.token_map ? p.tasks[0] : (p.tokens + 7u) / 8u;
     const uint32_t tile_units = p.rows / RW;     // whole: the launcher asks for it
     const uint64_t n_units = static_cast<uint64_t>(n_tiles) * tile_units;
-    const uint64_t unit0 = n_units * blockIdx.x / gridDim.x;
-    const uint32_t units = static_cast<uint32_t>(n_units * (blockIdx.x + 1) / gridDim.x - unit0);
-    const uint32_t tile0 = static_cast<uint32_t>(unit0 / tile_units), first0 = static_cast<uint32_t>(unit0 % tile_units);   // the run's first tile and unit in it
+    const uint64_t unit0 = WHOLE ? km_whole(n_tiles, tile_units, p.staging).x : n_units * blockIdx.x / gridDim.x;
+    const uint32_t units = WHOLE ? km_whole(n_tiles, tile_units, p.staging).y : static_cast<uint32_t>(n_units * (blockIdx.x + 1) / gridDim.x - unit0);
+    const uint32_t tile0 = WHOLE ? static_cast<uint32_t>(unit0) / tile_units : static_cast<uint32_t>(unit0 / tile_units);   // the run's first tile and unit in it
+    const uint32_t first0 = WHOLE ? static_cast<uint32_t>(unit0) - tile0 * tile_units : static_cast<uint32_t>(unit0 % tile_units);
     // expert, first route and count of a tile (count 0: an entry that names no expert)
     auto look_up = [&](uint32_t tile, uint32_t& expert, uint32_t& start, uint32_t& count) {
         expert = 0; start = tile * 8u; count = 0;
@@ -678,18 +693,18 @@ int launch_dequant_k5(uint32_t type, const uint8_t* m, uint64_t elements, float*
     return TSP_OK;
 }
 
-template <uint32_t TYPE, bool GATEUP>
+template <uint32_t TYPE, bool GATEUP, bool WHOLE>
 static int launch_km(const K5Maps& maps, const K5Params& p, size_t smem, int grid, cudaStream_t st) {
     static thread_local int regs_ok = -1;   // the register hand-over adds up for this build
     if (regs_ok < 0) {
         cudaFuncAttributes fa{};
-        TSP_CUDA(cudaFuncGetAttributes(&fa, gemv_k5_mma_kernel<TYPE, GATEUP>));
+        TSP_CUDA(cudaFuncGetAttributes(&fa, gemv_k5_mma_kernel<TYPE, GATEUP, WHOLE>));
         regs_ok = (fa.numRegs >= kKmProdRegs && static_cast<int>(kKmWarps) * (kKmConsRegs - fa.numRegs) <= 4 * (fa.numRegs - kKmProdRegs)) ? 1 : 0;
     }
     if (!regs_ok) return fail(TSP_E_CUDA, "five-bit projection kernel: the compiled register count does not allow the producer/consumer register hand-over");
     static thread_local SmemAttrCache configured;   // per kernel instantiation, keyed by device
-    TSP_CUDA(ensure_dynamic_smem(gemv_k5_mma_kernel<TYPE, GATEUP>, configured, smem));
-    TSP_CUDA(launch_pdl(gemv_k5_mma_kernel<TYPE, GATEUP>, dim3(grid), dim3(kKmThreads), smem, st, maps, p));
+    TSP_CUDA(ensure_dynamic_smem(gemv_k5_mma_kernel<TYPE, GATEUP, WHOLE>, configured, smem));
+    TSP_CUDA(launch_pdl(gemv_k5_mma_kernel<TYPE, GATEUP, WHOLE>, dim3(grid), dim3(kKmThreads), smem, st, maps, p));
     return TSP_OK;
 }
 
@@ -734,6 +749,7 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
     if (nc == 1 && a->rows % rw == 0 && groups % km_groups == 0 && a->cols <= 3328) {
         for (p.wpu = 1; p.wpu < kKmParts && groups / km_groups >= 2u * p.wpu;) p.wpu *= 2;
         const uint32_t lines = rw * p.row_bytes / 128u;   // whole: eight rows of 176 or 96 bytes a step
+        p.staging = min(4000u / a->cols, 5u);             // 2.5 us against 0.6 ns a column, and half a microsecond for a unit of few
         p.copies = (lines + 255u) / 256u;                 // a box holds 256 lines at most; 16 rows are an even number of lines
         p.copy_lines = lines / p.copies;
         p.mat_bytes = (lines * 128u + 1023u) & ~1023u;
@@ -760,8 +776,13 @@ int launch_gemv_k5(const tsp_matrix_set* a, const tsp_matrix_set* b, bool gateup
             }
         if (!gateup) { maps.m[2] = maps.m[0]; maps.m[3] = maps.m[1]; }
         const size_t km_smem = p.off_stage + static_cast<size_t>(p.stages) * p.stage_bytes + 1024;
-        if (a->type == TSP_TYPE_Q5_K) return gateup ? launch_km<13u, true>(maps, p, km_smem, sms, st) : launch_km<13u, false>(maps, p, km_smem, sms, st);
-        return gateup ? launch_km<7u, true>(maps, p, km_smem, sms, st) : launch_km<7u, false>(maps, p, km_smem, sms, st);
+        // Whole blocks per tile: routed batches whose tiles are little work beside a staging (up to 32 units of 512 columns). Larger ones gain little and pay
+        // 0.2 to 0.4 us a launch for the choice, as batches of a few rows do; 2048 columns in this form's arithmetic came out 2.5 % slower.
+        const bool whole = token_map && tokens >= 8 && a->rows / rw * a->cols <= 16384u;
+#define TSP_KM(T, G) (whole ? launch_km<T, G, true>(maps, p, km_smem, sms, st) : launch_km<T, G, false>(maps, p, km_smem, sms, st))
+        if (a->type == TSP_TYPE_Q5_K) return gateup ? TSP_KM(13u, true) : TSP_KM(13u, false);
+        return gateup ? TSP_KM(7u, true) : TSP_KM(7u, false);
+#undef TSP_KM
     }
     const size_t smem = static_cast<size_t>(p.tile_tokens) * groups * 9 * sizeof(float4);
     if (smem > 200 * 1024) return fail(TSP_E_ARG, "five-bit projection: %u columns x %u token rows do not fit the activation staging", a->cols, p.tile_tokens);
