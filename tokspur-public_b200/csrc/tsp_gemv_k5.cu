@@ -395,7 +395,7 @@ __device__ __noinline__ void k5_wide_unit(const KmTile* tile, const uint8_t* mA,
 __device__ __forceinline__ uint2 km_whole(uint32_t n_tiles, uint32_t tile_units, uint32_t staging) {   // first unit and number of units of this block
     const uint32_t n_units = n_tiles * tile_units, share = n_units / gridDim.x, rest = n_units - share * gridDim.x;
     const uint32_t per_tile = n_tiles ? gridDim.x / n_tiles : 0u;   // 0: more tiles than blocks
-    if (per_tile && share >= 2u && (tile_units + per_tile - 1u) / per_tile < share + staging) {   // uniform over the grid
+    if (per_tile && 2u * n_units >= 3u * gridDim.x && (tile_units + per_tile - 1u) / per_tile < share + staging) {   // uniform over the grid
         const uint32_t tile = blockIdx.x / per_tile, sub = blockIdx.x - tile * per_tile, from = tile_units * sub / per_tile;
         return tile < n_tiles ? make_uint2(tile * tile_units + from, tile_units * (sub + 1u) / per_tile - from) : make_uint2(0u, 0u);
     }
