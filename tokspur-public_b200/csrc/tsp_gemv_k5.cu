@@ -391,7 +391,8 @@ __device__ __noinline__ void k5_wide_unit(const KmTile* tile, const uint8_t* mA,
 // scaled values), partial sums [unit of a batch][K part][lane][4], stages [matrix][lines].
 // WHOLE: where whole blocks per tile come out shorter than an even split, each tile gets as many blocks as there are for all. An even split has blocks
 // that straddle tiles and stage the rows of both, a chain of loads and barriers worth p.staging units (about 2.5 us): a few units of short rows
-// take no longer than that. 256 x 512 of 16 experts, 72 tiles 16 -> 11 us, 12 tiles 9 -> 7.
+// take no longer than that. 256 x 512 of 16 experts: 72 tiles 16 -> 11 us, 16 tiles 10.4 -> 7.5. With fewer than one and a half units per block few
+// blocks straddle (12 tiles of 16 units 6.8 us, whole blocks 7.4).
 __device__ __forceinline__ uint2 km_whole(uint32_t n_tiles, uint32_t tile_units, uint32_t staging) {   // first unit and number of units of this block
     const uint32_t n_units = n_tiles * tile_units, share = n_units / gridDim.x, rest = n_units - share * gridDim.x;
     const uint32_t per_tile = n_tiles ? gridDim.x / n_tiles : 0u;   // 0: more tiles than blocks
